@@ -64,12 +64,9 @@ struct GridParams
 #endif
 constexpr double kNearRadius = RG_GRID_NEAR_RADIUS;
 
-// FP32: the hardware approximations unrefined; FP64: correctly rounded
+// FP32: the hardware approximation unrefined; FP64: refined to about 1 ulp
 __device__ __forceinline__ float rcpT(float x) { return rgd::rcpApprox(x); }
-__device__ __forceinline__ double rcpT(double x) { return __drcp_rn(x); }
-__device__ __forceinline__ double sqrtT(double x) { return sqrt(x); }
-__device__ __forceinline__ double erfcT(double x) { return erfc(x); }
-__device__ __forceinline__ double expT(double x) { return exp(x); }
+__device__ __forceinline__ double rcpT(double x) { return rgd::rcpHouseholder(x); }
 
 template <typename Real>
 struct Factor
@@ -144,26 +141,23 @@ __device__ __forceinline__ Factor<float> ewaldFactor<float>(float rr, float cq, 
   return f;
 }
 
+// FP64: the ladder of radial factors with the alternating signs
+template <bool CHECK>
+__device__ __forceinline__ Factor<double> ewaldFactor64(double rr, double cq, double alpha)
+{
+  double B[4];
+  rgd::ewaldLadder<4, CHECK>(rr, alpha, 2.0 * alpha * rg::kInvSqrtPi, 2.0 * alpha * alpha, B);
+  Factor<double> f;
+  f.e = cq * B[0];
+  f.f1 = -cq * B[1];
+  f.f2 = cq * B[2];
+  f.f3 = -cq * B[3];
+  return f;
+}
 template <>
 __device__ __forceinline__ Factor<double> ewaldFactor<double>(double rr, double cq, double alpha)
 {
-  using Real = double;
-  Real r = sqrtT(rr);
-  Real ec = erfcT(alpha * r);
-  Real ex = expT(-alpha * alpha * rr);
-  Real etr = Real(2) * alpha * r * ex * Real(0.564189583547756286948079451560772586);
-  Real ar2 = alpha * alpha * rr;
-  Real invr = rcpT(r);
-  Real invrr = invr * invr;
-  Real i3 = invr * invrr;
-  Real i5 = i3 * invrr;
-  Real i7 = i5 * invrr;
-  Factor<Real> f;
-  f.e = cq * ec * invr;
-  f.f1 = -cq * (etr + ec) * i3;
-  f.f2 = cq * (etr * (Real(2) * ar2 + Real(3)) + Real(3) * ec) * i5;
-  f.f3 = -cq * (etr * (Real(4) * ar2 * ar2 + Real(10) * ar2 + Real(15)) + Real(15) * ec) * i7;
-  return f;
+  return ewaldFactor64<true>(rr, cq, alpha);
 }
 
 // Accumulators: FP64 plain sums, or FP32 chunk partials folded into a TwoSum-compensated hi/lo pair.
@@ -301,8 +295,8 @@ __device__ __forceinline__ void addPair(Acc& acc, const Factor<R>& f, R dx, R dy
 // NP Lennard-Jones probes (1 or 2) share one candidate set: the distances, the reciprocal and the staging are computed
 // once per pair and each probe adds its own factors (ipar holds NP parameter sets per image).
 template <typename Real, int TYPE, bool TRICLINIC, bool COUNT, int NP, bool CLIP>
-__global__ void __launch_bounds__(256, (!TRICLINIC && sizeof(Real) == 4) ? 3 : 1) gridKernel(GridParams p, const double4* __restrict__ ipos,
-                                                  const double4* __restrict__ ipar, int bx, int by, int bz)
+__global__ void __launch_bounds__(256, (!TRICLINIC && sizeof(Real) == 4) ? 3 : (sizeof(Real) == 8 && NP == 1 ? 2 : 1))
+gridKernel(GridParams p, const double4* __restrict__ ipos, const double4* __restrict__ ipar, int bx, int by, int bz)
 {
   using V4 = typename Vec4<Real>::T;
   constexpr bool EWALD = (TYPE == RG_GRID_EWALD_REAL);
@@ -585,6 +579,208 @@ __global__ void __launch_bounds__(256, (!TRICLINIC && sizeof(Real) == 4) ? 3 : 1
   dst[1] = make_double2(v[2], v[3]);
   dst[2] = make_double2(v[4], v[5]);
   dst[3] = make_double2(v[6], v[7]);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------------------------
+// FP64 rectangular grids. The bound is the FP64 pipe (64 lanes per SM: an instruction of a warp holds its scheduler for
+// two cycles), so the kernel spends as few FP64 instructions per pair as it can: reciprocals and reciprocal square
+// roots by one Householder step, erfc and the derivative factors from one exponential (ewaldLadder), the products of
+// the displacements shared by the probes. A warp owns 4 x 4 x 2 points of the brick of 8 x 8 x 4 and compacts the staged
+// images within reach of them into an index list, and runs over it without branches (two candidates in flight): a lane
+// whose pair lies outside has its charge, or its epsilon and shift, zeroed. Measured at 80 x 80 x 54 points of the
+// 20.0 x 19.9 x 13.4 A cell: two Lennard-Jones probes 654 -> 567 us, the Ewald grid 2.02 -> 1.11 ms; the FP64 pipe is 75
+// and 69 % busy, the rest waits on the chain of one pair.
+// ---------------------------------------------------------------------------------------------------------------------
+constexpr int kRectThreads = 256;
+constexpr int kRectChunk = kRectThreads * kPer;
+
+template <int TYPE, int NP>
+constexpr size_t rectSharedBytes()
+{
+  return sizeof(double4) * kRectChunk * (TYPE == RG_GRID_EWALD_REAL ? 1 : 1 + NP) +
+         sizeof(unsigned short) * (kRectThreads / 32) * kRectChunk;
+}
+
+template <int TYPE, int NP, bool COUNT, bool CLIP>
+__global__ void __launch_bounds__(kRectThreads, 2) gridKernelRect64(GridParams p, const double4* __restrict__ ipos,
+                                                                    const double4* __restrict__ ipar)
+{
+  constexpr bool EWALD = TYPE == RG_GRID_EWALD_REAL;
+  extern __shared__ unsigned char smem_raw[];
+  double4* cpos = reinterpret_cast<double4*>(smem_raw);
+  double4* cpar = cpos + kRectChunk;  // NP parameter lists (Lennard-Jones)
+  unsigned short* wlists =
+      reinterpret_cast<unsigned short*>(smem_raw + sizeof(double4) * kRectChunk * (EWALD ? 1 : 1 + NP));
+  __shared__ int warp_sums[33];
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int wx = warp & 1, wy = (warp >> 1) & 1, wz = warp >> 2;
+  const int kb = static_cast<int>(blockIdx.z) + p.zb0;
+  const int i = blockIdx.x * 8 + 4 * wx + (lane & 3), j = blockIdx.y * 8 + 4 * wy + ((lane >> 2) & 3),
+            k = kb * 4 + 2 * wz + (lane >> 4);
+  const bool valid = i < p.nx && j < p.ny && k < p.nz;
+
+  // grid point (interpolation_energy_grid.cpp:3827-3829), brick centre, and the centre of the warp's points
+  const double s[3] = {i * p.delta[0], j * p.delta[1], k * p.delta[2]};
+  const double sc[3] = {(blockIdx.x * 8 + 3.5) * p.delta[0], (blockIdx.y * 8 + 3.5) * p.delta[1],
+                        (kb * 4 + 1.5) * p.delta[2]};
+  const double sw[3] = {(4 * wx - 2) * p.delta[0], (4 * wy - 2) * p.delta[1], (2 * wz - 1) * p.delta[2]};
+  double ctr[3], q[3], wc[3], half2 = 0.0;
+#pragma unroll
+  for (int r = 0; r < 3; ++r)
+  {
+    const double pos = p.cell[0][r] * s[0] + p.cell[1][r] * s[1] + p.cell[2][r] * s[2];
+    ctr[r] = p.cell[0][r] * sc[0] + p.cell[1][r] * sc[1] + p.cell[2][r] * sc[2];
+    q[r] = pos - ctr[r];
+    wc[r] = p.cell[0][r] * sw[0] + p.cell[1][r] * sw[1] + p.cell[2][r] * sw[2];
+  }
+#pragma unroll
+  for (int g = 0; g < 4; ++g)  // the longest of the four diagonals of the warp's points
+  {
+    double d2 = 0.0;
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+    {
+      const double v = 1.5 * p.cell[0][r] * p.delta[0] + ((g & 1) ? -1.5 : 1.5) * p.cell[1][r] * p.delta[1] +
+                       ((g & 2) ? -0.5 : 0.5) * p.cell[2][r] * p.delta[2];
+      d2 += v * v;
+    }
+    half2 = fmax(half2, d2);
+  }
+  const double reach = sqrt(p.rc2) + sqrt(half2) + 1e-6;
+  const double reach2 = reach * reach;
+  unsigned short* wl = wlists + warp * kRectChunk;
+
+  double acc[NP][8];
+#pragma unroll
+  for (int n = 0; n < NP; ++n)
+#pragma unroll
+    for (int c = 0; c < 8; ++c) acc[n][c] = 0.0;
+  unsigned long long npairs = 0;
+
+  for (int base = 0; base < p.n_images; base += kRectChunk)
+  {
+    double4 ip[kPer];
+    bool ok[kPer];
+    int cnt = 0;
+#pragma unroll
+    for (int r = 0; r < kPer; ++r)
+    {
+      const int idx = base + tid * kPer + r;
+      ok[r] = false;
+      if (idx < p.n_images)
+      {
+        ip[r] = ipos[idx];
+        ip[r].x -= ctr[0];
+        ip[r].y -= ctr[1];
+        ip[r].z -= ctr[2];
+        ok[r] = ip[r].x * ip[r].x + ip[r].y * ip[r].y + ip[r].z * ip[r].z < p.filter2;
+        cnt += ok[r] ? 1 : 0;
+      }
+    }
+    int total;
+    int off = blockExclusiveScan(cnt, warp_sums, &total);
+#pragma unroll
+    for (int r = 0; r < kPer; ++r)
+      if (ok[r])
+      {
+        cpos[off] = ip[r];
+        if constexpr (!EWALD)
+#pragma unroll
+          for (int n = 0; n < NP; ++n)
+            cpar[n * kRectChunk + off] = ipar[static_cast<long long>(base + tid * kPer + r) * NP + n];
+        ++off;
+      }
+    __syncthreads();
+    // this warp's candidates, in staging order
+    int nw = 0;
+    for (int b0 = 0; b0 < total; b0 += 32)
+    {
+      const int c = b0 + lane;
+      bool in = false;
+      if (c < total)
+      {
+        const double ex = cpos[c].x - wc[0], ey = cpos[c].y - wc[1], ez = cpos[c].z - wc[2];
+        in = ex * ex + ey * ey + ez * ez < reach2;
+      }
+      const unsigned ballot = __ballot_sync(0xffffffffu, in);
+      if (in) wl[nw + __popc(ballot & ((1u << lane) - 1u))] = static_cast<unsigned short>(c);
+      nw += __popc(ballot);
+    }
+    __syncwarp();
+#pragma unroll 2
+    for (int w = 0; w < nw; ++w)
+    {
+      const int c = wl[w];
+      const double4 a = cpos[c];
+      const double dx = q[0] - a.x, dy = q[1] - a.y, dz = q[2] - a.z;
+      double rr = dx * dx + dy * dy + dz * dz;
+      rr = rr > 0.1 ? rr : 0.1;
+      bool in = rr < p.rc2;
+      if constexpr (CLIP)
+      {
+        const double nine[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+        in = in && rgd::insideSupercell<false>(p.clip_h, nine, dx, dy, dz);
+      }
+      if (COUNT && in && valid) ++npairs;
+      const double dxy = dx * dy, dxz = dx * dz, dyz = dy * dz;
+      const double dxyz = dxy * dz;
+#pragma unroll
+      for (int n = 0; n < NP; ++n)
+      {
+        Factor<double> f;
+        if constexpr (EWALD)
+          f = ewaldFactor64<false>(rr, in ? a.w : 0.0, p.alpha);
+        else
+        {
+          const double4 pq = cpar[n * kRectChunk + c];
+          f = ljFactor<TYPE, double>(rr, in ? pq.x : 0.0, pq.y, in ? pq.z : 0.0);
+        }
+        acc[n][0] += f.e;
+        acc[n][1] = fma(dx, f.f1, acc[n][1]);
+        acc[n][2] = fma(dy, f.f1, acc[n][2]);
+        acc[n][3] = fma(dz, f.f1, acc[n][3]);
+        acc[n][4] = fma(dxy, f.f2, acc[n][4]);
+        acc[n][5] = fma(dxz, f.f2, acc[n][5]);
+        acc[n][6] = fma(dyz, f.f2, acc[n][6]);
+        acc[n][7] = fma(dxyz, f.f3, acc[n][7]);
+      }
+    }
+    __syncthreads();
+  }
+
+  if (COUNT)
+  {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) npairs += __shfl_down_sync(0xffffffffu, npairs, o);
+    if (lane == 0 && npairs) atomicAdd(p.pair_count, npairs);
+  }
+  if (!valid) return;
+#pragma unroll
+  for (int n = 0; n < NP; ++n)
+  {
+    // rectangular scaling by the cell diagonal (framework_molecule_grid.cpp:236-243), division by the cell counts and
+    // the overlap clamp (interpolation_energy_grid.cpp:3847-3874)
+    const double hx = p.cell[0][0] / p.ncells[0], hy = p.cell[1][1] / p.ncells[1], hz = p.cell[2][2] / p.ncells[2];
+    double v[8] = {acc[n][0],           acc[n][1] * hx,      acc[n][2] * hy,      acc[n][3] * hz,
+                   acc[n][4] * hx * hy, acc[n][5] * hx * hz, acc[n][6] * hy * hz, acc[n][7] * hx * hy * hz};
+    const double oc = p.overlap;
+    if (v[0] > oc)
+    {
+      v[0] = 2.0 * oc;
+      v[1] = fmin(fmax(v[1], -oc), oc);
+      v[2] = fmin(fmax(v[2], -oc), oc);
+      v[3] = fmin(fmax(v[3], -oc), oc);
+      v[4] = v[5] = v[6] = v[7] = 0.0;
+    }
+    double2* dst = reinterpret_cast<double2*>(
+        p.out[n] + 8 * (static_cast<long long>(i) +
+                        static_cast<long long>(p.nx) * (static_cast<long long>(j) + static_cast<long long>(p.ny) * k)));
+    dst[0] = make_double2(v[0], v[1]);
+    dst[1] = make_double2(v[2], v[3]);
+    dst[2] = make_double2(v[4], v[5]);
+    dst[3] = make_double2(v[6], v[7]);
   }
 }
 
@@ -1013,6 +1209,18 @@ cudaError_t launchPacked(const GridParams& p, const double4* ipos, const double4
   return cudaGetLastError();
 }
 
+template <int TYPE, int NP, bool COUNT, bool CLIP>
+cudaError_t launchRect64(const GridParams& p, const double4* ipos, const double4* ipar, cudaStream_t stream)
+{
+  const int zbricks = p.zb1 > p.zb0 ? p.zb1 - p.zb0 : (p.nz + 3) / 4;
+  dim3 grid((p.nx + 7) / 8, (p.ny + 7) / 8, zbricks);
+  constexpr size_t shmem = rectSharedBytes<TYPE, NP>();
+  auto kern = gridKernelRect64<TYPE, NP, COUNT, CLIP>;
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(shmem));
+  kern<<<grid, kRectThreads, shmem, stream>>>(p, ipos, ipar);
+  return cudaGetLastError();
+}
+
 // Dynamic shared memory of a launch: the FP32/FP64 candidate list, NP parameter lists for Lennard-Jones grids, and the
 // FP64 near list of the FP32C Ewald grid.
 template <typename Real, int TYPE, int NP>
@@ -1050,11 +1258,30 @@ cudaError_t launchTyped(const GridParams& p, const double4* ipos, const double4*
         p.cell[1][2] == 0.0 && p.cell[2][0] == 0.0 && p.cell[2][1] == 0.0)
       return count ? launchPacked<TYPE, NP, true>(p, ipos, ipar, stream)
                    : launchPacked<TYPE, NP, false>(p, ipos, ipar, stream);
-  if (clip)
-    return count ? launchKernel<Real, TYPE, TRI, NP, true, true>(p, ipos, ipar, bx, by, bz, stream)
-                 : launchKernel<Real, TYPE, TRI, NP, false, true>(p, ipos, ipar, bx, by, bz, stream);
-  return count ? launchKernel<Real, TYPE, TRI, NP, true, false>(p, ipos, ipar, bx, by, bz, stream)
-               : launchKernel<Real, TYPE, TRI, NP, false, false>(p, ipos, ipar, bx, by, bz, stream);
+  // FP64 rectangular grids: gridKernelRect64 (bricks of 8 x 8 x 4 points). Its Ewald terms take erfc from a polynomial
+  // that ends at alpha r = 6; a force field whose alpha rc lies beyond (alpha = 0.265 and rc = 12 give 3.2) takes
+  // gridKernel, which checks each pair.
+  if constexpr (sizeof(Real) == 8 && !TRI)
+  {
+    if (TYPE != RG_GRID_EWALD_REAL || p.alpha * std::sqrt(p.rc2) < rgd::kErfcxMax)
+    {
+      if (clip)
+        return count ? launchRect64<TYPE, NP, true, true>(p, ipos, ipar, stream)
+                     : launchRect64<TYPE, NP, false, true>(p, ipos, ipar, stream);
+      return count ? launchRect64<TYPE, NP, true, false>(p, ipos, ipar, stream)
+                   : launchRect64<TYPE, NP, false, false>(p, ipos, ipar, stream);
+    }
+  }
+  if constexpr (sizeof(Real) == 8 && !TRI && TYPE != RG_GRID_EWALD_REAL)
+    return cudaErrorInvalidValue;  // not reached
+  else
+  {
+    if (clip)
+      return count ? launchKernel<Real, TYPE, TRI, NP, true, true>(p, ipos, ipar, bx, by, bz, stream)
+                   : launchKernel<Real, TYPE, TRI, NP, false, true>(p, ipos, ipar, bx, by, bz, stream);
+    return count ? launchKernel<Real, TYPE, TRI, NP, true, false>(p, ipos, ipar, bx, by, bz, stream)
+                 : launchKernel<Real, TYPE, TRI, NP, false, false>(p, ipos, ipar, bx, by, bz, stream);
+  }
 }
 
 template <typename Real, bool TRI>

@@ -1,0 +1,75 @@
+"""FP64 grid kernels at the edges of their bricks and of their dispatch rule, against the FP64 oracle.
+
+Tolerance: a channel is a sum of N terms whose largest are M times the sum, evaluated with a few ulp per term, so its
+error is about (N + 8) M 2^-52 relative: N = 400 pairs and M up to 1e4 (the cancelling Ewald terms) give 1e-9."""
+
+import math
+
+import numpy as np
+import pytest
+
+from raspa3_b200 import native
+from raspa3_b200.forcefield import KELVIN_TO_ENERGY
+from raspa3_b200.synthetic import synthetic_forcefield, synthetic_framework
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-9
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    c = native.Context(0)
+    yield c
+    c.close()
+
+
+def worst(got, ref, channels):
+    """max |got - ref| / max(|ref|, RMS of the channel) over the points below 1e4 K; the clamped points exactly."""
+    g, r = got.reshape(-1, channels), ref.reshape(-1, channels)
+    ok = np.abs(r[:, 0]) < 1e4 * KELVIN_TO_ENERGY
+    if not ok.any():
+        return 0.0
+    rms = np.sqrt(np.mean(r[ok] ** 2, axis=0)) + 1e-300
+    return float((np.abs(g[ok] - r[ok]) / np.maximum(np.abs(r[ok]), rms)).max())
+
+
+# one brick short of, equal to and one point beyond the 8 x 8 x 4 brick and its 4 x 4 x 2 warps; the smallest grid
+@pytest.mark.parametrize("dims", [(2, 2, 2), (8, 8, 4), (9, 7, 5), (17, 3, 10)])
+@pytest.mark.parametrize("grid_type", [0, 1, 2, 3])
+def test_tricubic_fp64_bricks(ctx, oracle, dims, grid_type):
+    ff = synthetic_forcefield(charges=True)
+    cell, atoms = synthetic_framework(ff, seed=11)
+    probe = ff.index("C_co2")
+    for cutoff in (12.0, 6.5):  # the reference's supercell, and one that clips pairs
+        got, stats = ctx.grid_build(grid_type, ff, cell, atoms, probe, cutoff, dims, native.PRECISION_FP64,
+                                    count_pairs=True)
+        ref = oracle.make_grid(grid_type, ff, cell, atoms, probe, cutoff, dims)
+        assert worst(got, ref, 8) < TOL
+        assert stats["pair_count"] == oracle.grid_pair_count(grid_type, ff, cell, atoms, probe, cutoff, dims)
+
+
+# alpha rc on both sides of 6, where the Ewald terms leave the polynomial for the library's erfc
+@pytest.mark.parametrize("alpha", [0.1, 0.4999, 0.5001, 0.9])
+def test_ewald_fp64_alpha(ctx, oracle, alpha):
+    ff = synthetic_forcefield(charges=True, alpha=alpha)
+    cell, atoms = synthetic_framework(ff, seed=12)
+    dims = (9, 8, 6)
+    got, _ = ctx.grid_build(1, ff, cell, atoms, 0, 12.0, dims, native.PRECISION_FP64)
+    assert worst(got, oracle.make_grid(1, ff, cell, atoms, 0, 12.0, dims), 8) < TOL
+
+
+def test_fp64_pair_of_probes_equals_single_builds(ctx):
+    torch = pytest.importorskip("torch")
+    ff = synthetic_forcefield(charges=True)
+    cell, atoms = synthetic_framework(ff, seed=13)
+    dims = (19, 18, 13)
+    probes = [ff.index("C_co2"), ff.index("O_co2"), ff.index("CH4")]
+    out = [torch.empty(8 * math.prod(dims), dtype=torch.float64, device="cuda") for _ in probes]
+    ctx.grid_build_set(ff, cell, atoms, 12.0, dims, native.PRECISION_FP64, [0, 0, 0], probes,
+                       [o.data_ptr() for o in out])
+    ctx.synchronize()
+    for probe, o in zip(probes, out):
+        single, _ = ctx.grid_build(0, ff, cell, atoms, probe, 12.0, dims, native.PRECISION_FP64)
+        assert worst(o.cpu().numpy(), single, 8) < 1e-13  # the same pair terms in the same order
+
