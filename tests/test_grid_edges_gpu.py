@@ -73,3 +73,20 @@ def test_fp64_pair_of_probes_equals_single_builds(ctx):
         single, _ = ctx.grid_build(0, ff, cell, atoms, probe, 12.0, dims, native.PRECISION_FP64)
         assert worst(o.cpu().numpy(), single, 8) < 1e-13  # the same pair terms in the same order
 
+
+# the triquintic kernel's brick is 8 x 4 x 4; alpha rc beyond 6 takes the library's erfc
+@pytest.mark.parametrize("dims", [(2, 2, 2), (8, 4, 4), (9, 5, 3)])
+@pytest.mark.parametrize("grid_type,alpha", [(0, 0.265), (1, 0.265), (1, 0.6)])
+@pytest.mark.parametrize("reference_rectangular", [False, True])
+def test_triquintic_fp64_bricks(ctx, oracle, dims, grid_type, alpha, reference_rectangular):
+    ff = synthetic_forcefield(charges=True, alpha=alpha)
+    cell, atoms = synthetic_framework(ff, seed=14)
+    probe = ff.index("C_co2")
+    for cutoff in (12.0, 6.5):
+        got, stats = ctx.grid_build_triquintic(grid_type, ff, cell, atoms, probe, cutoff, dims,
+                                               reference_rectangular=reference_rectangular, count_pairs=True)
+        ref = oracle.make_grid_triquintic(grid_type, ff, cell, atoms, probe, cutoff, dims,
+                                          reference_rectangular=reference_rectangular)
+        assert worst(got, ref, 27) < TOL
+        assert stats["pair_count"] == oracle.grid_pair_count(grid_type, ff, cell, atoms, probe, cutoff, dims)
+
