@@ -90,3 +90,68 @@ def test_triquintic_fp64_bricks(ctx, oracle, dims, grid_type, alpha, reference_r
         assert worst(got, ref, 27) < TOL
         assert stats["pair_count"] == oracle.grid_pair_count(grid_type, ff, cell, atoms, probe, cutoff, dims)
 
+
+def _grid_test(ctx, ff, cell, atoms, dims, bufs, points, scheme):
+    probe = ff.index("C_co2")
+    call = ctx.grid_validate_triquintic if scheme == 27 else ctx.grid_validate
+    return call(ff, cell, atoms, cell, probe, dims, bufs[0].data_ptr(), bufs[1].data_ptr(), 0.70, 1.0 / 300.0,
+                points=points)
+
+
+# one point, the edges of warps (32), blocks (128) and bins, and enough points that the image lists are not split
+@pytest.mark.parametrize("n", [1, 31, 33, 127, 129, 700, 4100])
+@pytest.mark.parametrize("scheme,alpha", [(8, 0.265), (8, 0.6), (27, 0.265)])
+def test_grid_test_point_counts(ctx, oracle, n, scheme, alpha):
+    """Sums of w x within 1e-9 of sqrt(sum w x^2 sum w), the accuracy of the pair sums above. The interpolated side of
+    the triquintic scheme is left out: the oracle sums the reference's monomial form, whose own rounding at cells next
+    to clamped points is larger."""
+    torch = pytest.importorskip("torch")
+    ff = synthetic_forcefield(charges=True, alpha=alpha)
+    cell, atoms = synthetic_framework(ff, seed=15)
+    dims = (21, 20, 14)
+    host = []
+    for gt, probe in ((0, ff.index("C_co2")), (1, 0)):
+        if scheme == 27:
+            host.append(ctx.grid_build_triquintic(gt, ff, cell, atoms, probe, 12.0, dims)[0])
+        else:
+            host.append(ctx.grid_build(gt, ff, cell, atoms, probe, 12.0, dims, native.PRECISION_FP64)[0])
+    bufs = [torch.from_numpy(h).cuda() for h in host]
+    points = np.random.default_rng(n).random((n, 3))
+    got = _grid_test(ctx, ff, cell, atoms, dims, bufs, points, scheme)
+    check = oracle.grid_validate_triquintic if scheme == 27 else oracle.grid_validate
+    ref = check(ff, cell, atoms, cell, ff.index("C_co2"), dims, host[0], host[1], 0.70, 1.0 / 300.0, points)
+    assert got["n_points"] == ref[34] == n
+    assert got["n_points_charge"] == ref[35]
+    s = np.array(got["sums"])
+    for base in (0, 17):
+        o = np.asarray(ref[base:base + 17])
+        scale = np.abs(o).copy()
+        scale[[1, 2]] = np.sqrt(o[4] * o[0])
+        scale[3] = o[4]
+        for a in range(3):
+            scale[[5 + a, 8 + a]] = np.sqrt(o[14 + a] * o[0])
+            scale[11 + a] = o[14 + a]
+        use = [0, 2, 4, 8, 9, 10, 14, 15, 16] if scheme == 27 else list(range(17))
+        d = np.abs(s[base:base + 17] - o)
+        assert np.all(d[use] <= 1e-9 * scale[use] + 1e-280), (base, s[base:base + 17], o)
+
+
+def test_grid_test_in_rounds(ctx):
+    """More points than one round holds: the sums are those of the two parts (rounding of 2^21 added terms)."""
+    torch = pytest.importorskip("torch")
+    ff = synthetic_forcefield(charges=True)
+    cell, atoms = synthetic_framework(ff, seed=16)
+    dims = (21, 20, 14)
+    bufs = []
+    for gt, probe in ((0, ff.index("C_co2")), (1, 0)):
+        bufs.append(torch.from_numpy(ctx.grid_build(gt, ff, cell, atoms, probe, 12.0, dims,
+                                                    native.PRECISION_FP64)[0]).cuda())
+    n = (1 << 21) + 1000
+    points = np.random.default_rng(3).random((n, 3))
+    whole = _grid_test(ctx, ff, cell, atoms, dims, bufs, points, 8)
+    parts = [_grid_test(ctx, ff, cell, atoms, dims, bufs, p, 8) for p in (points[:777777], points[777777:])]
+    assert whole["n_points"] == n
+    assert whole["n_points_charge"] == sum(p["n_points_charge"] for p in parts)
+    a, b = np.array(whole["sums"]), np.array(parts[0]["sums"]) + np.array(parts[1]["sums"])
+    scale = np.maximum(np.abs(a), np.repeat([np.sqrt(a[0] * a[4]), np.sqrt(a[17] * a[21])], 17))
+    assert np.all(np.abs(a - b) <= 1e-11 * scale)
