@@ -4,6 +4,8 @@
 
 #include <cuda_runtime.h>
 
+#include <vector>
+
 #include "../../include/raspa_gpu.h"
 
 namespace rgd
@@ -170,6 +172,35 @@ __device__ __forceinline__ double interpolateCorner(const Grid& g, const GridCel
 #pragma unroll
   for (int l = 0; l < 8; ++l) value += v[l] * cl.h[0][cx][ox[l]] * cl.h[1][cy][oy[l]] * cl.h[2][cz][oz[l]];
   return value;
+}
+
+// The same share for a lane that owns one corner (0..7) of a position's cell: its own bases only, in registers.
+__device__ __forceinline__ double interpolateLaneCorner(const Grid& g, double px, double py, double pz, int corner)
+{
+  int at[3];
+  double v[3], d[3];  // value and derivative basis of the corner along each axis
+  const int nc[3] = {g.nx - 1, g.ny - 1, g.nz - 1};
+#pragma unroll
+  for (int a = 0; a < 3; ++a)
+  {
+    const double s = fract1(g.ic[0][a] * px + g.ic[1][a] * py + g.ic[2][a] * pz) * static_cast<double>(nc[a]);
+    const long long c = static_cast<long long>(s);
+    const int i0 = static_cast<int>(c < nc[a] - 1 ? c : nc[a] - 1);
+    const double x = s - static_cast<double>(i0), x2 = x * x, x3 = x2 * x;
+    const bool far = (corner >> a) & 1;
+    const double one = -2.0 * x3 + 3.0 * x2;
+    v[a] = far ? one : 2.0 * x3 - 3.0 * x2 + 1.0;
+    d[a] = far ? x3 - x2 : x3 - 2.0 * x2 + x;
+    at[a] = i0 + (far ? 1 : 0);
+  }
+  const double2* p = reinterpret_cast<const double2*>(
+      g.data + 8 * (static_cast<long long>(at[0]) +
+                    static_cast<long long>(g.nx) * (static_cast<long long>(at[1]) + static_cast<long long>(g.ny) * at[2])));
+  // channels f, fx | fy, fz | fxy, fxz | fyz, fxyz
+  const double2 q0 = __ldg(p), q1 = __ldg(p + 1), q2 = __ldg(p + 2), q3 = __ldg(p + 3);
+  const double near = v[1] * (q0.x * v[0] + q0.y * d[0]) + d[1] * (q1.x * v[0] + q2.x * d[0]);
+  const double up = v[1] * (q1.y * v[0] + q2.y * d[0]) + d[1] * (q3.x * v[0] + q3.y * d[0]);
+  return v[2] * near + d[2] * up;
 }
 
 // Value and Cartesian gradient of the interpolant (InterpolationEnergyGrid::interpolateHessian, tricubic branch,
@@ -432,6 +463,11 @@ int systemScheme(const rg_system* s);
 rg_status proposalExport(rg_proposal* p, const double** cdf, const double** density, int* G, double* eps);
 rg_status ewaldExport(rg_ewald* e, const char4** kvec, const double** temp, const double2** s_rigid, int64_t* nk,
                       int kmax[3], double* alpha, double* single_ion_sum);
+// the k-vectors of an Ewald state as runs of consecutive kz of one (kx, ky), in order of falling largest |kz|:
+// {kx, ky, index of the first, (first kz, last kz) as two shorts}
+std::vector<int4> ewaldRuns(const rg_ewald* e);
+// the prefactor of the k-vector with kz = +m, -m of run r at [(2 m + (sign < 0)) runs + r] (0: not in the run)
+cudaError_t ewaldRunPrefactors(const rg_ewald* e, const std::vector<int4>& runs, std::vector<double>& out);
 
 // The supercell's minimum image keeps a displacement iff it lies in (-1/2, 1/2] of the supercell along every axis
 // (SimulationBox::applyPeriodicBoundaryConditions, simulationbox.ixx:131-161, in the supercell of
