@@ -1325,6 +1325,8 @@ std::vector<int4> ewaldRuns(const rg_ewald* e)
       z0 = z1 + 1;
     }
   }
+  auto reach = [](const int4& r) { return std::max(-static_cast<int>(static_cast<short>(r.w & 0xffff)), r.w >> 16); };
+  std::stable_sort(runs.begin(), runs.end(), [&](const int4& x, const int4& y) { return reach(x) > reach(y); });
   return runs;
 }
 }  // namespace rgd
@@ -1334,34 +1336,34 @@ std::vector<int4> ewaldRuns(const rg_ewald* e)
 // ewald.cpp:1098-1162, for one move in each of n systems that share the box, the force field and the k-vectors).
 //
 // Each system keeps two structure-factor buffers, stored and trial, and a flag says which is which; an accepted move
-// flips its system's flag (acceptEwaldMove, ewald.cpp:1565-1574, without a copy). The launch is (k-tile, system): a
-// block loads its system's moved atoms, builds their phase tables e^{i 2 pi m s_d} (m = 0..kmax_d) in shared memory,
-// and every thread forms Delta rho(k) of its k-vectors from two complex products per atom, reads S(k), writes
-// S(k) + Delta rho(k) and sums temp(k) (2 Re(conj(S) Delta rho) + |Delta rho|^2). Block partials are reduced per system
-// in block order by the system's last block, which writes the total into mapped pinned host memory. The traffic per
-// system and move is 32 bytes per k-vector (read S, write the trial S); k-vectors and prefactors are shared by all
-// systems and stay in L2.
+// flips its system's flag (acceptEwaldMove, ewald.cpp:1565-1574, without a copy). The launch is (k-range, system). The
+// traffic per system and move is 32 bytes per k-vector (read S, write the trial S); k-vectors and prefactors are shared
+// by all systems and stay in L2.
 // ---------------------------------------------------------------------------------------------------------------------
 struct rg_ewald_batch
 {
   rg_ewald* ewald = nullptr;
+  rg_ctx* ctx = nullptr;  // of the Ewald state, which may be gone when the batch is destroyed
   int n = 0;
   int max_atoms = 0;
-  double2* sk = nullptr;           // [2][n][nk]
-  unsigned char* cur = nullptr;    // [n]: which buffer holds the stored S(k) of system s
-  std::vector<unsigned char> cur_host;
-  MovedAtom* atoms = nullptr;      // [n][kBatchAtoms] device
-  MovedAtom* atoms_host = nullptr; // pinned
-  int* counts = nullptr;           // [n] moved atoms per system (device)
-  int* counts_host = nullptr;      // pinned
+  // [2][n][slots]: S(k) by rows of (|kz|, sign), a row holding the k-vectors of that kz of all runs side by side, so that
+  // neighbouring threads, which take neighbouring runs, read and write neighbouring numbers
+  double2* sk = nullptr;
+  int64_t slots = 0;
+  int* slot_of = nullptr;          // [nk]: where each k-vector is
+  int* row_start = nullptr;        // [2 (kmax_z + 1)]
+  std::vector<unsigned char> cur;  // [n]: which buffer holds the stored S(k) of system s
+  // the moved atoms (fractional coordinates and signed charge), their counts and the buffer flags of one call: one
+  // block of memory on the device and one pinned on the host, so that a call uploads it in one copy
+  unsigned char* upload = nullptr;
+  unsigned char* upload_host = nullptr;
   double* partial = nullptr;       // [n][blocks]
-  unsigned int* counter = nullptr; // [n]
   double* result = nullptr;        // device view of result_host
   double* result_host = nullptr;   // [n] mapped pinned
-  int blocks = 0;                  // k-ranges per system
-  int4* desc = nullptr;            // [blocks]: first k, end k, first (kx, ky) pair, pairs
-  int* kinfo = nullptr;            // [nk]: pair * 256 + (kz + 128)
-  char2* pairs = nullptr;          // [pairs]: (kx, ky)
+  int blocks = 0;                  // blocks per system
+  int n_runs = 0;
+  double* run_temp = nullptr;      // prefactor of kz = +m, -m of run r at [(2 m + (sign < 0)) n_runs + r]
+  int4* runs = nullptr;            // runs of consecutive kz of one (kx, ky), longest first (rgd::ewaldRuns)
   // device time of the last rg_ewald_batch_delta: events before the atom upload, before and after the kernel
   cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
   float upload_ms = 0.0f, kernel_ms = 0.0f;
@@ -1369,93 +1371,130 @@ struct rg_ewald_batch
 
 namespace
 {
-constexpr int kBatchAtoms = 16;       // old + new atoms of one system's move
-constexpr int kBatchKPerThread = 8;   // k-vectors per thread: a block covers at most kThreads * 8 of them
-constexpr int kBatchPairs = 128;      // (kx, ky) pairs of one block's k-range
+constexpr int kBatchAtoms = 16;   // old + new atoms of one system's move
+constexpr int kBatchM = 4;        // consecutive |kz| of one thread (five spill at three blocks per SM)
 
-// Shared memory of a block: the phasor tables exp(2 pi i m s_d) of its system's moved atoms (x: m = 0..kmax_x; y and z:
-// m = -kmax..kmax, the negative m as conjugates) and the weighted xy products of its (kx, ky) pairs.
-__host__ __device__ inline size_t batchSharedBytes(int stride, int kxm, int kym, int kzm)
+// The upload of one call: n * stride atoms, n counts, n flags
+inline size_t batchUploadBytes(int n, int stride)
 {
-  return sizeof(double2) * static_cast<size_t>(stride) * ((kxm + 1) + (2 * kym + 1) + (2 * kzm + 1) + kBatchPairs);
+  return sizeof(double4) * static_cast<size_t>(n) * stride + (sizeof(int) + 1) * static_cast<size_t>(n);
 }
 
-// One block per (k-range, system). The k-vectors come in the reference's order (kx outer, then ky, then kz), so a
-// k-range spans few (kx, ky) pairs: the block forms w_a exp(2 pi i (kx s_a,x + ky s_a,y)) once per pair and atom, and
-// each k then costs one complex multiply-add per atom with its z phasor. desc[b] = {first k, end k, first pair,
-// pairs}; kinfo[k] = pair * 256 + (kz + 128); pairs[p] = (kx, ky).
-__global__ void __launch_bounds__(kThreads) ewaldBatchDeltaKernel(
-    const int4* __restrict__ desc, const int* __restrict__ kinfo, const char2* __restrict__ pairs, int64_t nk,
-    int n_systems, const double* __restrict__ temp, double2* sk, const unsigned char* __restrict__ cur,
-    const MovedAtom* __restrict__ atoms, int atom_stride, const int* __restrict__ counts, int kxm, int kym, int kzm,
-    double* partial, unsigned int* counter, double* result)
+// Shared memory of a block: the phasors exp(2 pi i m s_d) of its system's moved atoms (x: m = 0..kmax_x with the atom's
+// weight, y: m = -kmax_y..kmax_y, z: m = 0..kmax_z).
+__host__ __device__ inline size_t batchSharedBytes(int stride, int kxm, int kym, int kzm)
+{
+  return sizeof(double2) * static_cast<size_t>(stride) * ((kxm + 1) + (2 * kym + 1) + (kzm + 1));
+}
+
+// Blocks (part, system). An item is one run of kz of a (kx, ky) and kBatchM values of m = |kz|; block `part` of a system
+// takes every gridDim.x-th group of kThreads items. With P = w e^{2 pi i (kx s_x + ky s_y)} = (p, q) and
+// (c, s) = e^{2 pi i m s_z} the sums over the atoms of p c, q s, p s and q c give Delta rho at both kz = m and kz = -m,
+// four FMAs for two k-vectors, and every z phasor is read by a whole warp at once. S(k) goes straight from HBM to the
+// thread that adds to it and back (rows by kz, see rg_ewald_batch): the bound is HBM, 32 bytes per k-vector. Before, a
+// thread took one k-vector at a time in list order and read two phasors per atom and k-vector from shared memory, whose
+// bandwidth bound it: 114 us for 1,184 systems of 8,124 k-vectors, now 81 us (47 us at the measured copy rate, were all
+// of S read and all of the trial S written through HBM).
+__global__ void __launch_bounds__(kThreads, 3) ewaldBatchDeltaKernel(
+    const int4* __restrict__ runs, int n_runs, const int* __restrict__ row_start, int64_t slots, int n_systems,
+    const double* __restrict__ run_temp, double2* sk, const unsigned char* __restrict__ upload, int atom_stride, int kxm,
+    int kym, int kzm, double* partial)
 {
   extern __shared__ double2 tab[];
   __shared__ double red[kThreads / 32];
-  __shared__ bool last;
   const int sys = blockIdx.y;
-  const int4 d = desc[blockIdx.x];
+  const double4* atoms = reinterpret_cast<const double4*>(upload) + static_cast<int64_t>(sys) * atom_stride;
+  const int* counts = reinterpret_cast<const int*>(reinterpret_cast<const double4*>(upload) +
+                                                   static_cast<int64_t>(n_systems) * atom_stride);
+  const int cur = reinterpret_cast<const unsigned char*>(counts + n_systems)[sys];
   const int na = counts[sys];
-  const int nx = kxm + 1, ny = 2 * kym + 1, nz = 2 * kzm + 1;
+  const double2* S = sk + (static_cast<int64_t>(cur) * n_systems + sys) * slots;
+  double2* T = sk + (static_cast<int64_t>(1 - cur) * n_systems + sys) * slots;
+  const int nx = kxm + 1, ny = 2 * kym + 1, nz = kzm + 1;
   double2* ex = tab;
   double2* ey = ex + atom_stride * nx;
   double2* ez = ey + atom_stride * ny;
-  double2* wxy = ez + atom_stride * nz;  // [pair][atom]
-  const MovedAtom* ma = atoms + static_cast<long long>(sys) * atom_stride;
-  const int per = nx + (kym + 1) + (kzm + 1);
-  for (int idx = threadIdx.x; idx < na * per; idx += blockDim.x)
+  const int per = nx + (kym + 1) + nz;
+  for (int idx = threadIdx.x; idx < na * per; idx += kThreads)
   {
     const int a = idx / per, m = idx - a * per;
+    const double4 at = atoms[a];
     const int dim = m < nx ? 0 : (m < nx + kym + 1 ? 1 : 2);
     const int mm = dim == 0 ? m : (dim == 1 ? m - nx : m - nx - (kym + 1));
     double sn, cs;
-    sincospi(2.0 * static_cast<double>(mm) * ma[a].s[dim], &sn, &cs);
+    sincospi(2.0 * static_cast<double>(mm) * (dim == 0 ? at.x : (dim == 1 ? at.y : at.z)), &sn, &cs);
     if (dim == 0)
-      ex[a * nx + mm] = make_double2(cs, sn);
+      ex[a * nx + mm] = make_double2(at.w * cs, at.w * sn);
     else if (dim == 1)
     {
       ey[a * ny + kym + mm] = make_double2(cs, sn);
       ey[a * ny + kym - mm] = make_double2(cs, -sn);
     }
     else
-    {
-      ez[a * nz + kzm + mm] = make_double2(cs, sn);
-      ez[a * nz + kzm - mm] = make_double2(cs, -sn);
-    }
+      ez[a * nz + mm] = make_double2(cs, sn);
   }
   __syncthreads();
-  for (int idx = threadIdx.x; idx < d.w * na; idx += blockDim.x)
-  {
-    const int j = idx / na, a = idx - j * na;
-    const char2 pq = pairs[d.z + j];
-    const double2 x = ex[a * nx + pq.x], y = ey[a * ny + kym + pq.y];
-    const double w = ma[a].w;
-    wxy[j * atom_stride + a] = make_double2(w * (x.x * y.x - x.y * y.y), w * (x.x * y.y + x.y * y.x));
-  }
-  __syncthreads();
-  const double2* S = sk + (static_cast<long long>(cur[sys]) * n_systems + sys) * nk;
-  double2* T = sk + (static_cast<long long>(1 - cur[sys]) * n_systems + sys) * nk;
+  const int groups = (nz + kBatchM - 1) / kBatchM;
   double e = 0.0;
-#pragma unroll
-  for (int r = 0; r < kBatchKPerThread; ++r)
+  for (int item = blockIdx.x * kThreads + threadIdx.x; item < n_runs * groups; item += gridDim.x * kThreads)
   {
-    const int k = d.x + r * kThreads + static_cast<int>(threadIdx.x);
-    if (k >= d.y) continue;
-    const int info = kinfo[k];
-    const double2* w = wxy + ((info >> 8) - d.z) * atom_stride;
-    const double2* z = ez + (info & 0xff) - 128 + kzm;
-    double2 dr = make_double2(0.0, 0.0);
+    const int g = item / n_runs, r = item - g * n_runs, m0 = g * kBatchM;
+    const int4 run = runs[r];
+    const int lo = static_cast<short>(run.w & 0xffff), hi = run.w >> 16;
+    if (m0 > max(-lo, hi)) continue;
+    double pc[kBatchM], qs[kBatchM], ps[kBatchM], qc[kBatchM];
+#pragma unroll
+    for (int m = 0; m < kBatchM; ++m) pc[m] = qs[m] = ps[m] = qc[m] = 0.0;
+#pragma unroll 1
     for (int a = 0; a < na; ++a)
     {
-      const double2 wa = w[a], za = z[a * nz];
-      dr.x = fma(wa.x, za.x, fma(-wa.y, za.y, dr.x));
-      dr.y = fma(wa.x, za.y, fma(wa.y, za.x, dr.y));
+      const double2 x = ex[a * nx + run.x], y = ey[a * ny + kym + run.y];
+      const double p = x.x * y.x - x.y * y.y, q = x.x * y.y + x.y * y.x;
+#pragma unroll
+      for (int m = 0; m < kBatchM; ++m)
+      {
+        const double2 z = ez[a * nz + min(m0 + m, kzm)];
+        pc[m] = fma(p, z.x, pc[m]);
+        qs[m] = fma(q, z.y, qs[m]);
+        ps[m] = fma(p, z.y, ps[m]);
+        qc[m] = fma(q, z.x, qc[m]);
+      }
     }
-    const double2 s = __ldcs(S + k);
-    e += temp[k] * (2.0 * (s.x * dr.x + s.y * dr.y) + (dr.x * dr.x + dr.y * dr.y));
-    __stcs(T + k, make_double2(s.x + dr.x, s.y + dr.y));
+#pragma unroll
+    for (int m = 0; m < kBatchM; ++m)
+    {
+      // Delta rho at kz = +m in (u, v), at kz = -m in (w, z)
+      const double u = pc[m] - qs[m], v = ps[m] + qc[m], w = pc[m] + qs[m], z = qc[m] - ps[m];
+      pc[m] = u;
+      ps[m] = v;
+      qs[m] = w;
+      qc[m] = z;
+    }
+#pragma unroll
+    for (int sign = 0; sign < 2; ++sign)
+    {
+      double2 s[kBatchM];
+      int at[kBatchM];
+#pragma unroll
+      for (int m = 0; m < kBatchM; ++m)
+      {
+        const int kz = sign == 0 ? m0 + m : -(m0 + m);
+        const bool in = kz >= lo && kz <= hi && (sign == 0 || kz != 0);
+        at[m] = in ? row_start[2 * (m0 + m) + sign] + r : -1;
+        s[m] = in ? __ldcs(S + at[m]) : make_double2(0.0, 0.0);
+      }
+#pragma unroll
+      for (int m = 0; m < kBatchM; ++m)
+        if (at[m] >= 0)
+        {
+          const double dx = sign == 0 ? pc[m] : qs[m], dy = sign == 0 ? ps[m] : qc[m];
+          e += run_temp[(2 * (m0 + m) + sign) * n_runs + r] * (2.0 * (s[m].x * dx + s[m].y * dy) + (dx * dx + dy * dy));
+          __stcs(T + at[m], make_double2(s[m].x + dx, s[m].y + dy));
+        }
+    }
   }
-  // fixed-order reduction: warps, then the block, then (the system's last block) the blocks in order
+  // fixed-order reduction: warps, then the block; ewaldBatchTotalKernel adds the blocks. (A last block per system, found
+  // with a counter, kept every block until its fence and its atomic had returned.)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) e += __shfl_down_sync(0xffffffffu, e, o);
@@ -1466,26 +1505,31 @@ __global__ void __launch_bounds__(kThreads) ewaldBatchDeltaKernel(
     double x = 0.0;
     for (int q = 0; q < kThreads / 32; ++q) x += red[q];
     partial[static_cast<long long>(sys) * gridDim.x + blockIdx.x] = x;
-    __threadfence();
-    last = atomicAdd(counter + sys, 1u) == gridDim.x - 1;
   }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  double y = 0.0;
-  for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x)
-    y += __ldcg(partial + static_cast<long long>(sys) * gridDim.x + b);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) y += __shfl_down_sync(0xffffffffu, y, o);
-  if (lane == 0) red[warp] = y;
-  __syncthreads();
-  if (threadIdx.x == 0)
-  {
-    double x = 0.0;
-    for (int q = 0; q < kThreads / 32; ++q) x += red[q];
-    result[sys] = x;
-    counter[sys] = 0u;  // ready for the next launch
-  }
+}
+
+// S(k) of one system between list order (k * stride) and its slots
+__global__ void __launch_bounds__(kThreads) ewaldBatchPermuteKernel(int64_t nk, const int* __restrict__ slot_of,
+                                                                    double2* list, int64_t stride, double2* slots,
+                                                                    int to_slots)
+{
+  const int64_t k = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x;
+  if (k >= nk) return;
+  if (to_slots)
+    slots[slot_of[k]] = list[k * stride];
+  else
+    list[k * stride] = slots[slot_of[k]];
+}
+
+// The blocks' energies of each system added in block order, into mapped host memory
+__global__ void __launch_bounds__(kThreads) ewaldBatchTotalKernel(int n, int blocks, const double* __restrict__ partial,
+                                                                  double* result)
+{
+  const int sys = blockIdx.x * kThreads + threadIdx.x;
+  if (sys >= n) return;
+  double x = 0.0;
+  for (int b = 0; b < blocks; ++b) x += partial[static_cast<long long>(sys) * blocks + b];
+  result[sys] = x;
 }
 }  // namespace
 
@@ -1500,57 +1544,57 @@ rg_status rg_ewald_batch_create(rg_ewald* e, int n_systems, rg_ewald_batch** out
   RG_CUDA(ctx, cudaSetDevice(ctx->device));
   rg_ewald_batch* b = new rg_ewald_batch();
   b->ewald = e;
+  b->ctx = e->ctx;
   b->n = n_systems;
   const int64_t nk = std::max<int64_t>(1, e->nk);
-  // k-ranges of at most kThreads * kBatchKPerThread k-vectors and kBatchPairs (kx, ky) pairs, from the k-vector list
-  std::vector<char4> kv(static_cast<size_t>(e->nk));
-  std::vector<int> kinfo(static_cast<size_t>(nk), 0);
-  std::vector<char2> pairs;
-  std::vector<int4> desc;
-  cudaError_t err = cudaSuccess;
-  if (e->nk > 0)
+  // the runs come longest first, so that the rows of large |kz| hold the first runs only
+  std::vector<int4> runs = rgd::ewaldRuns(e);
+  const int rows = 2 * (e->ff.kmax_z + 1);
+  std::vector<int> row_start(rows, 0), row_len(rows, 0), slot_of(static_cast<size_t>(nk), 0);
+  for (int pass = 0; pass < 2; ++pass)
   {
-    err = cudaMemcpyAsync(kv.data(), e->kvec, sizeof(char4) * e->nk, cudaMemcpyDeviceToHost, ctx->stream);
-    if (!err) err = cudaStreamSynchronize(ctx->stream);
+    for (size_t r = 0; r < runs.size(); ++r)
+    {
+      const int lo = static_cast<short>(runs[r].w & 0xffff), hi = runs[r].w >> 16;
+      for (int kz = lo; kz <= hi; ++kz)
+      {
+        const int row = 2 * std::abs(kz) + (kz < 0 ? 1 : 0);
+        if (pass == 0)
+          row_len[row] = static_cast<int>(r) + 1;
+        else
+          slot_of[static_cast<size_t>(runs[r].z + kz - lo)] = row_start[row] + static_cast<int>(r);
+      }
+    }
+    if (pass == 0)
+    {
+      for (int row = 1; row < rows; ++row) row_start[row] = row_start[row - 1] + row_len[row - 1];
+      b->slots = std::max(1, row_start[rows - 1] + row_len[rows - 1]);
+    }
   }
-  if (err)
-  {
-    delete b;
-    return rg::cudaFail(ctx, err, "rg_ewald_batch_create");
-  }
-  for (int64_t k = 0; k < e->nk; ++k)
-  {
-    if (k == 0 || kv[k].x != kv[k - 1].x || kv[k].y != kv[k - 1].y) pairs.push_back(make_char2(kv[k].x, kv[k].y));
-    kinfo[k] = static_cast<int>(pairs.size() - 1) * 256 + (kv[k].z + 128);
-  }
-  for (int64_t k0 = 0; k0 < e->nk;)
-  {
-    const int p0 = kinfo[k0] >> 8;
-    int64_t k1 = k0;
-    while (k1 < e->nk && k1 - k0 < kThreads * kBatchKPerThread && (kinfo[k1] >> 8) - p0 < kBatchPairs) ++k1;
-    desc.push_back(make_int4(static_cast<int>(k0), static_cast<int>(k1), p0, (kinfo[k1 - 1] >> 8) - p0 + 1));
-    k0 = k1;
-  }
-  if (desc.empty()) desc.push_back(make_int4(0, 0, 0, 0));
-  if (pairs.empty()) pairs.push_back(make_char2(0, 0));
-  b->blocks = static_cast<int>(desc.size());
-  err = cudaMalloc(reinterpret_cast<void**>(&b->desc), sizeof(int4) * desc.size());
-  if (!err) err = cudaMemcpyAsync(b->desc, desc.data(), sizeof(int4) * desc.size(), cudaMemcpyHostToDevice, ctx->stream);
-  if (!err) err = cudaMalloc(reinterpret_cast<void**>(&b->kinfo), sizeof(int) * kinfo.size());
-  if (!err) err = cudaMemcpyAsync(b->kinfo, kinfo.data(), sizeof(int) * kinfo.size(), cudaMemcpyHostToDevice, ctx->stream);
-  if (!err) err = cudaMalloc(reinterpret_cast<void**>(&b->pairs), sizeof(char2) * pairs.size());
-  if (!err) err = cudaMemcpyAsync(b->pairs, pairs.data(), sizeof(char2) * pairs.size(), cudaMemcpyHostToDevice, ctx->stream);
-  if (!err) err = cudaMalloc(reinterpret_cast<void**>(&b->sk), sizeof(double2) * 2 * n_systems * nk);
-  if (!err) err = cudaMemsetAsync(b->sk, 0, sizeof(double2) * 2 * n_systems * nk, ctx->stream);
-  if (!err) err = cudaMalloc(reinterpret_cast<void**>(&b->cur), n_systems);
-  if (!err) err = cudaMemsetAsync(b->cur, 0, n_systems, ctx->stream);
-  if (!err) err = cudaMalloc(reinterpret_cast<void**>(&b->atoms), sizeof(MovedAtom) * kBatchAtoms * n_systems);
-  if (!err) err = cudaMallocHost(reinterpret_cast<void**>(&b->atoms_host), sizeof(MovedAtom) * kBatchAtoms * n_systems);
-  if (!err) err = cudaMalloc(reinterpret_cast<void**>(&b->counts), sizeof(int) * n_systems);
-  if (!err) err = cudaMallocHost(reinterpret_cast<void**>(&b->counts_host), sizeof(int) * n_systems);
+  if (runs.empty()) runs.push_back(make_int4(0, 0, 0, 0));
+  b->n_runs = static_cast<int>(runs.size());
+  std::vector<double> run_temp;
+  cudaError_t err = rgd::ewaldRunPrefactors(e, runs, run_temp);
+  if (!err) err = cudaMalloc(reinterpret_cast<void**>(&b->run_temp), sizeof(double) * run_temp.size());
+  if (!err)
+    err = cudaMemcpyAsync(b->run_temp, run_temp.data(), sizeof(double) * run_temp.size(), cudaMemcpyHostToDevice, ctx->stream);
+  // Blocks per system: as many as there are groups of kThreads items when the systems are few; for many systems fewer, so
+  // that a block's phasor tables serve more k-vectors (about eight blocks per place on the GPU remain)
+  const int64_t items = static_cast<int64_t>(b->n_runs) * ((e->ff.kmax_z + kBatchM) / kBatchM);
+  const int64_t most = std::max<int64_t>(1, (items + kThreads - 1) / kThreads);
+  b->blocks = static_cast<int>(std::min<int64_t>(most, std::max<int64_t>(1, 24LL * e->sms / n_systems)));
+  if (!err) err = cudaMalloc(reinterpret_cast<void**>(&b->slot_of), sizeof(int) * slot_of.size());
+  if (!err) err = cudaMemcpyAsync(b->slot_of, slot_of.data(), sizeof(int) * slot_of.size(), cudaMemcpyHostToDevice, ctx->stream);
+  if (!err) err = cudaMalloc(reinterpret_cast<void**>(&b->row_start), sizeof(int) * rows);
+  if (!err) err = cudaMemcpyAsync(b->row_start, row_start.data(), sizeof(int) * rows, cudaMemcpyHostToDevice, ctx->stream);
+  if (!err) err = cudaMalloc(reinterpret_cast<void**>(&b->runs), sizeof(int4) * runs.size());
+  if (!err) err = cudaMemcpyAsync(b->runs, runs.data(), sizeof(int4) * runs.size(), cudaMemcpyHostToDevice, ctx->stream);
+  if (!err) err = cudaMalloc(reinterpret_cast<void**>(&b->sk), sizeof(double2) * 2 * n_systems * b->slots);
+  if (!err) err = cudaMemsetAsync(b->sk, 0, sizeof(double2) * 2 * n_systems * b->slots, ctx->stream);
+  const size_t upload = batchUploadBytes(n_systems, kBatchAtoms);
+  if (!err) err = cudaMalloc(reinterpret_cast<void**>(&b->upload), upload);
+  if (!err) err = cudaMallocHost(reinterpret_cast<void**>(&b->upload_host), upload);
   if (!err) err = cudaMalloc(reinterpret_cast<void**>(&b->partial), sizeof(double) * n_systems * b->blocks);
-  if (!err) err = cudaMalloc(reinterpret_cast<void**>(&b->counter), sizeof(unsigned int) * n_systems);
-  if (!err) err = cudaMemsetAsync(b->counter, 0, sizeof(unsigned int) * n_systems, ctx->stream);
   if (!err) err = cudaHostAlloc(reinterpret_cast<void**>(&b->result_host), sizeof(double) * n_systems, cudaHostAllocMapped);
   if (!err) err = cudaHostGetDevicePointer(reinterpret_cast<void**>(&b->result), b->result_host, 0);
   for (int i = 0; i < 3 && !err; ++i) err = cudaEventCreate(&b->ev[i]);
@@ -1561,7 +1605,7 @@ rg_status rg_ewald_batch_create(rg_ewald* e, int n_systems, rg_ewald_batch** out
     rg_ewald_batch_destroy(b);
     return st;
   }
-  b->cur_host.assign(n_systems, 0);
+  b->cur.assign(n_systems, 0);
   *out = b;
   return RG_OK;
 }
@@ -1569,18 +1613,15 @@ rg_status rg_ewald_batch_create(rg_ewald* e, int n_systems, rg_ewald_batch** out
 rg_status rg_ewald_batch_destroy(rg_ewald_batch* b)
 {
   if (!b) return RG_OK;
-  if (b->ewald && b->ewald->ctx) cudaStreamSynchronize(b->ewald->ctx->stream);
+  if (b->ctx) cudaStreamSynchronize(b->ctx->stream);
   cudaFree(b->sk);
-  cudaFree(b->cur);
-  cudaFree(b->atoms);
-  cudaFree(b->counts);
+  cudaFree(b->upload);
   cudaFree(b->partial);
-  cudaFree(b->counter);
-  cudaFree(b->desc);
-  cudaFree(b->kinfo);
-  cudaFree(b->pairs);
-  if (b->atoms_host) cudaFreeHost(b->atoms_host);
-  if (b->counts_host) cudaFreeHost(b->counts_host);
+  cudaFree(b->slot_of);
+  cudaFree(b->row_start);
+  cudaFree(b->runs);
+  cudaFree(b->run_temp);
+  if (b->upload_host) cudaFreeHost(b->upload_host);
   if (b->result_host) cudaFreeHost(b->result_host);
   for (cudaEvent_t ev : b->ev)
     if (ev) cudaEventDestroy(ev);
@@ -1595,16 +1636,20 @@ rg_status rg_ewald_batch_set(rg_ewald_batch* b, int system, const double* sk)
   rg_ctx* ctx = e->ctx;
   if (e->nk == 0) return RG_OK;
   RG_CUDA(ctx, cudaSetDevice(ctx->device));
-  double2* dst = b->sk + (static_cast<long long>(b->cur_host[system]) * b->n + system) * e->nk;
+  double2* dst = b->sk + (static_cast<long long>(b->cur[system]) * b->n + system) * b->slots;
+  double2* list = e->stored;  // entry 0 of each k
   if (sk)
   {
     for (int64_t i = 0; i < 2 * e->nk; ++i)
       if (!std::isfinite(sk[i])) return rg::fail(ctx, RG_ERR_NONFINITE, "rg_ewald_batch_set: NaN or infinite S(k)");
-    RG_CUDA(ctx, cudaMemcpyAsync(dst, sk, sizeof(double2) * e->nk, cudaMemcpyHostToDevice, ctx->stream));
+    void* scr = nullptr;
+    if (rg_status st = rg::scratch(ctx, kSumsSlot, sizeof(double2) * e->nk, &scr)) return st;
+    list = static_cast<double2*>(scr);
+    RG_CUDA(ctx, cudaMemcpyAsync(list, sk, sizeof(double2) * e->nk, cudaMemcpyHostToDevice, ctx->stream));
   }
-  else  // the Ewald state's stored total structure factor (entry 0 of each k)
-    RG_CUDA(ctx, cudaMemcpy2DAsync(dst, sizeof(double2), e->stored, sizeof(double2) * (1 + e->n_groups),
-                                   sizeof(double2), e->nk, cudaMemcpyDeviceToDevice, ctx->stream));
+  ewaldBatchPermuteKernel<<<static_cast<unsigned>((e->nk + kThreads - 1) / kThreads), kThreads, 0, ctx->stream>>>(
+      e->nk, b->slot_of, list, sk ? 1 : 1 + e->n_groups, dst, 1);
+  RG_CUDA(ctx, cudaGetLastError());
   RG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   return RG_OK;
 }
@@ -1616,9 +1661,14 @@ rg_status rg_ewald_batch_get(rg_ewald_batch* b, int system, int which, double* s
   rg_ctx* ctx = e->ctx;
   if (e->nk == 0) return RG_OK;
   RG_CUDA(ctx, cudaSetDevice(ctx->device));
-  const int buf = which == 0 ? b->cur_host[system] : 1 - b->cur_host[system];
-  RG_CUDA(ctx, cudaMemcpyAsync(sk, b->sk + (static_cast<long long>(buf) * b->n + system) * e->nk,
-                               sizeof(double2) * e->nk, cudaMemcpyDeviceToHost, ctx->stream));
+  const int buf = which == 0 ? b->cur[system] : 1 - b->cur[system];
+  void* scr = nullptr;
+  if (rg_status st = rg::scratch(ctx, kSumsSlot, sizeof(double2) * e->nk, &scr)) return st;
+  double2* list = static_cast<double2*>(scr);
+  ewaldBatchPermuteKernel<<<static_cast<unsigned>((e->nk + kThreads - 1) / kThreads), kThreads, 0, ctx->stream>>>(
+      e->nk, b->slot_of, list, 1, b->sk + (static_cast<long long>(buf) * b->n + system) * b->slots, 0);
+  RG_CUDA(ctx, cudaGetLastError());
+  RG_CUDA(ctx, cudaMemcpyAsync(sk, list, sizeof(double2) * e->nk, cudaMemcpyDeviceToHost, ctx->stream));
   RG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   return RG_OK;
 }
@@ -1633,25 +1683,34 @@ rg_status rg_ewald_batch_delta(rg_ewald_batch* b, const rg_atom* atoms, int max_
   // the staging buffers are free: every call ends by synchronising the stream; system s's atoms are packed at
   // s * stride (stride = max_atoms, at most kBatchAtoms)
   const int stride = std::min(max_atoms, kBatchAtoms);
+  double4* packed = reinterpret_cast<double4*>(b->upload_host);
+  int* counts = reinterpret_cast<int*>(packed + static_cast<size_t>(b->n) * stride);
   for (int s = 0; s < b->n; ++s)
   {
     if (n_new[s] < 0 || n_old[s] < 0 || n_new[s] + n_old[s] > std::min(max_atoms, kBatchAtoms))
       return rg::fail(ctx, RG_ERR_INVALID_ARGUMENT, "rg_ewald_batch_delta: at most 16 old + new atoms per system");
     const rg_atom* a = atoms + static_cast<long long>(s) * max_atoms;
     if (rg_status fs = rg::checkFinite(ctx, a, n_new[s] + n_old[s], "rg_ewald_batch_delta")) return fs;
-    // new atoms with +q, then old atoms with -q (packMoved takes the old ones first)
-    packMoved(e, a + n_new[s], n_old[s], a, n_new[s], -1.0, b->atoms_host + static_cast<long long>(s) * stride);
-    b->counts_host[s] = e->use_charge ? n_new[s] + n_old[s] : 0;
+    // new atoms with +q, old atoms with -q
+    double4* to = packed + static_cast<size_t>(s) * stride;
+    for (int i = 0; i < n_new[s] + n_old[s]; ++i)
+    {
+      const double r[3] = {a[i].x, a[i].y, a[i].z};
+      double f[3];
+      rg::matvec(e->box.ic, r, f);
+      to[i] = make_double4(f[0], f[1], f[2], (i < n_new[s] ? 1.0 : -1.0) * a[i].scaling_coulomb * a[i].charge);
+    }
+    counts[s] = e->use_charge ? n_new[s] + n_old[s] : 0;
   }
+  std::memcpy(counts + b->n, b->cur.data(), b->n);
   if (e->nk == 0 || !e->use_charge)
   {
     for (int s = 0; s < b->n; ++s) delta_fourier[s] = 0.0;
     return RG_OK;
   }
   RG_CUDA(ctx, cudaEventRecord(b->ev[0], ctx->stream));
-  RG_CUDA(ctx, cudaMemcpyAsync(b->atoms, b->atoms_host, sizeof(MovedAtom) * stride * b->n, cudaMemcpyHostToDevice,
+  RG_CUDA(ctx, cudaMemcpyAsync(b->upload, b->upload_host, batchUploadBytes(b->n, stride), cudaMemcpyHostToDevice,
                                ctx->stream));
-  RG_CUDA(ctx, cudaMemcpyAsync(b->counts, b->counts_host, sizeof(int) * b->n, cudaMemcpyHostToDevice, ctx->stream));
   const int kxm = e->ff.kmax_x, kym = e->ff.kmax_y, kzm = e->ff.kmax_z;
   const size_t shmem = batchSharedBytes(stride, kxm, kym, kzm);
   if (shmem > 200 * 1024)
@@ -1660,9 +1719,11 @@ rg_status rg_ewald_batch_delta(rg_ewald_batch* b, const rg_atom* atoms, int max_
                                     static_cast<int>(shmem)));
   dim3 grid(b->blocks, b->n);
   RG_CUDA(ctx, cudaEventRecord(b->ev[1], ctx->stream));
-  ewaldBatchDeltaKernel<<<grid, kThreads, shmem, ctx->stream>>>(b->desc, b->kinfo, b->pairs, e->nk, b->n, e->temp,
-                                                               b->sk, b->cur, b->atoms, stride, b->counts, kxm, kym,
-                                                               kzm, b->partial, b->counter, b->result);
+  ewaldBatchDeltaKernel<<<grid, kThreads, shmem, ctx->stream>>>(b->runs, b->n_runs, b->row_start, b->slots, b->n,
+                                                               b->run_temp, b->sk, b->upload, stride, kxm, kym, kzm,
+                                                               b->partial);
+  ewaldBatchTotalKernel<<<(b->n + kThreads - 1) / kThreads, kThreads, 0, ctx->stream>>>(b->n, b->blocks, b->partial,
+                                                                                      b->result);
   RG_CUDA(ctx, cudaGetLastError());
   RG_CUDA(ctx, cudaEventRecord(b->ev[2], ctx->stream));
   RG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -1683,18 +1744,9 @@ rg_status rg_ewald_batch_timing(rg_ewald_batch* b, float* upload_ms, float* kern
 rg_status rg_ewald_batch_accept(rg_ewald_batch* b, const uint8_t* accept)
 {
   if (!b || !accept) return RG_ERR_INVALID_ARGUMENT;
-  rg_ctx* ctx = b->ewald->ctx;
-  bool any = false;
+  // the flags travel with the next call's atoms
   for (int s = 0; s < b->n; ++s)
-    if (accept[s])
-    {
-      b->cur_host[s] ^= 1;
-      any = true;
-    }
-  if (!any) return RG_OK;
-  RG_CUDA(ctx, cudaSetDevice(ctx->device));
-  RG_CUDA(ctx, cudaMemcpyAsync(b->cur, b->cur_host.data(), b->n, cudaMemcpyHostToDevice, ctx->stream));
-  RG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    if (accept[s]) b->cur[s] ^= 1;
   return RG_OK;
 }
 }  // extern "C"
