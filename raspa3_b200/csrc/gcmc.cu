@@ -10,18 +10,28 @@
 // with the framework-molecule energy from the tricubic grids, the molecule-molecule Lennard-Jones and real-space Ewald
 // pair sums, and the Ewald Fourier energy change on the chain's own structure factors (which include the framework).
 //
-// Work split inside a CTA of 128 threads: the external energy of a set of trial atoms is one warp's job (lanes own the
-// atoms' grid interpolations, then stride over the partner atoms; warp-shuffle reduction), four warps take four trial
-// sets at a time; the Ewald change is spread over all threads by k-vector, from per-atom phase tables built in shared
-// memory (e^{i 2 pi m s_d}, m = 0..kmax). All sums are in a fixed order (deterministic); arithmetic is FP64. Random
-// numbers come from a counter-based generator (Philox-4x32-10, Salmon et al., SC'11) keyed by seed and chain and
-// counted by (move, slot), so any thread can draw any move's numbers without shared state.
+// Work split inside a CTA of 128 threads. A move is a chain of short dependent steps, so each step is spread over the
+// CTA: a set's framework energy takes one lane per corner of each (atom, grid) interpolation; its molecule-molecule
+// pairs take a warp per set, which tests all distances and lists the pairs within a cutoff, and evaluates the listed
+// pairs of all its sets together; the exponentials of a selection take one lane per trial; the orientations of an
+// insertion are drawn by another warp than its first beads; the Ewald change takes one thread per run of kz of a
+// (kx, ky) and three values of |kz|, both signs from the same four sums, from phasor tables in shared memory. The chain's
+// structure factors (and their change), its molecule count, energy and statistics stay in shared memory for the whole
+// launch where they fit. All sums are in a fixed order (deterministic); arithmetic is FP64. Random numbers come from a
+// counter-based generator (Philox-4x32-10, Salmon et al., SC'11) keyed by seed and chain and counted by (move, slot),
+// so any thread can draw any move's numbers without shared state.
+//
+// What bounds it: the latency of a move's chain of steps, with four CTAs per SM to fill the gaps (44 % of the issue slots
+// used), and before that the code's own size: at 211 KB for four chains at different places of it, waiting for the next
+// instruction was two fifths of all stalls; the kernel is kept at 77 KB. 200 moves of 1,184 chains at a loading of about
+// eight CO2 (kmax 8): 21.5 ms with all of S in global memory and a thread per k-vector, pair and trial, now 6.1 ms.
 #include <cmath>
 #include <cstring>
 #include <vector>
 
 #include "common.cuh"
 #include "energy.cuh"
+#include "fastmath.cuh"
 #include "rng.cuh"
 
 namespace
@@ -31,6 +41,10 @@ constexpr int kWarps = kThreads / 32;
 constexpr int kMaxAtoms = 8;     // atoms per molecule
 constexpr int kMaxTrials = 16;   // first-bead positions / orientations per step
 constexpr int kMaxK = 16;        // kmax per axis + 1 supported by the phase tables
+constexpr int kEwaldM = 3;       // values of |kz| of one thread's share of a run
+constexpr size_t kSharedPerCta = 50 * 1024;  // dynamic shared memory with which four CTAs fit on an SM
+constexpr int kPairRoom = 64;    // listed pairs of a warp (evaluated 32 at a time)
+constexpr int kSetsPerWarp = kMaxTrials / kWarps;
 
 struct Component
 {
@@ -61,8 +75,11 @@ struct Params
   int use_ewald;
   int64_t nk;
   int kmax[3];
-  const char4* kvec;
-  const double* temp;
+  // runs of consecutive kz of one (kx, ky): {kx, ky, first k, (first kz, last kz) as shorts}, and the prefactor of the
+  // k-vector with kz = +m, -m of run r at [(2 m + (sign < 0)) n_runs + r] (0: not in the run)
+  int n_runs;
+  const int4* runs;
+  const double* run_temp;
   unsigned long long seed;
   // learned first-bead proposal (null: uniform): inclusive cumulative cell probabilities and the density relative to
   // uniform, over G^3 cells of the unit cell; the simulation box is rep[0] x rep[1] x rep[2] unit cells
@@ -84,8 +101,20 @@ struct Params
 
 constexpr int kStats = 24;  // attempted[4], accepted[4], sum_n, sum_n2, sum_energy, samples, block_n[5] (sums), block_cnt
 
-using rgd::philox;
-using rgd::uniform2;
+// The kernel's code has to stay small: four chains of an SM are at different places of it, and fetching instructions was
+// what held the kernel (211 KB of code: 6.3 of 16.4 cycles per instruction waiting for the next one). So each phase
+// stands once in the move's loop, and what several places call stays a function.
+__device__ __noinline__ double2 uniform2(unsigned long long seed, int stream, long long move, uint32_t slot)
+{
+  uint32_t c[4] = {slot, static_cast<uint32_t>(move), static_cast<uint32_t>(move >> 32), static_cast<uint32_t>(stream)};
+  uint32_t k0 = static_cast<uint32_t>(seed), k1 = static_cast<uint32_t>(seed >> 32);
+#pragma unroll 2
+  for (int r = 0; r < 10; ++r) rgd::philoxRound(c, k0, k1);
+  return rgd::uniformsOf(c);
+}
+__device__ __noinline__ double expCall(double x) { return exp(x); }
+__device__ __noinline__ double erfcCall(double x) { return erfc(x); }
+__device__ __noinline__ void sincospiCall(double x, double* sn, double* cs) { sincospi(x, sn, cs); }
 
 // random slots of one move
 enum Slot
@@ -101,8 +130,11 @@ enum Slot
 __device__ __forceinline__ void rotationFromUniforms(double u1, double u2, double u3, double R[3][3])
 {
   // uniform unit quaternion (Shoemake) -> rotation matrix
-  const double x = sqrt(1 - u1) * sinpi(2 * u2), y = sqrt(1 - u1) * cospi(2 * u2);
-  const double z = sqrt(u1) * sinpi(2 * u3), w = sqrt(u1) * cospi(2 * u3);
+  double s2, c2, s3, c3;
+  sincospiCall(2 * u2, &s2, &c2);
+  sincospiCall(2 * u3, &s3, &c3);
+  const double a = sqrt(1 - u1), b = sqrt(u1);
+  const double x = a * s2, y = a * c2, z = b * s3, w = b * c3;
   R[0][0] = 1 - 2 * (y * y + z * z);
   R[0][1] = 2 * (x * y - z * w);
   R[0][2] = 2 * (x * z + y * w);
@@ -114,211 +146,396 @@ __device__ __forceinline__ void rotationFromUniforms(double u1, double u2, doubl
   R[2][2] = 1 - 2 * (x * x + y * y);
 }
 
-struct Shared
+// One pair of component atoms at full scaling: 4 eps, 1 / sigma^2, shift (0 without a Lennard-Jones term), C q_A q_B
+struct PairTerm
 {
-  double trial[kMaxTrials][kMaxAtoms][3];  // positions of the trial sets
-  double setE[kMaxTrials];
-  int setOv[kMaxTrials];
-  double logq[kMaxTrials];
-  double newPos[kMaxAtoms][3];
-  double oldPos[kMaxAtoms][3];
-  double red[kWarps];
-  double u[8];
-  int ints[8];
-  double dbl[8];
+  double eps4, inv_sig2, shift, qq;
 };
 
-// External energy (framework grids + other molecules) of `count` atoms at pos[], component atom indices atomIdx[],
-// excluding molecule slot `skip`; evaluated by one warp. Returns the energy; *overlap set if the set overlaps.
-template <bool QUINTIC>  // the system's grids: triquintic (27 values per point) or tricubic (8)
-__device__ double warpExternal(const Params& p, int chain, int n, const double (*pos)[3], const int* atomIdx,
-                               int count, int skip, int* overlap)
+struct Shared
 {
-  const int lane = threadIdx.x & 31;
-  double e = 0.0;
-  int ov = 0;
-  const Component& c = p.comp;
-  // framework part: one lane per atom
-  if (lane < count)
-  {
-    const int ai = atomIdx[lane];
-    const double* g = p.vdw_grid[ai];
-    if (g)
-    {
-      rgd::Grid gg = p.grid;
-      gg.data = g;
-      const double v = QUINTIC ? rgd::interpolateQuintic(gg, pos[lane][0], pos[lane][1], pos[lane][2], nullptr)
-                               : rgd::interpolate(gg, pos[lane][0], pos[lane][1], pos[lane][2]);
-      if (v > p.ff.overlap) ov = 1;
-      e += v;
-      if (p.ff.use_charge && p.ewald_grid)
-      {
-        gg.data = p.ewald_grid;
-        e += c.charges[ai] * (QUINTIC ? rgd::interpolateQuintic(gg, pos[lane][0], pos[lane][1], pos[lane][2], nullptr)
-                                      : rgd::interpolate(gg, pos[lane][0], pos[lane][1], pos[lane][2]));
-      }
-    }
-  }
-  // molecule-molecule part: lanes stride over partner atoms of the other molecules
-  const int na = c.n_atoms;
-  const double4* cpos = p.pos + static_cast<long long>(chain) * p.capacity * na;
-  const int total = n * na;
-  for (int q = lane; q < total; q += 32)
-  {
-    const int m = q / na, bj = q - m * na;
-    if (m == skip) continue;
-    const double4 B = cpos[q];
-    const int tB = c.types[bj];
-    const double qB = c.charges[bj];
-    for (int i = 0; i < count; ++i)
-    {
-      const int ai = atomIdx[i];
-      double dx = B.x - pos[i][0], dy = B.y - pos[i][1], dz = B.z - pos[i][2];
-      rgd::pbc(p.box, dx, dy, dz);
-      const double rr = dx * dx + dy * dy + dz * dz;
-      if (rr < p.rcv_mol2)
-      {
-        const double2 f = rgd::pairVDW(p.ff, 1.0, 1.0, rr, tB, c.types[ai]);
-        if (f.x > p.ff.overlap) ov = 1;
-        e += f.x;
-      }
-      if (p.ff.use_charge && rr < p.rcc2) e += rgd::pairCoulomb(p.ff, 1.0, 1.0, sqrt(rr), qB, c.charges[ai]).x;
-    }
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
-  {
-    e += __shfl_down_sync(0xffffffffu, e, o);
-    ov |= __shfl_down_sync(0xffffffffu, ov, o);
-  }
-  *overlap = __shfl_sync(0xffffffffu, ov, 0);
-  return __shfl_sync(0xffffffffu, e, 0);
+  double pairE[kMaxTrials];  // per set (or half set) of evaluateSets: the molecule-molecule energy, and an overlap
+  int pairOv[kMaxTrials];
+  double logq[kMaxTrials];
+  double red[kWarps];
+  double pair_rr[kWarps][kPairRoom];
+  int pair_code[kWarps][kPairRoom];  // set of the warp << 8 | component atom << 4 | partner atom
+  int list[kMaxAtoms];               // component atoms of the sets
+  int n;
+  int sel;
+  double W, E;
+  double energy;
+  double stats[24];
+};
+
+// Dynamic shared memory: per trial and component atom the position and (orientations) the offset from the first bead,
+// the framework energies of a set's atoms, the pair table, the phasor tables of the moved atoms, and (SMEM) the chain's
+// structure factors and their change.
+struct Dyn
+{
+  double* trial;    // [kMaxTrials][na][3]
+  double* rel;      // [kMaxTrials][na][3]
+  double* gridE;    // [kMaxTrials][na][2]
+  PairTerm* pair;   // [na][na]
+  int* gridOv;      // [kMaxTrials][na]
+  double2* ex;      // [2 na][kx + 1], weighted by the signed charge
+  double2* ey;      // [2 na][2 ky + 1]
+  double2* ez;      // [2 na][kz + 1]
+  double2* S;       // [nk]
+  double2* D;       // [nk]
+};
+__host__ __device__ inline size_t dynFixedBytes(int na, const int* kmax, bool ewald)
+{
+  size_t b = sizeof(double) * kMaxTrials * na * 8 + sizeof(PairTerm) * na * na + ((sizeof(int) * kMaxTrials * na + 15) & ~size_t(15));
+  if (ewald) b += sizeof(double2) * 2 * na * ((kmax[0] + 1) + (2 * kmax[1] + 1) + (kmax[2] + 1));
+  return b;
+}
+__device__ __forceinline__ Dyn dynOf(const Params& p)
+{
+  extern __shared__ __align__(16) unsigned char dynSmem[];
+  const int na = p.comp.n_atoms;
+  Dyn d;
+  d.trial = reinterpret_cast<double*>(dynSmem);
+  d.rel = d.trial + kMaxTrials * na * 3;
+  d.gridE = d.rel + kMaxTrials * na * 3;
+  d.pair = reinterpret_cast<PairTerm*>(d.gridE + kMaxTrials * na * 2);
+  d.gridOv = reinterpret_cast<int*>(d.pair + na * na);
+  d.ex = reinterpret_cast<double2*>(reinterpret_cast<unsigned char*>(d.gridOv) + ((sizeof(int) * kMaxTrials * na + 15) & ~size_t(15)));
+  d.ey = d.ex + 2 * na * (p.kmax[0] + 1);
+  d.ez = d.ey + 2 * na * (2 * p.kmax[1] + 1);
+  d.S = d.ez + 2 * na * (p.kmax[2] + 1);
+  d.D = d.S + p.nk;
+  return d;
 }
 
-// Ewald Fourier energy change of replacing the old atoms by the new ones (either may be absent); leaves the change of
-// the structure factors in dsk. Block-wide; returns the energy on every thread.
-__device__ double blockEwaldDelta(const Params& p, int chain, const double (*newPos)[3], int nNew,
-                                  const double (*oldPos)[3], int nOld, double2* tab, double* red)
+// Energy of one pair at full scaling: Lennard-Jones (potentials/pair_vdw.ixx:85-101) within its cutoff, whose overlap is
+// tested, and real-space Ewald (pair_coulomb.ixx:51-77) within its own
+__device__ __forceinline__ double pairEnergy(const Params& p, const PairTerm& t, double rr, int* ov)
 {
-  const Component& c = p.comp;
-  const int nAt = nNew + nOld;
-  const int kx1 = p.kmax[0] + 1, ky1 = p.kmax[1] + 1, kz1 = p.kmax[2] + 1;
-  const int stride = kx1 + ky1 + kz1;
-  // phase tables e^{i 2 pi m s_d}
-  for (int idx = threadIdx.x; idx < nAt * stride; idx += blockDim.x)
+  double e = 0.0;
+  if (rr < p.rcv_mol2)
   {
-    const int a = idx / stride, m = idx - a * stride;
-    const double* r = a < nNew ? newPos[a] : oldPos[a - nNew];
-    const int d = m < kx1 ? 0 : (m < kx1 + ky1 ? 1 : 2);
-    const int mm = d == 0 ? m : (d == 1 ? m - kx1 : m - kx1 - ky1);
-    const double s = p.box.ic[0][d] * r[0] + p.box.ic[1][d] * r[1] + p.box.ic[2][d] * r[2];
-    double sn, cs;
-    sincospi(2.0 * static_cast<double>(mm) * s, &sn, &cs);
-    tab[idx] = make_double2(cs, sn);
+    const double x = rr * t.inv_sig2;
+    const double i3 = rgd::rcpHouseholder(x * x * x);
+    e = t.eps4 * (i3 * (i3 - 1.0)) - t.shift;
+    if (e > p.ff.overlap) *ov = 1;
+  }
+  if (p.ff.use_charge && rr < p.rcc2)
+  {
+    const double invr = rgd::rsqrtHouseholder(rr), ar = p.ff.alpha * (rr * invr);
+    const double ec = ar < rgd::kErfcxMax ? rgd::erfcFromExp64<false>(ar, expCall(-ar * ar)) : erfcCall(ar);
+    e += t.qq * ec * invr;
+  }
+  return e;
+}
+
+// Round to nearest for |x| < 2^51, on the FP64 pipe (a tie goes to the even number; either gives the same distance)
+__device__ __forceinline__ double nearest(double x) { return (x + 6755399441055744.0) - 6755399441055744.0; }
+
+// a / n for 0 <= a < 2^21 and small n, from the FP32 reciprocal of n (off by a 2^-22.5 of the quotient, below 1 / (2 n))
+constexpr int kDivideSmall = 1 << 21;
+__device__ __forceinline__ int divideSmall(int a, float inv) { return static_cast<int>((static_cast<float>(a) + 0.5f) * inv); }
+
+// External energies (framework grids + other molecules) of `ns` sets of the `cnt` component atoms sh.list, at
+// d.trial[set][atom], without molecule `skip`: left in sh.pairE, d.gridE and their overlap flags for setEnergy. Two sets
+// (old and new positions) are halved between the warps. Block-wide; ends with a barrier.
+__device__ __forceinline__ int halvesOf(int ns) { return 2 * ns <= kWarps ? 2 : 1; }
+template <bool QUINTIC>  // the system's grids: triquintic (27 values per point) or tricubic (8)
+__device__ __forceinline__ void evaluateSets(const Params& p, Shared& sh, const Dyn& d, const double4* cpos, int n, int ns,
+                                             int cnt, int skip)
+{
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int na = p.comp.n_atoms;
+  // framework: lanes of a group of 8 take the corners of one (set, atom, grid); triquintic grids one lane each
+  constexpr int kCorners = QUINTIC ? 1 : 8;
+  const int tasks = ns * cnt * 2 * kCorners;
+  const float inv_cnt = 1.0f / static_cast<float>(cnt), inv_na = 1.0f / static_cast<float>(na);
+#pragma unroll 1
+  for (int base = 32 * warp; base < tasks; base += kThreads)
+  {
+    const int idx = base + lane;
+    const int item = idx / kCorners, g = item & 1, sj = item >> 1;
+    double v = 0.0;
+    int ai = 0;
+    if (idx < tasks)
+    {
+      const int s = divideSmall(sj, inv_cnt);
+      ai = sh.list[sj - s * cnt];
+      rgd::Grid gg = p.grid;
+      gg.data = p.vdw_grid[ai];
+      if (g == 1 && gg.data) gg.data = p.ff.use_charge ? p.ewald_grid : nullptr;
+      if (gg.data)
+      {
+        const double* r = d.trial + 3 * (s * na + ai);
+        if constexpr (QUINTIC)
+          v = rgd::interpolateQuintic(gg, r[0], r[1], r[2], nullptr);
+        else
+          v = rgd::interpolateLaneCorner(gg, r[0], r[1], r[2], idx & 7);
+      }
+    }
+    if constexpr (!QUINTIC)
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (idx < tasks && (QUINTIC || (idx & 7) == 0))
+    {
+      if (g == 0) d.gridOv[sj] = v > p.ff.overlap ? 1 : 0;
+      d.gridE[item] = g == 0 ? v : p.comp.charges[ai] * v;
+    }
+  }
+  // molecule-molecule pairs: warp w takes (half) sets w, w + kWarps, ...
+  const double reach2 = p.ff.use_charge ? fmax(p.rcv_mol2, p.rcc2) : p.rcv_mol2;
+  double e[kSetsPerWarp];
+  int ov = 0;  // bit q: an overlap in the warp's q-th set
+#pragma unroll
+  for (int q = 0; q < kSetsPerWarp; ++q) e[q] = 0.0;
+  double* rrs = sh.pair_rr[warp];
+  int* codes = sh.pair_code[warp];
+  int listed = 0;
+  // one loop over the distance tests of all the warp's sets, whose last turn only evaluates what is still listed
+  const int halves = halvesOf(ns), nv = ns * halves;
+  const int total = n * na * cnt, length = (total + halves - 1) / halves;
+  const int rounds = (length + 31) / 32;  // of one (half) set
+  const int turns = warp < nv ? (nv - warp + kWarps - 1) / kWarps * rounds : 0;
+  int q = 0, round = 0;
+#pragma unroll 1
+  for (int turn = 0; turn <= turns; ++turn)
+  {
+    const bool testing = turn < turns;
+    if (testing)
+    {
+      const int v = warp + q * kWarps, half = halves == 2 ? v & 1 : 0, s = halves == 2 ? v >> 1 : v;
+      const int t = half * length + 32 * round + lane;
+      bool in = false;
+      double rr = 0.0;
+      int code = 0;
+      if (32 * round + lane < length && t < total)
+      {
+        // t runs over partner atoms, and over the set's atoms within a partner
+        const int b = total < kDivideSmall ? divideSmall(t, inv_cnt) : t / cnt, j = t - b * cnt;
+        const int m = total < kDivideSmall ? divideSmall(b, inv_na) : b / na;
+        if (m != skip)
+        {
+          const int ai = sh.list[j];
+          const double4 B = cpos[b];
+          const double* r = d.trial + 3 * (s * na + ai);
+          double dx = B.x - r[0], dy = B.y - r[1], dz = B.z - r[2];
+          if (!p.box.triclinic)
+          {
+            dx -= nearest(dx * p.box.ic[0][0]) * p.box.c[0][0];
+            dy -= nearest(dy * p.box.ic[1][1]) * p.box.c[1][1];
+            dz -= nearest(dz * p.box.ic[2][2]) * p.box.c[2][2];
+          }
+          else
+            rgd::pbc(p.box, dx, dy, dz);
+          rr = dx * dx + dy * dy + dz * dz;
+          in = rr < reach2;
+          code = q << 8 | ai << 4 | (b - m * na);
+        }
+      }
+      const unsigned ballot = __ballot_sync(0xffffffffu, in);
+      if (in)
+      {
+        const int at = listed + __popc(ballot & ((1u << lane) - 1u));
+        rrs[at] = rr;
+        codes[at] = code;
+      }
+      listed += __popc(ballot);
+      if (++round == rounds)
+      {
+        round = 0;
+        ++q;
+      }
+    }
+    const int count = listed >= 32 ? 32 : (testing ? 0 : listed);
+    if (count == 0) continue;
+    listed -= count;  // the last ones listed; the others stay
+    __syncwarp();
+    if (lane < count)
+    {
+      const int code = codes[listed + lane];
+      int o = 0;
+      const double x = pairEnergy(p, d.pair[((code >> 4) & 15) * na + (code & 15)], rrs[listed + lane], &o);
+      ov |= o << (code >> 8);
+#pragma unroll
+      for (int u = 0; u < kSetsPerWarp; ++u)
+        if (code >> 8 == u) e[u] += x;
+    }
+    __syncwarp();
+  }
+  ov = __reduce_or_sync(0xffffffffu, ov);
+#pragma unroll
+  for (int u = 0; u < kSetsPerWarp; ++u)
+  {
+    const int v = warp + u * kWarps;
+    if (v >= nv) break;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) e[u] += __shfl_down_sync(0xffffffffu, e[u], o);
+    if (lane == 0)
+    {
+      sh.pairE[v] = e[u];
+      sh.pairOv[v] = (ov >> u) & 1;
+    }
   }
   __syncthreads();
-  const double2* S = p.sk + static_cast<long long>(chain) * p.nk;
-  double2* D = p.dsk + static_cast<long long>(chain) * p.nk;
-  double e = 0.0;
-  for (long long k = threadIdx.x; k < p.nk; k += blockDim.x)
+}
+
+// The energy of set s of the last evaluateSets, and whether it overlaps
+__device__ __forceinline__ double setEnergy(const Shared& sh, const Dyn& d, int ns, int cnt, int s, int* ov)
+{
+  const int halves = halvesOf(ns);
+  double e = sh.pairE[s * halves];
+  int o = sh.pairOv[s * halves];
+  if (halves == 2)
   {
-    const char4 kv = p.kvec[k];
-    const int ay = abs(kv.y), az = abs(kv.z);
-    const double sy = kv.y < 0 ? -1.0 : 1.0, sz = kv.z < 0 ? -1.0 : 1.0;
-    double2 d = make_double2(0.0, 0.0);
+    e += sh.pairE[2 * s + 1];
+    o |= sh.pairOv[2 * s + 1];
+  }
+#pragma unroll 1
+  for (int j = 0; j < cnt; ++j)
+  {
+    const double2 g = reinterpret_cast<const double2*>(d.gridE)[s * cnt + j];
+    e += g.x + g.y;
+    o |= d.gridOv[s * cnt + j];
+  }
+  *ov = o;
+  return e;
+}
+
+// Ewald Fourier energy change of the moved atoms: `nNew` atoms of set newSet with their charges, `nOld` of set oldSet
+// with the opposite ones; leaves the change of the structure factors in D. Block-wide; returns the energy on every
+// thread. P = w e^{2 pi i (kx s_x + ky s_y)} = (p, q) and (c, s) = e^{2 pi i m s_z} give kz = m as (pc - qs, ps + qc)
+// and kz = -m as (pc + qs, qc - ps): four FMAs per atom for two k-vectors.
+__device__ __forceinline__ double blockEwaldDelta(const Params& p, Shared& sh, const Dyn& d, const double2* S, double2* D, int newSet,
+                                  int nNew, int oldSet, int nOld)
+{
+  const Component& c = p.comp;
+  const int na = c.n_atoms, nAt = nNew + nOld;
+  const int nx = p.kmax[0] + 1, ny = 2 * p.kmax[1] + 1, nz = p.kmax[2] + 1;
+  const int per = nx + (p.kmax[1] + 1) + nz;
+#pragma unroll 1
+  for (int idx = threadIdx.x; idx < nAt * per; idx += kThreads)
+  {
+    const int a = idx / per, m = idx - a * per;
+    const int ai = a < nNew ? a : a - nNew;
+    const double* r = d.trial + 3 * ((a < nNew ? newSet : oldSet) * na + ai);
+    const int dim = m < nx ? 0 : (m < nx + p.kmax[1] + 1 ? 1 : 2);
+    const int mm = dim == 0 ? m : (dim == 1 ? m - nx : m - nx - (p.kmax[1] + 1));
+    const double s = p.box.ic[0][dim] * r[0] + p.box.ic[1][dim] * r[1] + p.box.ic[2][dim] * r[2];
+    double sn, cs;
+    sincospiCall(2.0 * static_cast<double>(mm) * s, &sn, &cs);
+    if (dim == 0)
+    {
+      const double w = a < nNew ? c.charges[ai] : -c.charges[ai];
+      d.ex[a * nx + mm] = make_double2(w * cs, w * sn);
+    }
+    else if (dim == 1)
+    {
+      d.ey[a * ny + p.kmax[1] + mm] = make_double2(cs, sn);
+      d.ey[a * ny + p.kmax[1] - mm] = make_double2(cs, -sn);
+    }
+    else
+      d.ez[a * nz + mm] = make_double2(cs, sn);
+  }
+  __syncthreads();
+  const int groups = (nz + kEwaldM - 1) / kEwaldM;
+  double e = 0.0;
+#pragma unroll 1
+  for (int item = threadIdx.x; item < p.n_runs * groups; item += kThreads)
+  {
+    const int g = item / p.n_runs, run_at = item - g * p.n_runs, m0 = g * kEwaldM;
+    const int4 run = p.runs[run_at];
+    const int lo = static_cast<short>(run.w & 0xffff), hi = run.w >> 16;
+    if (m0 > max(-lo, hi)) continue;
+    double pc[kEwaldM], qs[kEwaldM], ps[kEwaldM], qc[kEwaldM];
+#pragma unroll
+    for (int m = 0; m < kEwaldM; ++m) pc[m] = qs[m] = ps[m] = qc[m] = 0.0;
+#pragma unroll 1
     for (int a = 0; a < nAt; ++a)
     {
-      const double2* t = tab + a * stride;
-      const double2 ex = t[kv.x];
-      double2 ey = t[kx1 + ay], ez = t[kx1 + ky1 + az];
-      ey.y *= sy;
-      ez.y *= sz;
-      const double2 xy = make_double2(ex.x * ey.x - ex.y * ey.y, ex.x * ey.y + ex.y * ey.x);
-      const double2 ph = make_double2(xy.x * ez.x - xy.y * ez.y, xy.x * ez.y + xy.y * ez.x);
-      const double w = a < nNew ? c.charges[a] : -c.charges[a - nNew];
-      d.x += w * ph.x;
-      d.y += w * ph.y;
+      const double2 x = d.ex[a * nx + run.x], y = d.ey[a * ny + p.kmax[1] + run.y];
+      const double pp = x.x * y.x - x.y * y.y, qq = x.x * y.y + x.y * y.x;
+#pragma unroll
+      for (int m = 0; m < kEwaldM; ++m)
+      {
+        const double2 z = d.ez[a * nz + min(m0 + m, nz - 1)];
+        pc[m] = fma(pp, z.x, pc[m]);
+        qs[m] = fma(qq, z.y, qs[m]);
+        ps[m] = fma(pp, z.y, ps[m]);
+        qc[m] = fma(qq, z.x, qc[m]);
+      }
     }
-    const double2 s = S[k];
-    e += p.temp[k] * (2.0 * (s.x * d.x + s.y * d.y) + (d.x * d.x + d.y * d.y));
-    D[k] = d;
+    const int first = run.z - lo;  // index of kz = 0, were it in the run
+#pragma unroll
+    for (int m = 0; m < kEwaldM; ++m)
+#pragma unroll
+      for (int sign = 0; sign < 2; ++sign)
+      {
+        const int kz = sign == 0 ? m0 + m : -(m0 + m);
+        if (kz < lo || kz > hi || (sign == 1 && kz == 0)) continue;
+        const double2 dr = sign == 0 ? make_double2(pc[m] - qs[m], ps[m] + qc[m])
+                                     : make_double2(pc[m] + qs[m], qc[m] - ps[m]);
+        const double2 s = S[first + kz];
+        e += p.run_temp[(2 * (m0 + m) + sign) * p.n_runs + run_at] *
+             (2.0 * (s.x * dr.x + s.y * dr.y) + (dr.x * dr.x + dr.y * dr.y));
+        D[first + kz] = dr;
+      }
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) e += __shfl_down_sync(0xffffffffu, e, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = e;
+  if ((threadIdx.x & 31) == 0) sh.red[threadIdx.x >> 5] = e;
   __syncthreads();
   double tot = 0.0;
-  for (int w = 0; w < kWarps; ++w) tot += red[w];
-  __syncthreads();
+  for (int w = 0; w < kWarps; ++w) tot += sh.red[w];
   return tot;
 }
 
-__device__ void blockAcceptEwald(const Params& p, int chain)
+__device__ __forceinline__ void blockAcceptEwald(const Params& p, double2* S, const double2* D)
 {
-  double2* S = p.sk + static_cast<long long>(chain) * p.nk;
-  const double2* D = p.dsk + static_cast<long long>(chain) * p.nk;
-  for (long long k = threadIdx.x; k < p.nk; k += blockDim.x)
+#pragma unroll 2
+  for (int k = threadIdx.x; k < p.nk; k += kThreads)
   {
-    const double2 d = D[k];
-    S[k].x += d.x;
-    S[k].y += d.y;
+    const double2 d = D[k], s = S[k];
+    S[k] = make_double2(s.x + d.x, s.y + d.y);
   }
 }
 
-// CBMC::selectTrialPosition (cbmc/util.cpp:14-47) over the non-overlapping trials; returns the chosen trial index and
-// the Rosenbluth weight sum_i exp(-beta U_i) / k, or -1 if every trial overlaps.
-// With a proposal density, trial t's log weight is -beta U_t - log q_t (logq may be null: uniform, q = 1).
-__device__ int selectTrial(const double* E, const int* ov, const double* logq, int k, double beta, double u, double* W)
+// CBMC::selectTrialPosition (cbmc/util.cpp:14-47) over the non-overlapping trials, by one warp with a lane per trial:
+// the chosen trial (the first whose running sum of weights reaches u times their total, else the last) and the
+// Rosenbluth weight sum_i exp(-beta U_i) / k, or -1 if every trial overlaps (`in`: the lane holds one that does not). The
+// log weight of trial t is -beta U_t - log q_t (logq 0: uniform, q = 1).
+__device__ __forceinline__ int selectTrial(double E, bool in, double logq, int k, double beta, double u, double* W)
 {
-  double largest = -1e300;
-  bool any = false;
-  for (int t = 0; t < k; ++t)
-    if (!ov[t])
-    {
-      largest = fmax(largest, -beta * E[t] - (logq ? logq[t] : 0.0));
-      any = true;
-    }
-  if (!any)
+  const int lane = threadIdx.x & 31;
+  const unsigned mask = __ballot_sync(0xffffffffu, in);
+  if (mask == 0u)
   {
     *W = 0.0;
     return -1;
   }
-  double sum = 0.0, w = 0.0;
-  for (int t = 0; t < k; ++t)
-    if (!ov[t])
-    {
-      const double lw = -beta * E[t] - (logq ? logq[t] : 0.0);
-      sum += exp(lw - largest);
-      w += exp(lw);
-    }
-  *W = w / static_cast<double>(k);
-  const double ws = u * sum;
-  int first = -1, selected = -1;
-  double cumw = 0.0;
-  for (int t = 0; t < k; ++t)
+  const double lw = in ? -beta * E - logq : -1e300;
+  double largest = lw;
+#pragma unroll
+  for (int o = kMaxTrials / 2; o > 0; o >>= 1) largest = fmax(largest, __shfl_xor_sync(0xffffffffu, largest, o));
+  largest = __shfl_sync(0xffffffffu, largest, 0);
+  double run = in ? expCall(lw - largest) : 0.0, w = in ? expCall(lw) : 0.0;
+#pragma unroll
+  for (int o = 1; o < kMaxTrials; o <<= 1)
   {
-    if (ov[t]) continue;
-    const double lw = -beta * E[t] - (logq ? logq[t] : 0.0);
-    if (first < 0)
-    {
-      first = t;
-      selected = t;
-      cumw = exp(lw - largest);
-      continue;
-    }
-    if (cumw < ws)
-    {
-      cumw += exp(lw - largest);
-      selected = t;
-    }
+    const double x = __shfl_up_sync(0xffffffffu, run, o);
+    if (lane >= o) run += x;
+    w += __shfl_xor_sync(0xffffffffu, w, o);
   }
-  return selected;
+  *W = __shfl_sync(0xffffffffu, w, 0) / static_cast<double>(k);
+  const double ws = u * __shfl_sync(0xffffffffu, run, kMaxTrials - 1);
+  const unsigned reach = __ballot_sync(0xffffffffu, in && !(run < ws));
+  return reach ? __ffs(reach) - 1 : 31 - __clz(mask);
 }
 
 // Proposal density (relative to uniform) of a position: the cell of its unit-cell fractional coordinates.
 __device__ __forceinline__ double proposalDensity(const Params& p, const double r[3])
 {
   int c[3];
+#pragma unroll
   for (int a = 0; a < 3; ++a)
   {
     const double s = rgd::fract1(p.uic[0][a] * r[0] + p.uic[1][a] * r[1] + p.uic[2][a] * r[2]);
@@ -327,313 +544,320 @@ __device__ __forceinline__ double proposalDensity(const Params& p, const double 
   return p.prop_q[c[0] + p.prop_G * (c[1] + p.prop_G * c[2])];
 }
 
-extern __shared__ double2 gcmcDyn[];
-
-template <bool QUINTIC>
-__global__ void __launch_bounds__(kThreads) gcmcKernel(Params p, long long move0, int nmoves, int record,
-                                                       long long block_len)
+template <bool QUINTIC, bool SMEM>
+__global__ void __launch_bounds__(kThreads, 4) gcmcKernel(Params p, long long move0, int nmoves, int record,
+                                                          long long block_len)
 {
   const int chain = blockIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   __shared__ Shared sh;
-  double2* tab = gcmcDyn;  // phase tables: 2 * kMaxAtoms atoms x (kx+ky+kz+3)
+  const Dyn d = dynOf(p);
   const Component& c = p.comp;
-  const int na = c.n_atoms;
+  const int na = c.n_atoms, sb = c.starting_bead;
   double4* cpos = p.pos + static_cast<long long>(chain) * p.capacity * na;
   double* st = p.stats + static_cast<long long>(chain) * kStats;
+  double2* gS = p.sk + static_cast<long long>(chain) * p.nk;
+  double2* S = SMEM ? d.S : gS;
+  double2* D = SMEM ? d.D : p.dsk + static_cast<long long>(chain) * p.nk;
   const double ptot = p.p_translation + p.p_rotation + p.p_swap;
+
+  // the chain's state of this launch
+  for (int i = threadIdx.x; i < na * na; i += kThreads)
+  {
+    const int idx = c.types[i % na] * p.ff.n + c.types[i / na];
+    const bool lj = p.ff.lj[idx] != 0;
+    d.pair[i] = {lj ? p.ff.eps4[idx] : 0.0, lj ? 1.0 / p.ff.sig2[idx] : 1.0, lj ? p.ff.shift[idx] : 0.0,
+                 p.ff.coul * c.charges[i % na] * c.charges[i / na]};
+  }
+  if (SMEM && p.use_ewald)
+    for (int k = threadIdx.x; k < p.nk; k += kThreads) S[k] = gS[k];
+  if (threadIdx.x < kStats) sh.stats[threadIdx.x] = st[threadIdx.x];
+  if (threadIdx.x == 0)
+  {
+    sh.n = p.n[chain];
+    sh.energy = p.energy[chain];
+  }
+  __syncthreads();
 
   for (int it = 0; it < nmoves; ++it)
   {
     const long long mv = move0 + it;
-    const int n = p.n[chain];
-    const double2 uMove = uniform2(p.seed, chain, mv, kSlotMove);
-    const double2 uPick = uniform2(p.seed, chain, mv, kSlotPick);
-    const double2 uChange = uniform2(p.seed, chain, mv, kSlotChange);
+    const int n = sh.n;
+    // the move's own numbers: four lanes of each warp draw one block each
+    static_assert(kSlotMove == 0 && kSlotPick == 1 && kSlotChange == 2 && kSlotSelect == 3, "slots of lanes 0..3");
+    const double2 uLane = uniform2(p.seed, chain, mv, lane & 3);
+    auto fromLane = [&](int l)
+    { return make_double2(__shfl_sync(0xffffffffu, uLane.x, l), __shfl_sync(0xffffffffu, uLane.y, l)); };
+    const double2 uMove = fromLane(kSlotMove), uPick = fromLane(kSlotPick), uChange = fromLane(kSlotChange),
+                  uSel = fromLane(kSlotSelect);
     const double x = uMove.x * ptot;
     const int kind = x < p.p_translation ? 0 : (x < p.p_translation + p.p_rotation ? 1 : (uMove.y < 0.5 ? 2 : 3));
-    int accepted = 0;
+    const bool swap = kind >= 2, insert = kind == 2, retrace = kind == 3;
+    // the molecule moved, deleted or (the next place) inserted
+    const int m = insert ? n : min(n - 1, static_cast<int>(uPick.x * n));
+    bool alive = insert ? n < p.capacity : n > 0;  // the move goes on
+    const int skip = insert ? -1 : m;
+    double W1 = 1.0, e1 = 0.0;  // first bead: Rosenbluth weight and energy
+    int chosen = 0;
 
-    if (kind <= 1 && n > 0)
+    // Translation and rotation: one evaluation, of set 0 (new positions) and set 1 (old). Swap: two, the first-bead
+    // positions and then the orientations about the chosen one.
+    if (alive)
     {
-      // ---- translation / rotation ----
-      const int m = min(n - 1, static_cast<int>(uPick.x * n));
-      const int dir = min(2, static_cast<int>(3.0 * uPick.y));
-      if (threadIdx.x < na)
+      if (!swap)
       {
-        const int i = threadIdx.x;
-        const double4 o = cpos[m * na + i];
-        sh.oldPos[i][0] = o.x;
-        sh.oldPos[i][1] = o.y;
-        sh.oldPos[i][2] = o.z;
-      }
-      __syncthreads();
-      if (threadIdx.x == 0)
-      {
-        if (kind == 0)
-        {
-          const double disp = p.max_translation * 2.0 * (uChange.x - 0.5);
-          for (int i = 0; i < na; ++i)
-            for (int d = 0; d < 3; ++d) sh.newPos[i][d] = sh.oldPos[i][d] + (d == dir ? disp : 0.0);
-        }
-        else
-        {
-          const double angle = p.max_rotation * 2.0 * (uChange.x - 0.5);
-          const double cs = cos(angle), sn = sin(angle);
-          double com[3] = {0, 0, 0}, wsum = 0.0;
-          for (int i = 0; i < na; ++i)
-          {
-            for (int d = 0; d < 3; ++d) com[d] += c.masses[i] * sh.oldPos[i][d];
-            wsum += c.masses[i];
-          }
-          for (int d = 0; d < 3; ++d) com[d] /= wsum;
-          const int a = (dir + 1) % 3, b = (dir + 2) % 3;
-          for (int i = 0; i < na; ++i)
-          {
-            double r[3] = {sh.oldPos[i][0] - com[0], sh.oldPos[i][1] - com[1], sh.oldPos[i][2] - com[2]};
-            double q[3] = {r[0], r[1], r[2]};
-            q[a] = cs * r[a] - sn * r[b];
-            q[b] = sn * r[a] + cs * r[b];
-            for (int d = 0; d < 3; ++d) sh.newPos[i][d] = com[d] + q[d];
-          }
-        }
-      }
-      __syncthreads();
-      int idx[kMaxAtoms];
-      for (int i = 0; i < kMaxAtoms; ++i) idx[i] = i;
-      if (warp < 2)
-      {
-        int ov;
-        const double e = warpExternal<QUINTIC>(p, chain, n, warp == 0 ? sh.newPos : sh.oldPos, idx, na, m, &ov);
-        if (lane == 0)
-        {
-          sh.setE[warp] = e;
-          sh.setOv[warp] = ov;
-        }
-      }
-      __syncthreads();
-      double dEw = 0.0;
-      if (p.use_ewald) dEw = blockEwaldDelta(p, chain, sh.newPos, na, sh.oldPos, na, tab, sh.red);
-      const double dU = sh.setE[0] - sh.setE[1] + dEw;
-      accepted = (!sh.setOv[0]) && (uChange.y < exp(-p.beta * dU));
-      if (accepted)
-      {
+        const int dir = min(2, static_cast<int>(3.0 * uPick.y));
         if (threadIdx.x < na)
-          cpos[m * na + threadIdx.x] = make_double4(sh.newPos[threadIdx.x][0], sh.newPos[threadIdx.x][1],
-                                                    sh.newPos[threadIdx.x][2], 0.0);
-        if (p.use_ewald) blockAcceptEwald(p, chain);
-        if (threadIdx.x == 0) p.energy[chain] += dU;
-      }
-    }
-    else if (kind >= 2)
-    {
-      const bool insert = kind == 2;
-      const bool retrace = !insert;
-      if ((insert && n < p.capacity) || (retrace && n > 0))
-      {
-        const int m = insert ? n : min(n - 1, static_cast<int>(uPick.x * n));
-        const int skip = insert ? -1 : m;
-        const int sb = c.starting_bead;
-        const double2 uSel = uniform2(p.seed, chain, mv, kSlotSelect);
-        // first-bead trial positions (retrace: trial 0 is the existing first bead)
-        for (int t = threadIdx.x; t < p.k1; t += blockDim.x)
         {
-          if (retrace && t == 0)
+          const int i = threadIdx.x;
+          const double4 o = cpos[m * na + i];
+          const double old[3] = {o.x, o.y, o.z};
+          double now[3];
+          if (kind == 0)
           {
-            const double4 o = cpos[m * na + sb];
-            sh.trial[0][0][0] = o.x;
-            sh.trial[0][0][1] = o.y;
-            sh.trial[0][0][2] = o.z;
-            continue;
-          }
-          const double2 a = uniform2(p.seed, chain, mv, kSlotFirst + 4 * t);
-          const double2 b = uniform2(p.seed, chain, mv, kSlotFirst + 4 * t + 1);
-          const double2 u = uniform2(p.seed, chain, mv, kSlotFirst + 4 * t + 2);
-          if (!p.prop_cdf || u.x < p.prop_eps)
-          {
-            // SimulationBox::randomPosition (simulationbox.cpp:132-135)
-            const double s0 = a.x, s1 = a.y, s2 = b.x;
-            for (int r = 0; r < 3; ++r)
-              sh.trial[t][0][r] = p.box.c[0][r] * s0 + p.box.c[1][r] * s1 + p.box.c[2][r] * s2;
+            const double disp = p.max_translation * 2.0 * (uChange.x - 0.5);
+#pragma unroll
+            for (int r = 0; r < 3; ++r) now[r] = old[r] + (r == dir ? disp : 0.0);
           }
           else
           {
-            // a cell of the tabulated proposal (binary search of the cumulative probabilities), a uniform point in
-            // it, and a uniformly chosen unit-cell replica of the simulation box
-            const double2 v = uniform2(p.seed, chain, mv, kSlotFirst + 4 * t + 3);
-            const int G = p.prop_G;
-            const int ncell = G * G * G;
-            int lo = 0, hi = ncell - 1;
-            while (lo < hi)
+            const double angle = p.max_rotation * 2.0 * (uChange.x - 0.5);
+            double sn, cs;
+            sincospiCall(angle * (1.0 / rg::kPi), &sn, &cs);
+            double com[3] = {0, 0, 0}, wsum = 0.0;
+#pragma unroll 1
+            for (int j = 0; j < na; ++j)
             {
-              const int mid = (lo + hi) >> 1;
-              if (p.prop_cdf[mid] < u.y)
-                lo = mid + 1;
-              else
-                hi = mid;
+              const double4 q = cpos[m * na + j];
+              com[0] += c.masses[j] * q.x;
+              com[1] += c.masses[j] * q.y;
+              com[2] += c.masses[j] * q.z;
+              wsum += c.masses[j];
             }
-            const int ci = lo % G, cj = (lo / G) % G, ck = lo / (G * G);
-            const double sf[3] = {(ci + a.x) / G + static_cast<double>(min(p.rep[0] - 1, static_cast<int>(b.y * p.rep[0]))),
-                                  (cj + a.y) / G + static_cast<double>(min(p.rep[1] - 1, static_cast<int>(v.x * p.rep[1]))),
-                                  (ck + b.x) / G + static_cast<double>(min(p.rep[2] - 1, static_cast<int>(v.y * p.rep[2])))};
-            for (int r = 0; r < 3; ++r)
-              sh.trial[t][0][r] = p.uc[0][r] * sf[0] + p.uc[1][r] * sf[1] + p.uc[2][r] * sf[2];
+            const double inv = 1.0 / wsum;
+            double r[3], q[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+            {
+              com[k] *= inv;
+              r[k] = old[k] - com[k];
+            }
+            // about axis dir: (a, b) are the two others in cyclic order
+            q[0] = dir == 0 ? r[0] : (dir == 1 ? sn * r[2] + cs * r[0] : cs * r[0] - sn * r[1]);
+            q[1] = dir == 0 ? cs * r[1] - sn * r[2] : (dir == 1 ? r[1] : sn * r[0] + cs * r[1]);
+            q[2] = dir == 0 ? sn * r[1] + cs * r[2] : (dir == 1 ? cs * r[2] - sn * r[0] : r[2]);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) now[k] = com[k] + q[k];
           }
+#pragma unroll
+          for (int r = 0; r < 3; ++r)
+          {
+            d.trial[3 * i + r] = now[r];
+            d.trial[3 * (na + i) + r] = old[r];
+          }
+          sh.list[i] = i;
         }
-        __syncthreads();
-        for (int t = threadIdx.x; t < p.k1; t += blockDim.x)
-          sh.logq[t] = p.prop_cdf ? log(proposalDensity(p, sh.trial[t][0])) : 0.0;
-        int one[1] = {sb};
-        for (int t = warp; t < p.k1; t += kWarps)
+      }
+      else
+      {
+        // first-bead trial positions on warp 0 (retrace: trial 0 is the existing first bead); each lane's four draws
+        if (warp == 0 && lane < p.k1)
         {
-          int ov;
-          const double e = warpExternal<QUINTIC>(p, chain, n, sh.trial[t], one, 1, skip, &ov);
+          const int t = lane;
+          double* r = d.trial + 3 * (t * na + sb);
+          if (retrace && t == 0)
+          {
+            const double4 o = cpos[m * na + sb];
+            r[0] = o.x;
+            r[1] = o.y;
+            r[2] = o.z;
+          }
+          else
+          {
+            const double2 a = uniform2(p.seed, chain, mv, kSlotFirst + 4 * t);
+            const double2 b = uniform2(p.seed, chain, mv, kSlotFirst + 4 * t + 1);
+            double sf[3] = {a.x, a.y, b.x};
+            bool tabulated = false;
+            if (p.prop_cdf)
+            {
+              const double2 u = uniform2(p.seed, chain, mv, kSlotFirst + 4 * t + 2);
+              tabulated = !(u.x < p.prop_eps);
+              if (tabulated)
+              {
+                // a cell of the tabulated proposal (binary search of the cumulative probabilities), a uniform point in
+                // it, and a uniformly chosen unit-cell replica of the simulation box
+                const double2 v = uniform2(p.seed, chain, mv, kSlotFirst + 4 * t + 3);
+                const int G = p.prop_G;
+                int lo = 0, hi = G * G * G - 1;
+                while (lo < hi)
+                {
+                  const int mid = (lo + hi) >> 1;
+                  if (p.prop_cdf[mid] < u.y)
+                    lo = mid + 1;
+                  else
+                    hi = mid;
+                }
+                const int ci = lo % G, cj = (lo / G) % G, ck = lo / (G * G);
+                const double at[3] = {ci + a.x, cj + a.y, ck + b.x}, pick[3] = {b.y, v.x, v.y};
+#pragma unroll
+                for (int q = 0; q < 3; ++q)
+                  sf[q] = at[q] / G + static_cast<double>(min(p.rep[q] - 1, static_cast<int>(pick[q] * p.rep[q])));
+              }
+            }
+            // SimulationBox::randomPosition (simulationbox.cpp:132-135), or the cell's point in unit cells
+#pragma unroll
+            for (int q = 0; q < 3; ++q)
+              r[q] = tabulated ? p.uc[0][q] * sf[0] + p.uc[1][q] * sf[1] + p.uc[2][q] * sf[2]
+                               : p.box.c[0][q] * sf[0] + p.box.c[1][q] * sf[1] + p.box.c[2][q] * sf[2];
+          }
+          sh.logq[t] = p.prop_cdf ? log(proposalDensity(p, r)) : 0.0;
+        }
+        // the orientations' offsets from the first bead, meanwhile, on warp 1
+        if (warp == 1 && lane < p.k2 && !(retrace && lane == 0))
+        {
+          const double2 a = uniform2(p.seed, chain, mv, kSlotOrient + 2 * lane);
+          const double2 b = uniform2(p.seed, chain, mv, kSlotOrient + 2 * lane + 1);
+          double R[3][3];
+          rotationFromUniforms(a.x, a.y, b.x, R);
+          double* rel = d.rel + 3 * lane * na;
+#pragma unroll 1
+          for (int i = 0; i < na; ++i)
+#pragma unroll
+            for (int r = 0; r < 3; ++r)
+              rel[3 * i + r] = R[r][0] * (c.offsets[i][0] - c.offsets[sb][0]) +
+                               R[r][1] * (c.offsets[i][1] - c.offsets[sb][1]) +
+                               R[r][2] * (c.offsets[i][2] - c.offsets[sb][2]);
+        }
+        if (threadIdx.x == 0) sh.list[0] = sb;
+      }
+      __syncthreads();
+#pragma unroll 1
+      for (int phase = 0; phase < (swap ? 2 : 1); ++phase)
+      {
+        const int ns = swap ? (phase == 0 ? p.k1 : p.k2) : 2, cnt = swap ? (phase == 0 ? 1 : na - 1) : na;
+        evaluateSets<QUINTIC>(p, sh, d, cpos, n, ns, cnt, skip);
+        if (!swap) break;
+        if (warp == 0)
+        {
+          double W, E = 0.0;
+          int ov = 1;
+          if (lane < ns) E = setEnergy(sh, d, ns, cnt, lane, &ov);
+          int sel = selectTrial(E, !ov, phase == 0 && lane < ns ? sh.logq[lane] : 0.0, ns, p.beta,
+                                phase == 0 ? uSel.x : uSel.y, &W);
+          if (retrace) sel = __shfl_sync(0xffffffffu, ov, 0) ? -1 : 0;
+          E = __shfl_sync(0xffffffffu, E, max(sel, 0));
           if (lane == 0)
           {
-            sh.setE[t] = e;
-            sh.setOv[t] = ov;
+            sh.sel = sel;
+            sh.W = W;
+            sh.E = E;
           }
         }
         __syncthreads();
-        if (threadIdx.x == 0)
+        chosen = sh.sel;
+        W1 *= sh.W;
+        e1 += sh.E;
+        if (chosen < 0)
         {
-          double W1;
-          int sel = selectTrial(sh.setE, sh.setOv, sh.logq, p.k1, p.beta, uSel.x, &W1);
-          if (retrace) sel = sh.setOv[0] ? -1 : 0;
-          sh.ints[0] = sel;
-          sh.dbl[0] = W1;
-          sh.dbl[1] = sel >= 0 ? sh.setE[sel] : 0.0;
-          if (sel >= 0)
-            for (int d = 0; d < 3; ++d) sh.dbl[2 + d] = sh.trial[sel][0][d];
+          alive = false;
+          break;
         }
+        if (phase == 1) break;
+        const double fb[3] = {d.trial[3 * (chosen * na + sb)], d.trial[3 * (chosen * na + sb) + 1],
+                              d.trial[3 * (chosen * na + sb) + 2]};
         __syncthreads();
-        const int sel1 = sh.ints[0];
-        if (sel1 >= 0)
+        // orientation trials about the first bead (retrace: trial 0 is the existing orientation)
+#pragma unroll 1
+        for (int q = threadIdx.x; q < p.k2 * na; q += kThreads)
         {
-          const double W1 = sh.dbl[0], e1 = sh.dbl[1];
-          const double fb[3] = {sh.dbl[2], sh.dbl[3], sh.dbl[4]};
-          __syncthreads();
-          // orientation trials about the first bead (retrace: trial 0 is the existing orientation)
-          for (int t = threadIdx.x; t < p.k2; t += blockDim.x)
+          double* r = d.trial + 3 * q;
+          if (retrace && q < na)
           {
-            if (retrace && t == 0)
-            {
-              for (int i = 0; i < na; ++i)
-              {
-                const double4 o = cpos[m * na + i];
-                sh.trial[0][i][0] = o.x;
-                sh.trial[0][i][1] = o.y;
-                sh.trial[0][i][2] = o.z;
-              }
-              continue;
-            }
-            const double2 a = uniform2(p.seed, chain, mv, kSlotOrient + 2 * t);
-            const double2 b = uniform2(p.seed, chain, mv, kSlotOrient + 2 * t + 1);
-            double R[3][3];
-            rotationFromUniforms(a.x, a.y, b.x, R);
-            double rsb[3];
-            for (int r = 0; r < 3; ++r)
-              rsb[r] = R[r][0] * c.offsets[sb][0] + R[r][1] * c.offsets[sb][1] + R[r][2] * c.offsets[sb][2];
-            for (int i = 0; i < na; ++i)
-              for (int r = 0; r < 3; ++r)
-                sh.trial[t][i][r] = fb[r] - rsb[r] + R[r][0] * c.offsets[i][0] + R[r][1] * c.offsets[i][1] +
-                                    R[r][2] * c.offsets[i][2];
+            const double4 o = cpos[m * na + q];
+            r[0] = o.x;
+            r[1] = o.y;
+            r[2] = o.z;
           }
-          __syncthreads();
-          int others[kMaxAtoms];
-          int no = 0;
-          for (int i = 0; i < na; ++i)
-            if (i != sb) others[no++] = i;
-          for (int t = warp; t < p.k2; t += kWarps)
-          {
-            // gather the non-starting-bead atoms of trial t
-            double op[kMaxAtoms][3];
-            for (int j = 0; j < no; ++j)
-              for (int d = 0; d < 3; ++d) op[j][d] = sh.trial[t][others[j]][d];
-            int ov = 0;
-            const double e = no > 0 ? warpExternal<QUINTIC>(p, chain, n, op, others, no, skip, &ov) : 0.0;
-            if (lane == 0)
-            {
-              sh.setE[t] = e;
-              sh.setOv[t] = ov;
-            }
-          }
-          __syncthreads();
-          if (threadIdx.x == 0)
-          {
-            double W2;
-            int sel = selectTrial(sh.setE, sh.setOv, nullptr, p.k2, p.beta, uSel.y, &W2);
-            if (retrace) sel = sh.setOv[0] ? -1 : 0;
-            sh.ints[1] = sel;
-            sh.dbl[5] = W2;
-            sh.dbl[6] = sel >= 0 ? sh.setE[sel] : 0.0;
-            if (sel >= 0)
-              for (int i = 0; i < na; ++i)
-                for (int d = 0; d < 3; ++d)
-                {
-                  if (insert)
-                    sh.newPos[i][d] = sh.trial[sel][i][d];
-                  else
-                    sh.oldPos[i][d] = sh.trial[sel][i][d];
-                }
-          }
-          __syncthreads();
-          const int sel2 = sh.ints[1];
-          if (sel2 >= 0)
-          {
-            const double W = W1 * sh.dbl[5];
-            const double eExt = e1 + sh.dbl[6];
-            double dEw = 0.0;
-            if (p.use_ewald)
-            {
-              dEw = insert ? blockEwaldDelta(p, chain, sh.newPos, na, sh.oldPos, 0, tab, sh.red)
-                           : blockEwaldDelta(p, chain, sh.newPos, 0, sh.oldPos, na, tab, sh.red);
-              dEw += insert ? c.self_excl : -c.self_excl;
-            }
-            double pacc;
-            if (insert)
-              pacc = W < 1e-150 ? 0.0
-                                : exp(-p.beta * dEw) * p.beta * p.fugacity * p.volume / static_cast<double>(n + 1) * W;
-            else
-              pacc = exp(-p.beta * dEw) * static_cast<double>(n) / (p.beta * p.fugacity * p.volume) / W;
-            accepted = uChange.y < pacc;
-            if (accepted)
-            {
-              if (insert)
-              {
-                if (threadIdx.x < na)
-                  cpos[n * na + threadIdx.x] = make_double4(sh.newPos[threadIdx.x][0], sh.newPos[threadIdx.x][1],
-                                                            sh.newPos[threadIdx.x][2], 0.0);
-              }
-              else if (m != n - 1 && threadIdx.x < na)
-              {
-                cpos[m * na + threadIdx.x] = cpos[(n - 1) * na + threadIdx.x];
-              }
-              if (p.use_ewald) blockAcceptEwald(p, chain);
-              if (threadIdx.x == 0)
-              {
-                p.energy[chain] += insert ? (eExt + dEw) : (-eExt + dEw);
-                p.n[chain] = insert ? n + 1 : n - 1;
-              }
-            }
-          }
+          else
+#pragma unroll
+            for (int k = 0; k < 3; ++k) r[k] = fb[k] + d.rel[3 * q + k];
         }
+        if (threadIdx.x < na && static_cast<int>(threadIdx.x) != sb)
+          sh.list[threadIdx.x - (static_cast<int>(threadIdx.x) > sb ? 1 : 0)] = threadIdx.x;
+        __syncthreads();
+      }
+    }
+    int accepted = 0;
+    double dE = 0.0;
+    if (alive)
+    {
+      double dEw = 0.0;
+      if (p.use_ewald)
+      {
+        dEw = blockEwaldDelta(p, sh, d, S, D, chosen, retrace ? 0 : na, swap ? chosen : 1, insert ? 0 : na);
+        if (swap) dEw += insert ? c.self_excl : -c.self_excl;
+      }
+      double pacc;
+      if (!swap)
+      {
+        int ov, old_ov;
+        dE = setEnergy(sh, d, 2, na, 0, &ov) - setEnergy(sh, d, 2, na, 1, &old_ov) + dEw;
+        pacc = expCall(-p.beta * dE);
+        accepted = !ov && uChange.y < pacc;
+      }
+      else
+      {
+        dE = insert ? e1 + dEw : dEw - e1;
+        pacc = expCall(-p.beta * dEw);
+        if (insert)
+          pacc = W1 < 1e-150 ? 0.0 : pacc * p.beta * p.fugacity * p.volume / static_cast<double>(n + 1) * W1;
+        else
+          pacc = pacc * static_cast<double>(n) / (p.beta * p.fugacity * p.volume) / W1;
+        accepted = uChange.y < pacc;
+      }
+      if (accepted)
+      {
+        if (threadIdx.x < na)
+        {
+          const double* r = d.trial + 3 * (chosen * na + threadIdx.x);
+          if (!retrace)
+            cpos[m * na + threadIdx.x] = make_double4(r[0], r[1], r[2], 0.0);
+          else if (m != n - 1)
+            cpos[m * na + threadIdx.x] = cpos[(n - 1) * na + threadIdx.x];
+        }
+        if (p.use_ewald) blockAcceptEwald(p, S, D);
+      }
+    }
+    if (threadIdx.x == 0)
+    {
+      if (accepted)
+      {
+        sh.energy += dE;
+        if (swap) sh.n = insert ? n + 1 : n - 1;
+      }
+      if (record)
+      {
+        const int nn = sh.n;
+        double* q = sh.stats;
+        q[kind] += 1.0;
+        q[4 + kind] += accepted ? 1.0 : 0.0;
+        q[8] += nn;
+        q[9] += static_cast<double>(nn) * nn;
+        q[10] += sh.energy;
+        q[11] += 1.0;
+        const long long b = block_len > 0 ? static_cast<long long>(q[11] - 1.0) / block_len : 0;
+        if (b < 5) q[12 + b] += nn;
       }
     }
     __syncthreads();
-    if (threadIdx.x == 0 && record)
-    {
-      const int nn = p.n[chain];
-      st[kind] += 1.0;
-      st[4 + kind] += accepted ? 1.0 : 0.0;
-      st[8] += nn;
-      st[9] += static_cast<double>(nn) * nn;
-      st[10] += p.energy[chain];
-      st[11] += 1.0;
-      const long long b = block_len > 0 ? static_cast<long long>(st[11] - 1.0) / block_len : 0;
-      if (b < 5) st[12 + b] += nn;
-    }
-    __syncthreads();
+  }
+  if (SMEM && p.use_ewald)
+    for (int k = threadIdx.x; k < p.nk; k += kThreads) gS[k] = S[k];
+  if (threadIdx.x < kStats) st[threadIdx.x] = sh.stats[threadIdx.x];
+  if (threadIdx.x == 0)
+  {
+    p.n[chain] = sh.n;
+    p.energy[chain] = sh.energy;
   }
 }
 }  // namespace
@@ -647,6 +871,9 @@ struct rg_gcmc
   long long recorded = 0;
   long long block_len = 0;
   size_t shmem = 0;
+  bool smem = true;  // the structure factors fit in shared memory
+  int4* runs = nullptr;
+  double* run_temp = nullptr;
   int max_moves_per_launch = 2048;
 };
 
@@ -717,7 +944,9 @@ rg_status rg_gcmc_create(rg_system* system, rg_ewald* ewald, const rg_gcmc_compo
   {
     const double2* s_rigid;
     double alpha, single_ion;
-    st = rgd::ewaldExport(ewald, &p.kvec, &p.temp, &s_rigid, &nk, p.kmax, &alpha, &single_ion);
+    const char4* kvec;
+    const double* temp;
+    st = rgd::ewaldExport(ewald, &kvec, &temp, &s_rigid, &nk, p.kmax, &alpha, &single_ion);
     if (st)
     {
       delete g;
@@ -747,9 +976,23 @@ rg_status rg_gcmc_create(rg_system* system, rg_ewald* ewald, const rg_gcmc_compo
       }
     p.comp.self_excl = se;
     p.nk = nk;
+    // the k-vectors as runs of kz, and their prefactors by (|kz|, sign, run)
+    const std::vector<int4> runs = rgd::ewaldRuns(ewald);  // longest first: the threads of large |kz| are neighbours
+    p.n_runs = static_cast<int>(runs.size());
+    std::vector<double> rt;
+    cudaError_t err = rgd::ewaldRunPrefactors(ewald, runs, rt);
+    if (!err && !runs.empty()) err = cudaMalloc(reinterpret_cast<void**>(&g->runs), sizeof(int4) * runs.size());
+    if (!err && !runs.empty()) err = cudaMalloc(reinterpret_cast<void**>(&g->run_temp), sizeof(double) * rt.size());
+    if (!err && !runs.empty())
+      err = cudaMemcpyAsync(g->runs, runs.data(), sizeof(int4) * runs.size(), cudaMemcpyHostToDevice, ctx->stream);
+    if (!err && !runs.empty())
+      err = cudaMemcpyAsync(g->run_temp, rt.data(), sizeof(double) * rt.size(), cudaMemcpyHostToDevice, ctx->stream);
+    if (!err) err = cudaStreamSynchronize(ctx->stream);
+    p.runs = g->runs;
+    p.run_temp = g->run_temp;
     // all chains start from the framework structure factor
     const size_t skb = sizeof(double2) * static_cast<size_t>(nk) * n_chains;
-    cudaError_t err = cudaMalloc(reinterpret_cast<void**>(&p.sk), skb);
+    if (!err) err = cudaMalloc(reinterpret_cast<void**>(&p.sk), skb);
     if (!err) err = cudaMalloc(reinterpret_cast<void**>(&p.dsk), skb);
     for (int c = 0; c < n_chains && !err; ++c)
       err = cudaMemcpyAsync(p.sk + static_cast<size_t>(c) * nk, s_rigid, sizeof(double2) * nk,
@@ -775,8 +1018,12 @@ rg_status rg_gcmc_create(rg_system* system, rg_ewald* ewald, const rg_gcmc_compo
     rg_gcmc_destroy(g);
     return rg::cudaFail(ctx, err, "rg_gcmc_create");
   }
-  const int stride = (p.kmax[0] + 1) + (p.kmax[1] + 1) + (p.kmax[2] + 1);
-  g->shmem = sizeof(double2) * 2 * kMaxAtoms * (p.use_ewald ? stride : 1);
+  // The structure factors and their change stay in shared memory where four CTAs still fit on an SM (the registers'
+  // limit): at kmax 8 the 1,152 k-vectors of the sphere take 37 KB. Larger sets stay in global memory.
+  const size_t fixed = dynFixedBytes(comp->n_atoms, p.kmax, p.use_ewald != 0);
+  const size_t sk_bytes = 2 * sizeof(double2) * static_cast<size_t>(p.nk);
+  g->smem = fixed + sk_bytes <= kSharedPerCta;
+  g->shmem = fixed + (g->smem ? sk_bytes : 0);
   *out = g;
   return RG_OK;
 }
@@ -791,6 +1038,8 @@ rg_status rg_gcmc_destroy(rg_gcmc* g)
   cudaFree(g->p.n);
   cudaFree(g->p.energy);
   cudaFree(g->p.stats);
+  cudaFree(g->runs);
+  cudaFree(g->run_temp);
   delete g;
   return RG_OK;
 }
@@ -805,13 +1054,17 @@ rg_status rg_gcmc_run(rg_gcmc* g, int64_t moves, int record)
   while (left > 0)
   {
     const int chunk = static_cast<int>(left < g->max_moves_per_launch ? left : g->max_moves_per_launch);
-    if (g->p.quintic)
-      gcmcKernel<true><<<g->n_chains, kThreads, g->shmem, ctx->stream>>>(g->p, g->moves_done, chunk, record,
-                                                                         g->block_len);
-    else
-      gcmcKernel<false><<<g->n_chains, kThreads, g->shmem, ctx->stream>>>(g->p, g->moves_done, chunk, record,
-                                                                          g->block_len);
-    RG_CUDA(ctx, cudaGetLastError());
+    auto launch = [&](auto kern)
+    {
+      // another object's call may have set this kernel's limit lower
+      const cudaError_t err =
+          cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(g->shmem));
+      if (err) return err;
+      kern<<<g->n_chains, kThreads, g->shmem, ctx->stream>>>(g->p, g->moves_done, chunk, record, g->block_len);
+      return cudaGetLastError();
+    };
+    RG_CUDA(ctx, g->p.quintic ? (g->smem ? launch(gcmcKernel<true, true>) : launch(gcmcKernel<true, false>))
+                              : (g->smem ? launch(gcmcKernel<false, true>) : launch(gcmcKernel<false, false>)));
     g->moves_done += chunk;
     left -= chunk;
   }
