@@ -187,10 +187,14 @@ struct Shared
   int binned;                          // 1: the cells describe the staged slice as it is
 };
 
-__device__ __forceinline__ double2 urand(const Params& p, long long move, uint32_t sl)
-{
-  return rgd::uniform2(gs.seed, 0, move, sl);
-}
+// The launch's parameters, the CTA's working state and the trial atoms' VDW grids, at file scope so that the functions
+// below read them as shared memory whether they are inlined or not. Those that several kinds of move call are not: the
+// kernel was 493 KB of code with five copies of phase(), and fetching it held every move.
+__shared__ Params sp;
+__shared__ Shared ss;
+__shared__ const double* sGrid[kMaxItems];
+
+__device__ __noinline__ double2 urand(long long move, uint32_t sl) { return rgd::uniform2(gs.seed, 0, move, sl); }
 
 __device__ __forceinline__ uint32_t fixOf(double s)
 {
@@ -383,8 +387,11 @@ __device__ __forceinline__ void segmentDelta(const Params& p, const Shared& sh, 
 
 // The accepted candidate's structure-factor change added to this CTA's S(k) range (the phasor tables of the phase
 // that evaluated it are still in shared memory).
-__device__ void addCandidate(const Params& p, const Shared& sh, const Dyn& dy, int c)
+__device__ __noinline__ void addCandidate(int c)
 {
+  const Params& p = sp;
+  const Shared& sh = ss;
+  const Dyn dy = dynOf(p);
   for (int sg = threadIdx.x; sg < sh.nseg; sg += kThreads)
   {
     const int k0 = dy.segStart[sg], n = dy.segStart[sg + 1] - k0;
@@ -494,8 +501,11 @@ __device__ __forceinline__ void pairTerm(const PC& p, const Shared& sh, int4 B, 
 // per trial atom in sh.ovl. vdwOf/qOf: the framework grid and charge of each trial atom (set by the caller in
 // sh.tf[].w = type; the grids come from the type). Returns false if a barrier failed.
 template <bool QUINTIC>  // the system's grids: triquintic (27 values per point) or tricubic (8)
-__device__ bool phase(const Params& p, Shared& sh, int skip, const double* const* atomGrid)
+__device__ __noinline__ bool phase(int skip)
 {
+  const Params& p = sp;
+  Shared& sh = ss;
+  const double* const* atomGrid = sGrid;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int G = p.group, cta = static_cast<int>(blockIdx.x) % p.group;
   const int nta = sh.nta, ncand = sh.ncand;
@@ -534,7 +544,7 @@ __device__ bool phase(const Params& p, Shared& sh, int skip, const double* const
         g.data = l16 < 8 ? vdw : p.ewald_grid;
         const double3 r = sh.ta[b];
         if (!QUINTIC)
-          v = rgd::interpolateCorner(g, rgd::gridCell(g, r.x, r.y, r.z), l16 & 7);
+          v = rgd::interpolateLaneCorner(g, r.x, r.y, r.z, l16 & 7);
         else if ((l16 & 7) == 0)  // triquintic grids: lanes 0 and 8 of the half take the whole interpolant
           v = rgd::interpolateQuintic(g, r.x, r.y, r.z, nullptr);
       }
@@ -876,11 +886,12 @@ __device__ double proposalDensity(const Params& p, const Comp& c, double3 r)
 }
 
 // First-bead trial position t of component c: uniform in the box, or from the component's tabulated proposal
-__device__ double3 firstBeadPosition(const Params& p, const Comp& c, long long move, int t)
+__device__ __noinline__ double3 firstBeadPosition(const Comp& c, long long move, int t)
 {
-  const double2 a = urand(p, move, slot(kKindFirst, t, 0));
-  const double2 b = urand(p, move, slot(kKindFirst, t, 1));
-  const double2 u = urand(p, move, slot(kKindFirst, t, 2));
+  const Params& p = sp;
+  const double2 a = urand(move, slot(kKindFirst, t, 0));
+  const double2 b = urand(move, slot(kKindFirst, t, 1));
+  const double2 u = urand(move, slot(kKindFirst, t, 2));
   double sf[3];
   const double(*cell)[3] = p.box.c;
   if (!c.prop_cdf || u.x < c.prop_eps)
@@ -891,7 +902,7 @@ __device__ double3 firstBeadPosition(const Params& p, const Comp& c, long long m
   }
   else
   {
-    const double2 v = urand(p, move, slot(kKindFirst, t, 3));
+    const double2 v = urand(move, slot(kKindFirst, t, 3));
     const int G = c.prop_G, ncell = G * G * G;
     int lo = 0, hi = ncell - 1;
     while (lo < hi)
@@ -914,10 +925,10 @@ __device__ double3 firstBeadPosition(const Params& p, const Comp& c, long long m
 }
 
 // orientation (kind, t) of component c as offsets from its starting bead: rel[i] = R o_i - R o_sb
-__device__ void orientationOffsets(const Params& p, const Comp& c, long long move, uint32_t kind, int t, double3* rel)
+__device__ __noinline__ void orientationOffsets(const Comp& c, long long move, uint32_t kind, int t, double3* rel)
 {
-  const double2 a = urand(p, move, slot(kind, t, 0));
-  const double2 b = urand(p, move, slot(kind, t, 1));
+  const double2 a = urand(move, slot(kind, t, 0));
+  const double2 b = urand(move, slot(kind, t, 1));
   double R[3][3];
   rotationFromUniforms(a.x, a.y, b.x, R);
   const double* o0 = c.offsets[c.starting_bead];
@@ -934,11 +945,11 @@ __device__ void orientationOffsets(const Params& p, const Comp& c, long long mov
 }
 
 // the atoms of component c with its starting bead at `first`, orientation from (kind, t)
-__device__ void orientedMolecule(const Params& p, const Comp& c, double3 first, long long move, uint32_t kind, int t,
-                                 double3* out)
+__device__ __noinline__ void orientedMolecule(const Comp& c, double3 first, long long move, uint32_t kind, int t,
+                                              double3* out)
 {
-  const double2 a = urand(p, move, slot(kind, t, 0));
-  const double2 b = urand(p, move, slot(kind, t, 1));
+  const double2 a = urand(move, slot(kind, t, 0));
+  const double2 b = urand(move, slot(kind, t, 1));
   double R[3][3];
   rotationFromUniforms(a.x, a.y, b.x, R);
   const double* o0 = c.offsets[c.starting_bead];
@@ -958,7 +969,7 @@ __device__ void orientedMolecule(const Params& p, const Comp& c, double3 first, 
 // holds the log-weight lw of trial t and whether it is allowed. Returns in every lane the selected trial (-1 if none)
 // and W = sum over the allowed trials of exp(lw) / k. The maximum, the prefix sums and the total come from fixed
 // shuffle patterns, so every CTA takes the same decision.
-__device__ int warpSelect(double lw, bool ok, int k, double u, double* W)
+__device__ __noinline__ int warpSelect(double lw, bool ok, int k, double u, double* W)
 {
   const int lane = threadIdx.x & 31;
   const bool on = ok && lane < k;
@@ -994,14 +1005,18 @@ __device__ __forceinline__ double3 loadPos(const Params& p, int site)
 // write the atoms of molecule m (every CTA writes the same values; each reads back only its own writes). Sites of
 // this CTA's staged slice are updated in shared memory as well, which then needs new cells; a change of the number of
 // molecules, made by the caller after this, moves every CTA's slice and so has it staged again.
-__device__ void storeMolecule(const Params& p, Shared& sh, int m, int cidx, const double3* x)
+// By warp 0, a lane per atom; x is in shared memory.
+__device__ __noinline__ void storeMolecule(int m, int cidx, const double3* x)
 {
+  const Params& p = sp;
+  Shared& sh = ss;
   const Comp& c = p.comp[cidx];
   const int G = p.group, cta = static_cast<int>(blockIdx.x) % p.group;
   const int ns = sh.n * p.na, chunk = (ns + G - 1) / G, s0 = min(ns, cta * chunk), s1 = min(ns, s0 + chunk);
   const int nst = min(s1 - s0, p.nslice);
   int4* slice = dynOf(p).slice;
-  for (int i = 0; i < p.na; ++i)
+  const int i = threadIdx.x;
+  if (i < p.na)
   {
     const int4 f = toFixed(p, x[i], c.types[i] | (m << 8));
     gs.pos[m * p.na + i] = make_double4(x[i].x, x[i].y, x[i].z, 0.0);
@@ -1013,12 +1028,15 @@ __device__ void storeMolecule(const Params& p, Shared& sh, int m, int cidx, cons
       sh.binned = 0;
     }
   }
+  __syncwarp();
 }
 
 // the atoms of one orientation trial other than the starting bead, in atom order, into trial-atom slots base, base+1, ..
-__device__ void storeOrientation(const Params& p, Shared& sh, const double** atomGrid, const Comp& cc,
-                                 const double3* x, int base)
+__device__ __noinline__ void storeOrientation(const Comp& cc, const double3* x, int base)
 {
+  const Params& p = sp;
+  Shared& sh = ss;
+  const double** atomGrid = sGrid;
   int a = base;
   for (int i = 0; i < p.na; ++i)
   {
@@ -1043,11 +1061,15 @@ static_assert(sizeof(Launch) <= 32000, "kernel parameter space");
 template <bool QUINTIC>
 __global__ void __launch_bounds__(kThreads, 1) mixtureKernel(const __grid_constant__ Launch L, int moves)
 {
-  const Params& p = L.p;
-  const int cta = static_cast<int>(blockIdx.x) % p.group;
-  if (threadIdx.x == 0) gs = *L.st[blockIdx.x / p.group];
+  static_assert(sizeof(Params) % sizeof(int) == 0, "copied word by word");
+  for (int i = threadIdx.x; i < static_cast<int>(sizeof(Params) / sizeof(int)); i += kThreads)
+    reinterpret_cast<int*>(&sp)[i] = reinterpret_cast<const int*>(&L.p)[i];
+  if (threadIdx.x == 0) gs = *L.st[blockIdx.x / L.p.group];
   __syncthreads();
-  __shared__ Shared sh;
+  const Params& p = sp;
+  Shared& sh = ss;
+  const double** atomGrid = sGrid;
+  const int cta = static_cast<int>(blockIdx.x) % p.group;
   const int tid = threadIdx.x;
   const int na = p.na;
   for (int i = tid; i < kMaxTypes * kMaxTypes; i += kThreads) sh.tab[i] = gs.ljf[i];
@@ -1068,7 +1090,6 @@ __global__ void __launch_bounds__(kThreads, 1) mixtureKernel(const __grid_consta
   const int G = p.group;
   const int kchunk = (p.nk + G - 1) / G, k0 = cta * kchunk, k1 = min(p.nk, k0 + kchunk);
   const long long move0 = *gs.move_base;
-  __shared__ const double* atomGrid[kMaxItems];
   const Dyn dyk = dynOf(p);
   // this CTA's k-range and framework slice, kept in shared memory for the whole launch
   for (int kk = tid; kk < k1 - k0; kk += kThreads)
@@ -1117,7 +1138,7 @@ __global__ void __launch_bounds__(kThreads, 1) mixtureKernel(const __grid_consta
     // the move's eight uniform numbers: four Philox draws, one per lane of warp 0
     if (tid < 4)
     {
-      const double2 u = urand(p, move, slot(kKindMove, 0, tid));
+      const double2 u = urand(move, slot(kKindMove, 0, tid));
       sh.u[2 * tid] = u.x;
       sh.u[2 * tid + 1] = u.y;
     }
@@ -1140,69 +1161,62 @@ __global__ void __launch_bounds__(kThreads, 1) mixtureKernel(const __grid_consta
     int c = sh.c;
     if ((kind == 0 || kind == 1) && sh.count[c] > 0)
     {
-      // translation (one Cartesian direction) or rotation (one Cartesian axis about the centre of mass)
-      if (tid == 0)
+      // translation (one Cartesian direction) or rotation (one Cartesian axis about the centre of mass): a lane per
+      // atom of the new and of the old positions, each from the same loads
+      if (tid < 2 * na)
       {
         const Comp& cc = p.comp[c];
         const int m = __ldcg(gs.list + c * p.capacity + min(sh.count[c] - 1, static_cast<int>(sh.u[3] * sh.count[c])));
-        sh.m = m;
         const int dir = min(2, static_cast<int>(3.0 * sh.u[4]));
-        double3 old[kMaxAtoms], nw[kMaxAtoms];
-        for (int i = 0; i < na; ++i) old[i] = nw[i] = loadPos(p, m * na + i);
-        if (kind == 0)
+        const bool isNew = tid < na;
+        const int i = isNew ? tid : tid - na;
+        double3 x = loadPos(p, m * na + i);
+        if (isNew && kind == 0)
         {
           const double d = p.max_translation * 2.0 * (sh.u[5] - 0.5);
-          for (int i = 0; i < na; ++i)
-          {
-            if (dir == 0) nw[i].x += d;
-            if (dir == 1) nw[i].y += d;
-            if (dir == 2) nw[i].z += d;
-          }
+          if (dir == 0) x.x += d;
+          if (dir == 1) x.y += d;
+          if (dir == 2) x.z += d;
         }
-        else
+        else if (isNew)
         {
           const double ang = p.max_rotation * 2.0 * (sh.u[5] - 0.5);
           double sn, cs;
           sincos(ang, &sn, &cs);
           double ctr[3] = {0, 0, 0}, w = 0.0;
-          for (int i = 0; i < na; ++i)
+          for (int j = 0; j < na; ++j)
           {
-            ctr[0] += cc.masses[i] * old[i].x;
-            ctr[1] += cc.masses[i] * old[i].y;
-            ctr[2] += cc.masses[i] * old[i].z;
-            w += cc.masses[i];
+            const double3 o = loadPos(p, m * na + j);
+            ctr[0] += cc.masses[j] * o.x;
+            ctr[1] += cc.masses[j] * o.y;
+            ctr[2] += cc.masses[j] * o.z;
+            w += cc.masses[j];
           }
+#pragma unroll
           for (int d = 0; d < 3; ++d) ctr[d] /= w;
-          const int a1 = (dir + 1) % 3, a2 = (dir + 2) % 3;
-          for (int i = 0; i < na; ++i)
-          {
-            const double dv[3] = {old[i].x - ctr[0], old[i].y - ctr[1], old[i].z - ctr[2]};
-            double r[3] = {dv[0], dv[1], dv[2]};
-            r[a1] = cs * dv[a1] - sn * dv[a2];
-            r[a2] = sn * dv[a1] + cs * dv[a2];
-            nw[i] = make_double3(ctr[0] + r[0], ctr[1] + r[1], ctr[2] + r[2]);
-          }
+          const double dv[3] = {x.x - ctr[0], x.y - ctr[1], x.z - ctr[2]};
+          // about axis dir: (a, b) are the two others in cyclic order
+          const double rx = dir == 0 ? dv[0] : (dir == 1 ? sn * dv[2] + cs * dv[0] : cs * dv[0] - sn * dv[1]);
+          const double ry = dir == 0 ? cs * dv[1] - sn * dv[2] : (dir == 1 ? dv[1] : sn * dv[0] + cs * dv[1]);
+          const double rz = dir == 0 ? sn * dv[1] + cs * dv[2] : (dir == 1 ? cs * dv[2] - sn * dv[0] : dv[2]);
+          x = make_double3(ctr[0] + rx, ctr[1] + ry, ctr[2] + rz);
         }
-        for (int i = 0; i < na; ++i)
+        sh.ta[tid] = x;
+        sh.tf[tid] = toFixed(p, x, cc.types[i]);
+        atomGrid[tid] = cc.vdw_grid[i];
+        sh.cpos[0][tid] = x;
+        sh.cq[0][tid] = isNew ? cc.charges[i] : -cc.charges[i];
+        if (isNew) sh.mol[i] = x;
+        if (tid == 0)
         {
-          sh.ta[i] = nw[i];
-          sh.tf[i] = toFixed(p, nw[i], cc.types[i]);
-          atomGrid[i] = cc.vdw_grid[i];
-          sh.ta[na + i] = old[i];
-          sh.tf[na + i] = toFixed(p, old[i], cc.types[i]);
-          atomGrid[na + i] = cc.vdw_grid[i];
-          sh.cpos[0][i] = nw[i];
-          sh.cq[0][i] = cc.charges[i];
-          sh.cpos[0][na + i] = old[i];
-          sh.cq[0][na + i] = -cc.charges[i];
-          sh.mol[i] = nw[i];
+          sh.m = m;
+          sh.cn[0] = 2 * na;
+          sh.nta = 2 * na;
+          sh.ncand = p.use_charge ? 1 : 0;
         }
-        sh.cn[0] = 2 * na;
-        sh.nta = 2 * na;
-        sh.ncand = p.use_charge ? 1 : 0;
       }
       __syncthreads();
-      if (!phase<QUINTIC>(p, sh, sh.m, atomGrid)) break;
+      if (!phase<QUINTIC>(sh.m)) break;
       if (tid == 0)
       {
         bool ovn = false;
@@ -1222,8 +1236,8 @@ __global__ void __launch_bounds__(kThreads, 1) mixtureKernel(const __grid_consta
       __syncthreads();
       if (sh.accept)
       {
-        if (tid == 0) storeMolecule(p, sh, sh.m, c, sh.mol);
-        if (p.use_charge) addCandidate(p, sh, dyk, 0);
+        if (tid < 32) storeMolecule(sh.m, c, sh.mol);
+        if (p.use_charge) addCandidate(0);
       }
     }
     else if (kind == 2 && sh.n < p.capacity)
@@ -1233,7 +1247,7 @@ __global__ void __launch_bounds__(kThreads, 1) mixtureKernel(const __grid_consta
       const int sb = cc.starting_bead;
       if (tid < p.k1)
       {
-        const double3 r = firstBeadPosition(p, cc, move, tid);
+        const double3 r = firstBeadPosition(cc, move, tid);
         sh.ta[tid] = r;
         sh.tf[tid] = toFixed(p, r, cc.types[sb]);
         atomGrid[tid] = cc.vdw_grid[sb];
@@ -1245,15 +1259,15 @@ __global__ void __launch_bounds__(kThreads, 1) mixtureKernel(const __grid_consta
         sh.ncand = 0;
       }
       // the orientations depend only on the move: their offsets are computed now, by threads of another warp
-      if (tid >= 32 && tid < 32 + p.k2) orientationOffsets(p, cc, move, kKindOrient, tid - 32, sh.rel[tid - 32]);
+      if (tid >= 32 && tid < 32 + p.k2) orientationOffsets(cc, move, kKindOrient, tid - 32, sh.rel[tid - 32]);
       __syncthreads();
-      if (!phase<QUINTIC>(p, sh, -1, atomGrid)) break;
+      if (!phase<QUINTIC>(-1)) break;
       if (tid < 32)
       {
         const int t = tid;
         const double lw = t < p.k1 ? -p.beta * sh.tot[t] - sh.logq[t] : 0.0;
         double W;
-        const int sel = warpSelect(lw, t < p.k1 && !ovlOf(sh, t), p.k1, urand(p, move, slot(kKindMove, 1, 0)).x, &W);
+        const int sel = warpSelect(lw, t < p.k1 && !ovlOf(sh, t), p.k1, urand(move, slot(kKindMove, 1, 0)).x, &W);
         if (tid == 0)
         {
           sh.selFirst = sel;
@@ -1283,10 +1297,10 @@ __global__ void __launch_bounds__(kThreads, 1) mixtureKernel(const __grid_consta
             sh.cq[tid][i] = cc.charges[i];
           }
           sh.cn[tid] = na;
-          storeOrientation(p, sh, atomGrid, cc, x, tid * (na - 1));
+          storeOrientation(cc, x, tid * (na - 1));
         }
         __syncthreads();
-        if (!phase<QUINTIC>(p, sh, -1, atomGrid)) break;
+        if (!phase<QUINTIC>(-1)) break;
         if (tid < 32)
         {
           const int per = na - 1, t = tid;
@@ -1299,7 +1313,7 @@ __global__ void __launch_bounds__(kThreads, 1) mixtureKernel(const __grid_consta
               o |= ovlOf(sh, t * per + i);
             }
           double W2;
-          const int sel = warpSelect(-p.beta * e, t < p.k2 && !o, p.k2, urand(p, move, slot(kKindMove, 2, 0)).x, &W2);
+          const int sel = warpSelect(-p.beta * e, t < p.k2 && !o, p.k2, urand(move, slot(kKindMove, 2, 0)).x, &W2);
           if (tid == 0 && sel >= 0 && sh.W * W2 >= 1e-150)
           {
             const double dEw = p.use_charge ? sh.tot[sh.nta + sel] + cc.self_excl : 0.0;
@@ -1320,17 +1334,17 @@ __global__ void __launch_bounds__(kThreads, 1) mixtureKernel(const __grid_consta
         __syncthreads();
         if (sh.accept)
         {
+          if (tid < 32) storeMolecule(sh.n, c, sh.mol);
           if (tid == 0)
           {
             const int m = sh.n;
-            storeMolecule(p, sh, m, c, sh.mol);
             gs.comp_of[m] = c;
             gs.slot[m] = sh.count[c];
             gs.list[c * p.capacity + sh.count[c]] = m;
             sh.count[c] += 1;
             sh.n += 1;
           }
-          if (p.use_charge) addCandidate(p, sh, dyk, sh.selOrient);
+          if (p.use_charge) addCandidate(sh.selOrient);
         }
       }
     }
@@ -1344,7 +1358,7 @@ __global__ void __launch_bounds__(kThreads, 1) mixtureKernel(const __grid_consta
       const int m = sh.m;
       if (tid < p.k1)
       {
-        const double3 r = tid == 0 ? loadPos(p, m * na + sb) : firstBeadPosition(p, cc, move, tid);
+        const double3 r = tid == 0 ? loadPos(p, m * na + sb) : firstBeadPosition(cc, move, tid);
         sh.ta[tid] = r;
         sh.tf[tid] = toFixed(p, r, cc.types[sb]);
         atomGrid[tid] = cc.vdw_grid[sb];
@@ -1381,11 +1395,11 @@ __global__ void __launch_bounds__(kThreads, 1) mixtureKernel(const __grid_consta
         if (tid == 0)
           for (int i = 0; i < na; ++i) x[i] = loadPos(p, m * na + i);
         else
-          orientedMolecule(p, cc, loadPos(p, m * na + sb), move, kKindOrient, tid, x);
-        storeOrientation(p, sh, atomGrid, cc, x, p.k1 + tid * (na - 1));
+          orientedMolecule(cc, loadPos(p, m * na + sb), move, kKindOrient, tid, x);
+        storeOrientation(cc, x, p.k1 + tid * (na - 1));
       }
       __syncthreads();
-      if (!phase<QUINTIC>(p, sh, m, atomGrid)) break;
+      if (!phase<QUINTIC>(m)) break;
       if (tid < 32)
       {
         // Rosenbluth weights of the retrace: first beads (trial 0 = the old bead) and orientations (trial 0 = the
@@ -1421,6 +1435,7 @@ __global__ void __launch_bounds__(kThreads, 1) mixtureKernel(const __grid_consta
       __syncthreads();
       if (sh.accept)
       {
+        if (tid < 32 && m != sh.n - 1) storeMolecule(m, sh.preCl, sh.preLast);
         if (tid == 0)
         {
           // remove m from its component list, then move the last molecule into slot m (from the values read before
@@ -1434,14 +1449,13 @@ __global__ void __launch_bounds__(kThreads, 1) mixtureKernel(const __grid_consta
           {
             const int cl = sh.preCl;
             const int sl = (lastC == last) ? k : sh.preSl;
-            storeMolecule(p, sh, m, cl, sh.preLast);
             gs.comp_of[m] = cl;
             gs.slot[m] = sl;
             gs.list[cl * p.capacity + sl] = m;
           }
           sh.n -= 1;
         }
-        if (p.use_charge) addCandidate(p, sh, dyk, 0);
+        if (p.use_charge) addCandidate(0);
       }
     }
     else if (kind == 4 && p.n_comp > 1)
@@ -1490,7 +1504,7 @@ __global__ void __launch_bounds__(kThreads, 1) mixtureKernel(const __grid_consta
         {
           const int t = tid;
           double3 x[kMaxAtoms];
-          orientedMolecule(p, cn, first, move, kKindNewOrient, t, x);
+          orientedMolecule(cn, first, move, kKindNewOrient, t, x);
           for (int i = 0; i < na; ++i)
           {
             sh.cpos[t][i] = x[i];
@@ -1499,7 +1513,7 @@ __global__ void __launch_bounds__(kThreads, 1) mixtureKernel(const __grid_consta
             sh.cq[t][na + i] = -co.charges[i];
           }
           sh.cn[t] = 2 * na;
-          storeOrientation(p, sh, atomGrid, cn, x, 1 + t * (na - 1));
+          storeOrientation(cn, x, 1 + t * (na - 1));
         }
         else if (tid < 2 * p.k2)
         {
@@ -1508,11 +1522,11 @@ __global__ void __launch_bounds__(kThreads, 1) mixtureKernel(const __grid_consta
           if (t == 0)
             for (int i = 0; i < na; ++i) x[i] = loadPos(p, m * na + i);
           else
-            orientedMolecule(p, co, first, move, kKindOldOrient, t, x);
-          storeOrientation(p, sh, atomGrid, co, x, base2 + 1 + t * (na - 1));
+            orientedMolecule(co, first, move, kKindOldOrient, t, x);
+          storeOrientation(co, x, base2 + 1 + t * (na - 1));
         }
         __syncthreads();
-        if (!phase<QUINTIC>(p, sh, m, atomGrid)) break;
+        if (!phase<QUINTIC>(m)) break;
         if (tid < 32)
         {
           const int per = na - 1;
@@ -1529,7 +1543,7 @@ __global__ void __launch_bounds__(kThreads, 1) mixtureKernel(const __grid_consta
               oo |= ovlOf(sh, base2 + 1 + t * per + i);
             }
           double Wn2, Wo2;
-          const int sel = warpSelect(-p.beta * e, t < p.k2 && !o, p.k2, urand(p, move, slot(kKindMove, 3, 0)).x, &Wn2);
+          const int sel = warpSelect(-p.beta * e, t < p.k2 && !o, p.k2, urand(move, slot(kKindMove, 3, 0)).x, &Wn2);
           warpSelect(-p.beta * eo, t < p.k2 && !oo, p.k2, 0.0, &Wo2);
           const double eSel = __shfl_sync(0xffffffffu, e, sel >= 0 ? sel : 0);
           const double e0 = eo;  // lane 0: the old molecule's own orientation
@@ -1554,9 +1568,9 @@ __global__ void __launch_bounds__(kThreads, 1) mixtureKernel(const __grid_consta
         __syncthreads();
         if (sh.accept)
         {
+          if (tid < 32) storeMolecule(m, newC, sh.mol);
           if (tid == 0)
           {
-            storeMolecule(p, sh, m, newC, sh.mol);
             // move m from the old component's list to the new one's (from the values read before the barrier)
             const int k = sh.preSlot, lastC = sh.preLastC;
             gs.list[oldC * p.capacity + k] = lastC;
@@ -1567,7 +1581,7 @@ __global__ void __launch_bounds__(kThreads, 1) mixtureKernel(const __grid_consta
             gs.list[newC * p.capacity + sh.count[newC]] = m;
             sh.count[newC] += 1;
           }
-          if (p.use_charge) addCandidate(p, sh, dyk, sh.selOrient);
+          if (p.use_charge) addCandidate(sh.selOrient);
         }
         c = oldC;
       }
