@@ -20,10 +20,18 @@
 // uniform azimuth (the reference's own comment at system.ixx:593-600 notes that this MC targets exp(-beta U_intra)
 // whatever its seed): a Gaussian proposal around theta0 accepted with probability sin(theta), 32 proposals per warp
 // round. This replaces a serial chain of 2*2*150 dependent updates per step by one warp vote.
+//
+// What bounds it: the latency of a move's chain of steps. Per step of a chain in the largest system of the benchmark's
+// batch (1,016 framework atoms, 8 beads, one CTA of 512 threads) in cycles: pairs 5,400 (issue), reductions 2,300, trial
+// positions 1,900, selection 2,000; and once per growth 21,000 for the torsion weights (FP64 pipe). 64 systems, 200 moves:
+// 7.5 ms with the spins' cosines from cospi, two exponentials and three more shuffles per selection, the displacements
+// scaled twice and the system's constants in global memory, now 6.7 ms. Listing the pairs within the cutoff per thread
+// and evaluating them together was slower (5,400 against 7,100 cycles: each round waits for a chain of loads).
 #include <cooperative_groups.h>
 
 #include <algorithm>
 #include <cmath>
+#include <climits>
 #include <cstring>
 #include <numeric>
 #include <vector>
@@ -108,7 +116,8 @@ struct Shared
 {
   float4 tab[kMaxTypes * kMaxTypes];
   int4 bead[kMaxTrials];  // beads evaluated (fixed point, .w = type)
-  double red[2][32 * kMaxWarps];  // per-thread framework / molecule partial sums
+  double red[2][kMaxWarps][kMaxTrials];  // per warp its framework / molecule sums per bead
+  SysDev sys;                            // the system, read throughout a move
   unsigned red_ovl[kMaxWarps];
   double xch[2][2 * kMaxTrials];  // per-CTA sums exchanged across the cluster (double-buffered)
   unsigned xch_ovl[2];
@@ -118,11 +127,12 @@ struct Shared
   double3 old[kMaxBeads];  // molecule being retraced or translated
   double3 dir[kMaxTrials];
   double tw[kMaxTrials];
-  double intra[kMaxTrials];
-  double theta[kMaxBeads], psi[kMaxBeads];   // base-conformation bend angle and azimuth / pi per step (insertion)
+  // base conformation per step (insertion): cosine and sine of the bend angle and of the azimuth; the random number that
+  // selects a direction
+  double ct[kMaxBeads], st[kMaxBeads], cp[kMaxBeads], sp[kMaxBeads], su[kMaxBeads];
   double tD[kMaxBeads];                      // retrace: cosine of the old dihedral at step j
   double ttw[kMaxBeads][kMaxTrials];         // torsion weight per step and direction
-  int tsel[kMaxBeads][kMaxTrials];           // selected spin per step and direction
+  uint32_t tword[kMaxBeads][kMaxTrials];     // random word of the selected spin per step and direction
   double W, eext, dU, stats[kStats];
   int fail, kind, m, axis, n, accept;
   unsigned long long pairs;
@@ -218,52 +228,67 @@ __device__ __noinline__ double internalEnergy(const Params& p, const SysDev& S, 
 // exp(lbf) (the Rosenbluth sum), and the index chosen by CBMC::selectTrialPosition (cbmc/util.cpp:14-47): the first
 // trial whose cumulative shifted Boltzmann factor reaches u times the total. retrace: trial 0 (the old position).
 // Returns -1 when every trial overlaps. Called by all 32 lanes of warp 0.
+// The shift of the Boltzmann factors is the largest exponent rounded to FP32 (one warp instruction; any shift near it
+// serves), and the trials are in the first kMaxTrials lanes.
 __device__ __forceinline__ int warpSelect(double lbf, bool ok, bool retrace, double u, double* sum)
 {
   const int lane = threadIdx.x & 31;
   const unsigned okMask = __ballot_sync(0xffffffffu, ok);
-  double mx = ok ? lbf : -1e300;
+  const int bits = __float_as_int(static_cast<float>(fmax(lbf, -1e38)));
+  const int key = __reduce_max_sync(0xffffffffu, ok ? (bits >= 0 ? bits : bits ^ 0x7fffffff) : INT_MIN);
+  const double mx = static_cast<double>(__int_as_float(key >= 0 ? key : key ^ 0x7fffffff));
+  double incl = ok ? exp(lbf - mx) : 0.0;
+  const double factor = exp(mx);
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  double direct = ok ? exp(lbf) : 0.0;
-  const double shifted = ok ? exp(lbf - mx) : 0.0;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) direct += __shfl_xor_sync(0xffffffffu, direct, o);
-  double incl = shifted;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1)
+  for (int o = 1; o < kMaxTrials; o <<= 1)
   {
     const double t = __shfl_up_sync(0xffffffffu, incl, o);
     if (lane >= o) incl += t;
   }
-  const double total = __shfl_sync(0xffffffffu, incl, 31);
-  *sum = direct;
+  const double total = __shfl_sync(0xffffffffu, incl, kMaxTrials - 1);
+  *sum = okMask == 0u ? 0.0 : factor * total;
   if (okMask == 0u) return -1;
   if (retrace) return 0;
   const unsigned hit = __ballot_sync(0xffffffffu, ok && incl >= u * total);
   return hit ? __ffs(hit) - 1 : 31 - __clz(okMask);
 }
 
+// The cell's matrix times 2^-32 (exact), for displacements in fixed point
+template <bool TRI>
+struct Cell32
+{
+  float h[TRI ? 9 : 3];
+  __device__ __forceinline__ explicit Cell32(const SysDev& S)
+  {
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+      if constexpr (TRI)
+        for (int r = 0; r < 3; ++r) h[3 * c + r] = S.hf[c][r] * kFix;
+      else
+        h[c] = S.hf[c][c] * kFix;
+  }
+};
+
 // Squared distance of bead B and partner P in FP32 from their exact fixed-point displacement (the uint32 wrap is the
 // minimum image).
 template <bool TRI>
-__device__ __forceinline__ float beadDistance2(const SysDev& S, int4 B, int4 P)
+__device__ __forceinline__ float beadDistance2(const Cell32<TRI>& C, int4 B, int4 P)
 {
-  const float f0 = static_cast<float>(static_cast<int>(static_cast<uint32_t>(B.x) - static_cast<uint32_t>(P.x))) * kFix;
-  const float f1 = static_cast<float>(static_cast<int>(static_cast<uint32_t>(B.y) - static_cast<uint32_t>(P.y))) * kFix;
-  const float f2 = static_cast<float>(static_cast<int>(static_cast<uint32_t>(B.z) - static_cast<uint32_t>(P.z))) * kFix;
+  const float f0 = static_cast<float>(static_cast<int>(static_cast<uint32_t>(B.x) - static_cast<uint32_t>(P.x)));
+  const float f1 = static_cast<float>(static_cast<int>(static_cast<uint32_t>(B.y) - static_cast<uint32_t>(P.y)));
+  const float f2 = static_cast<float>(static_cast<int>(static_cast<uint32_t>(B.z) - static_cast<uint32_t>(P.z)));
   float rx, ry, rz;
-  if (TRI)
+  if constexpr (TRI)
   {
-    rx = fmaf(S.hf[0][0], f0, fmaf(S.hf[1][0], f1, S.hf[2][0] * f2));
-    ry = fmaf(S.hf[0][1], f0, fmaf(S.hf[1][1], f1, S.hf[2][1] * f2));
-    rz = fmaf(S.hf[0][2], f0, fmaf(S.hf[1][2], f1, S.hf[2][2] * f2));
+    rx = fmaf(C.h[0], f0, fmaf(C.h[3], f1, C.h[6] * f2));
+    ry = fmaf(C.h[1], f0, fmaf(C.h[4], f1, C.h[7] * f2));
+    rz = fmaf(C.h[2], f0, fmaf(C.h[5], f1, C.h[8] * f2));
   }
   else
   {
-    rx = S.hf[0][0] * f0;
-    ry = S.hf[1][1] * f1;
-    rz = S.hf[2][2] * f2;
+    rx = C.h[0] * f0;
+    ry = C.h[1] * f1;
+    rz = C.h[2] * f2;
   }
   return fmaf(rx, rx, fmaf(ry, ry, rz * rz));
 }
@@ -292,15 +317,16 @@ __device__ __forceinline__ void beadPartners(const Shared& sh, const SysDev& S, 
                                              int begin, int n, int stride, int skip, float rc2, float ovlf,
                                              double& acc, unsigned& ovl, unsigned& inside, int b)
 {
+  const Cell32<TRI> C(S);
   const int bt = (B.w & 0xff) * kMaxTypes;
   int i = begin;
   for (; i + 3 * stride < n; i += 4 * stride)
   {
     const int4 P0 = partners[i], P1 = partners[i + stride], P2 = partners[i + 2 * stride], P3 = partners[i + 3 * stride];
-    const float r0 = SKIP && (P0.w >> 8) == skip ? INFINITY : beadDistance2<TRI>(S, B, P0);
-    const float r1 = SKIP && (P1.w >> 8) == skip ? INFINITY : beadDistance2<TRI>(S, B, P1);
-    const float r2 = SKIP && (P2.w >> 8) == skip ? INFINITY : beadDistance2<TRI>(S, B, P2);
-    const float r3 = SKIP && (P3.w >> 8) == skip ? INFINITY : beadDistance2<TRI>(S, B, P3);
+    const float r0 = SKIP && (P0.w >> 8) == skip ? INFINITY : beadDistance2<TRI>(C, B, P0);
+    const float r1 = SKIP && (P1.w >> 8) == skip ? INFINITY : beadDistance2<TRI>(C, B, P1);
+    const float r2 = SKIP && (P2.w >> 8) == skip ? INFINITY : beadDistance2<TRI>(C, B, P2);
+    const float r3 = SKIP && (P3.w >> 8) == skip ? INFINITY : beadDistance2<TRI>(C, B, P3);
     if (fminf(fminf(r0, r1), fminf(r2, r3)) < rc2)
     {
       beadPairEnergy(sh, bt, P0, r0, rc2, ovlf, acc, ovl, inside, b);
@@ -313,7 +339,7 @@ __device__ __forceinline__ void beadPartners(const Shared& sh, const SysDev& S, 
   {
     const int4 P = partners[i];
     if (SKIP && (P.w >> 8) == skip) continue;
-    beadPairEnergy(sh, bt, P, beadDistance2<TRI>(S, B, P), rc2, ovlf, acc, ovl, inside, b);
+    beadPairEnergy(sh, bt, P, beadDistance2<TRI>(C, B, P), rc2, ovlf, acc, ovl, inside, b);
   }
 }
 
@@ -360,8 +386,8 @@ __device__ __noinline__ void evalBeads(Shared& sh, const Params& p, const SysDev
   if (lane < nbd)
   {
     const int bb = (32 * warp + lane) % nbd;
-    sh.red[0][warp * kMaxTrials + bb] = afw;
-    sh.red[1][warp * kMaxTrials + bb] = amm;
+    sh.red[0][warp][bb] = afw;
+    sh.red[1][warp][bb] = amm;
   }
   inside = __reduce_add_sync(0xffffffffu, inside);
   if (lane == 0 && inside) atomicAdd(&sh.pairs, static_cast<unsigned long long>(inside));
@@ -375,7 +401,7 @@ __device__ __noinline__ void evalBeads(Shared& sh, const Params& p, const SysDev
   double sum = 0.0;
   const int which = tid >= kMaxTrials, bb = tid - which * kMaxTrials;
   if (tid < 2 * kMaxTrials && bb < nbd)
-    for (int w = 0; w < nw; ++w) sum += sh.red[which][w * kMaxTrials + bb];
+    for (int w = 0; w < nw; ++w) sum += sh.red[which][w][bb];
   unsigned octa = 0;
   if (tid == 2 * kMaxTrials)
     for (int w = 0; w < nw; ++w) octa |= sh.red_ovl[w];
@@ -426,11 +452,28 @@ __device__ __forceinline__ void spinAngle(uint32_t word, double* sa, double* ca)
   sincospi(2.0 * u - 1.0, sa, ca);
 }
 
-// TraPPE torsion energy from the torsion cosine (torsion_potential.cpp:464-473)
-__device__ __forceinline__ double trappe(const SysDev& S, double cp)
+__device__ __forceinline__ uint32_t wordOf(uint4 w, int k)
 {
-  const double* q = S.torsion;
-  return q[0] + (1.0 + cp) * (q[1] + q[3] - 2.0 * (cp - 1.0) * (q[2] - 2.0 * q[3] * cp));
+  return k < 2 ? (k == 0 ? w.x : w.y) : (k == 2 ? w.z : w.w);
+}
+
+// The cosine of a word's spin angle pi a, a in (-1, 1), for the torsion weights: with x = |a| - 1/2 it is -sin(pi x), an odd
+// polynomial on |x| <= 1/2 (Chebyshev interpolation of sin(pi x) / x in x^2 at nine nodes, 8e-19 off; in FP64 3.2e-16, as
+// cospi). Twelve FP64 instructions, a third of cospi's, whose pipe bounds the weights of a growth.
+__device__ __forceinline__ double spinCosine(uint32_t word)
+{
+  const double a = fma(static_cast<double>(word), 0x1.0p-31, 0x1.0p-32 - 1.0);
+  const double x = fabs(a) - 0.5, t = x * x;
+  double r = 7.697877575412416e-07;
+  r = fma(r, t, -2.1903489466044935e-05);
+  r = fma(r, t, 0.0004662998078202794);
+  r = fma(r, t, -0.0073704305030779715);
+  r = fma(r, t, 0.08214588657266207);
+  r = fma(r, t, -0.5992645293189114);
+  r = fma(r, t, 2.5501640398772993);
+  r = fma(r, t, -5.167712780049969);
+  r = fma(r, t, 3.141592653589793);
+  return -x * r;
 }
 
 // Signed dihedral (cos D, sin D) about the unit axis a = normalized(x2 - x3) of the position y grown from x3, with
@@ -464,6 +507,8 @@ __device__ __noinline__ void precomputeGrowth(Shared& sh, const Params& p, const
   const double beta = S.beta;
   const int nTheta = retrace ? 0 : max(0, nb - 2);
   const int nTors = max(0, nb - 2) * kd;  // steps j = 2..nb-1
+  // the numbers that select a direction at each step, by the warp that has the least to do
+  if (warp == nw - 1 && lane >= 1 && lane < nb) sh.su[lane] = urand(p, s, move, slot(kKindSelect, lane, 255, 0)).x;
   for (int task = warp; task < nTheta + nTors; task += nw)
   {
     if (task < nTheta)
@@ -488,8 +533,8 @@ __device__ __noinline__ void precomputeGrowth(Shared& sh, const Params& p, const
       }
       if (lane == 0)
       {
-        sh.theta[j] = theta;
-        sh.psi[j] = psi;
+        sincospi(psi, &sh.sp[j], &sh.cp[j]);
+        sincospi(theta / kPi, &sh.st[j], &sh.ct[j]);
       }
       continue;
     }
@@ -500,11 +545,16 @@ __device__ __noinline__ void precomputeGrowth(Shared& sh, const Params& p, const
       if (lane == 0)
       {
         sh.ttw[j][i] = 1.0;
-        sh.tsel[j][i] = static_cast<int>(urand(p, s, move, slot(kKindSelect, j, i, 0)).x * nt) % nt;
+        const int sel = static_cast<int>(urand(p, s, move, slot(kKindSelect, j, i, 0)).x * nt) % nt;
+        sh.tword[j][i] = wordOf(spinWords(p, s, move, j, i, sel >> 2), sel & 3);
       }
       continue;
     }
     // lane owns spins 4 lane .. 4 lane + 3 (one Philox draw, four 32-bit words)
+    // -beta U (TraPPE, torsion_potential.cpp:464-473) as a polynomial in the torsion's cosine
+    const double* q = S.torsion;
+    const double u3 = -4.0 * beta * q[3], u2 = 2.0 * beta * q[2];
+    const double u1 = beta * (3.0 * q[3] - q[1]), u0 = -beta * (q[0] + q[1] + 2.0 * q[2] + q[3]);
     double lbf[4];
     const uint4 w = spinWords(p, s, move, j, i, lane);
     const uint32_t words[4] = {w.x, w.y, w.z, w.w};
@@ -517,9 +567,9 @@ __device__ __noinline__ void precomputeGrowth(Shared& sh, const Params& p, const
       if (sp < nt)
       {
         const double cp = (retrace && i == 0 && sp == 0)
-                              ? sh.tD[j]
-                              : cospi(2.0 * ((static_cast<double>(words[k]) + 0.5) * 0x1.0p-32) - 1.0);
-        lbf[k] = -beta * trappe(S, fmin(1.0, fmax(-1.0, cp)));
+                              ? fmin(1.0, fmax(-1.0, sh.tD[j]))
+                              : spinCosine(words[k]);
+        lbf[k] = fma(fma(fma(u3, cp, u2), cp, u1), cp, u0);
         mx = fmax(mx, lbf[k]);
       }
     }
@@ -540,7 +590,7 @@ __device__ __noinline__ void precomputeGrowth(Shared& sh, const Params& p, const
       if (lane >= o) incl += v;
     }
     const double total = __shfl_sync(0xffffffffu, incl, 31);
-    int sel = 0;
+    uint32_t word = 0;
     if (!(retrace && i == 0))
     {
       const double target = urand(p, s, move, slot(kKindSelect, j, i, 0)).x * total;
@@ -559,12 +609,13 @@ __device__ __noinline__ void precomputeGrowth(Shared& sh, const Params& p, const
         }
         if (mine < 0) mine = min(4 * lane + 3, nt - 1);
       }
-      sel = __shfl_sync(0xffffffffu, mine, l);
+      const int sel = __shfl_sync(0xffffffffu, mine, l);
+      word = __shfl_sync(0xffffffffu, wordOf(w, sel & 3), sel >> 2);
     }
     if (lane == 0)
     {
       sh.ttw[j][i] = exp(mx) * total / static_cast<double>(nt);
-      sh.tsel[j][i] = sel;
+      sh.tword[j][i] = word;
     }
   }
 }
@@ -588,9 +639,7 @@ __device__ __noinline__ void stepTrials(Shared& sh, const Params& p, const SysDe
       const double3 h = fabs(a.x) < 0.6 ? d3(1, 0, 0) : (fabs(a.y) < 0.6 ? d3(0, 1, 0) : d3(0, 0, 1));
       const double3 e1 = normalized(cross(a, h));
       const double3 e2 = cross(a, e1);
-      double sp, cp, st, ct;
-      sincospi(sh.psi[j], &sp, &cp);
-      sincospi(sh.theta[j] / kPi, &st, &ct);
+      const double sp = sh.sp[j], cp = sh.cp[j], st = sh.st[j], ct = sh.ct[j];
       base = add(cur, scale(S.bond, add(scale(ct, a), scale(st, add(scale(cp, e1), scale(sp, e2))))));
     }
     double3 pos;
@@ -598,11 +647,8 @@ __device__ __noinline__ void stepTrials(Shared& sh, const Params& p, const SysDe
       pos = sh.old[j];
     else
     {
-      const int sel = sh.tsel[j][i];
-      const uint4 w = spinWords(p, s, move, j, i, sel >> 2);
-      const uint32_t words[4] = {w.x, w.y, w.z, w.w};
       double sphi, cphi;
-      spinAngle(words[sel & 3], &sphi, &cphi);
+      spinAngle(sh.tword[j][i], &sphi, &cphi);
       double sa = sphi, ca = cphi;  // step 2: any uniform angle (no dihedral)
       if (j >= 3)
       {
@@ -719,7 +765,7 @@ __device__ __noinline__ void growChain(Shared& sh, const Params& p, const SysDev
       const double intra = (ok && j >= 4) ? intraVdw(p, S, sh.x, j, sh.dir[tid]) : 0.0;
       const double lbf = ok ? -beta * (sh.efw[tid] + sh.emm[tid] + intra) : 0.0;
       double sum;
-      const int sel = warpSelect(lbf, ok, retrace, urand(p, s, move, slot(kKindSelect, j, 255, 0)).x, &sum);
+      const int sel = warpSelect(lbf, ok, retrace, sh.su[j], &sum);
       if (tid == 0)
       {
         sh.fail = (sel < 0) || (retrace && ((sh.ovl & 1u) != 0u));
@@ -743,6 +789,16 @@ __device__ __forceinline__ int4* dynamicBase(unsigned char* smem)
   return reinterpret_cast<int4*>(smem + ((sizeof(Shared) + 15) & ~static_cast<size_t>(15)));
 }
 
+// The system's constants into shared memory (from global memory each use would be a load of its own, behind the barriers
+// of a step)
+__device__ __forceinline__ void copySystem(Shared& sh, const SysDev& S)
+{
+  static_assert(sizeof(SysDev) % sizeof(int) == 0, "copied word by word");
+  for (int i = threadIdx.x; i < static_cast<int>(sizeof(SysDev) / sizeof(int)); i += blockDim.x)
+    reinterpret_cast<int*>(&sh.sys)[i] = reinterpret_cast<const int*>(&S)[i];
+  __syncthreads();
+}
+
 // The persistent Monte Carlo kernel: one cluster per system, `moves` move attempts per system.
 template <int T>
 __global__ void __launch_bounds__(T, 1) alkaneKernel(Params p, const int* __restrict__ order, int fw_cap, int moves)
@@ -754,7 +810,8 @@ __global__ void __launch_bounds__(T, 1) alkaneKernel(Params p, const int* __rest
   const int rank = static_cast<int>(cluster.block_rank()), C = static_cast<int>(cluster.num_blocks());
   const Cl cl{rank, C};
   const int s = order[blockIdx.x / C];
-  const SysDev& S = p.sys[s];
+  const SysDev& S = sh.sys;
+  copySystem(sh, p.sys[s]);
   int4* molS = fwS + fw_cap;
   const int tid = threadIdx.x;
   const int nb = S.nb;
@@ -936,7 +993,8 @@ __global__ void __launch_bounds__(128) beadKernel(Params p, int s, int fw_cap, c
   int4* fwS = dynamicBase(smem);
   int4* molS = fwS + fw_cap;
   const Cl cl{0, 1};
-  const SysDev& S = p.sys[s];
+  const SysDev& S = sh.sys;
+  copySystem(sh, p.sys[s]);
   const int tid = threadIdx.x;
   for (int i = tid; i < S.n_fw; i += blockDim.x) fwS[i] = p.fw[S.fw_offset + i];
   for (int i = tid; i < kMaxTypes * kMaxTypes; i += blockDim.x) sh.tab[i] = p.ljf[i];
@@ -966,7 +1024,8 @@ __global__ void __launch_bounds__(128) vacuumKernel(Params p, long long n, doubl
   extern __shared__ __align__(16) unsigned char smem[];
   Shared& sh = *reinterpret_cast<Shared*>(smem);
   const Cl cl{0, 1};
-  const SysDev& S = p.sys[0];
+  const SysDev& S = sh.sys;
+  copySystem(sh, p.sys[0]);
   const int tid = threadIdx.x, nb = S.nb;
   for (int i = tid; i < kMaxTypes * kMaxTypes; i += blockDim.x) sh.tab[i] = p.ljf[i];
   if (tid == 0) sh.pairs = 0ull;
