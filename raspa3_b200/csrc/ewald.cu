@@ -1452,7 +1452,7 @@ struct rg_ewald_batch
 namespace
 {
 constexpr int kBatchAtoms = 16;   // old + new atoms of one system's move
-constexpr int kBatchM = 4;        // consecutive |kz| of one thread (five spill at three blocks per SM)
+constexpr int kBatchM = 2;        // consecutive |kz| of one thread (five spill at three blocks per SM)
 
 // The upload of one call: n * stride atoms, n counts, n flags
 inline size_t batchUploadBytes(int n, int stride)
@@ -1473,9 +1473,10 @@ __host__ __device__ inline size_t batchSharedBytes(int stride, int kxm, int kym,
 // four FMAs for two k-vectors, and every z phasor is read by a whole warp at once. S(k) goes straight from HBM to the
 // thread that adds to it and back (rows by kz, see rg_ewald_batch): the bound is HBM, 32 bytes per k-vector. Before, a
 // thread took one k-vector at a time in list order and read two phasors per atom and k-vector from shared memory, whose
-// bandwidth bound it: 114 us for 1,184 systems of 8,124 k-vectors, now 81 us (47 us at the measured copy rate, were all
-// of S read and all of the trial S written through HBM).
-__global__ void __launch_bounds__(kThreads, 3) ewaldBatchDeltaKernel(
+// bandwidth bound it: 114 us for 1,184 systems of 8,124 k-vectors. With four |kz| per thread, whose sums came before the
+// loads of S, three blocks fitted on an SM: 88 us. With two, S loaded first, four blocks fit: 73 us (47 us at the measured
+// copy rate, were all of S read and all of the trial S written through HBM).
+__global__ void __launch_bounds__(kThreads, 4) ewaldBatchDeltaKernel(
     const int4* __restrict__ runs, int n_runs, const int* __restrict__ row_start, int64_t slots, int n_systems,
     const double* __restrict__ run_temp, double2* sk, const unsigned char* __restrict__ upload, int atom_stride, int kxm,
     int kym, int kzm, double* partial)
@@ -1522,6 +1523,19 @@ __global__ void __launch_bounds__(kThreads, 3) ewaldBatchDeltaKernel(
     const int4 run = runs[r];
     const int lo = static_cast<short>(run.w & 0xffff), hi = run.w >> 16;
     if (m0 > max(-lo, hi)) continue;
+    // S(k) first: its loads are in flight while the sums are formed
+    double2 sk[2][kBatchM];
+    int at[2][kBatchM];
+#pragma unroll
+    for (int sign = 0; sign < 2; ++sign)
+#pragma unroll
+      for (int m = 0; m < kBatchM; ++m)
+      {
+        const int kz = sign == 0 ? m0 + m : -(m0 + m);
+        const bool in = kz >= lo && kz <= hi && (sign == 0 || kz != 0);
+        at[sign][m] = in ? row_start[2 * (m0 + m) + sign] + r : -1;
+        sk[sign][m] = in ? __ldcs(S + at[sign][m]) : make_double2(0.0, 0.0);
+      }
     double pc[kBatchM], qs[kBatchM], ps[kBatchM], qc[kBatchM];
 #pragma unroll
     for (int m = 0; m < kBatchM; ++m) pc[m] = qs[m] = ps[m] = qc[m] = 0.0;
@@ -1553,23 +1567,13 @@ __global__ void __launch_bounds__(kThreads, 3) ewaldBatchDeltaKernel(
 #pragma unroll
     for (int sign = 0; sign < 2; ++sign)
     {
-      double2 s[kBatchM];
-      int at[kBatchM];
 #pragma unroll
       for (int m = 0; m < kBatchM; ++m)
-      {
-        const int kz = sign == 0 ? m0 + m : -(m0 + m);
-        const bool in = kz >= lo && kz <= hi && (sign == 0 || kz != 0);
-        at[m] = in ? row_start[2 * (m0 + m) + sign] + r : -1;
-        s[m] = in ? __ldcs(S + at[m]) : make_double2(0.0, 0.0);
-      }
-#pragma unroll
-      for (int m = 0; m < kBatchM; ++m)
-        if (at[m] >= 0)
+        if (at[sign][m] >= 0)
         {
           const double dx = sign == 0 ? pc[m] : qs[m], dy = sign == 0 ? ps[m] : qc[m];
-          e += run_temp[(2 * (m0 + m) + sign) * n_runs + r] * (2.0 * (s[m].x * dx + s[m].y * dy) + (dx * dx + dy * dy));
-          __stcs(T + at[m], make_double2(s[m].x + dx, s[m].y + dy));
+          e += run_temp[(2 * (m0 + m) + sign) * n_runs + r] * (2.0 * (sk[sign][m].x * dx + sk[sign][m].y * dy) + (dx * dx + dy * dy));
+          __stcs(T + at[sign][m], make_double2(sk[sign][m].x + dx, sk[sign][m].y + dy));
         }
     }
   }
@@ -1659,10 +1663,11 @@ rg_status rg_ewald_batch_create(rg_ewald* e, int n_systems, rg_ewald_batch** out
   if (!err)
     err = cudaMemcpyAsync(b->run_temp, run_temp.data(), sizeof(double) * run_temp.size(), cudaMemcpyHostToDevice, ctx->stream);
   // Blocks per system: as many as there are groups of kThreads items when the systems are few; for many systems fewer, so
-  // that a block's phasor tables serve more k-vectors (about eight blocks per place on the GPU remain)
+  // that a block's phasor tables serve more k-vectors (four blocks per place on the GPU remain: 1,184 systems of 3,609 and
+  // of 8,124 k-vectors take 40.4 and 72.8 us, with six 44.5 and 73.2; 700 systems 31.8 and 50.3, with two 34.1 and 60.6)
   const int64_t items = static_cast<int64_t>(b->n_runs) * ((e->ff.kmax_z + kBatchM) / kBatchM);
   const int64_t most = std::max<int64_t>(1, (items + kThreads - 1) / kThreads);
-  b->blocks = static_cast<int>(std::min<int64_t>(most, std::max<int64_t>(1, 24LL * e->sms / n_systems)));
+  b->blocks = static_cast<int>(std::min<int64_t>(most, std::max<int64_t>(1, 16LL * e->sms / n_systems)));
   if (!err) err = cudaMalloc(reinterpret_cast<void**>(&b->slot_of), sizeof(int) * slot_of.size());
   if (!err) err = cudaMemcpyAsync(b->slot_of, slot_of.data(), sizeof(int) * slot_of.size(), cudaMemcpyHostToDevice, ctx->stream);
   if (!err) err = cudaMalloc(reinterpret_cast<void**>(&b->row_start), sizeof(int) * rows);

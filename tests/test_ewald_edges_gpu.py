@@ -103,7 +103,7 @@ def test_difference(ctx, oracle, kmax, sphere, cell, new, old, groups):
 
 @pytest.mark.parametrize("kmax,sphere,systems", [((1, 1, 1), False, 1), ((3, 3, 13), False, 2), ((6, 6, 3), True, 5)])
 def test_batch(ctx, oracle, kmax, sphere, systems):
-    """One system and few; groups of four |kz| that the runs do not fill; atom counts of every parity. The batch gives the
+    """One system and few; groups of |kz| that the runs do not fill; atom counts of every parity. The batch gives the
     Fourier sum alone: the oracle's correction for a change of the net charge is taken off."""
     ff = forcefield(kmax, sphere)
     ew = native.Ewald(ctx, ff, BOX)
