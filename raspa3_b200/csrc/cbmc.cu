@@ -71,10 +71,9 @@ struct rg_system
   rg_trial_energy* out = nullptr;
   int out_cap = 0;
   rg_atom* trials_host = nullptr;     // pinned
-  rg_trial_energy* out_host = nullptr;    // mapped pinned: the last CTA of each trial writes its result here directly
-  rg_trial_energy* out_mapped = nullptr;  // device view of out_host
-  unsigned int* flag_host = nullptr;      // mapped pinned: the number of the last call whose results are complete
-  unsigned int* flag_mapped = nullptr;
+  ulonglong2* out_host = nullptr;     // mapped pinned: the last CTA of each trial posts its result here (rg::collect)
+  ulonglong2* out_mapped = nullptr;   // device view of out_host
+  int out_trials = 0;                 // trials it has room for
   unsigned int calls = 0;
   int precision = RG_PRECISION_FP64;      // of rg_cbmc_external_energies
   int sms = 148;
@@ -120,10 +119,9 @@ struct TrialArgs
   int chunk;               // partner atoms per CTA
   int fw_partners;         // framework atoms scanned (0 if every trial atom has a grid)
   double* partial;         // [trial][chunk][kNumOut + 1]
-  unsigned int* counters;  // per trial, and (the last) the finished trials
-  rg_trial_energy* out;
-  unsigned int* flag;      // set to flag_value once every trial's result is written
-  unsigned int flag_value;
+  unsigned int* counters;  // per trial
+  ulonglong2* out;         // [trial][kNumOut + 1] results, posted with the number of the call
+  unsigned int call;
   // two trial sets of counts[t] atoms (stored atoms_per_trial apart) with their own squared cutoffs (framework VDW,
   // molecule VDW, Coulomb); otherwise every set has atoms_per_trial atoms and the cutoffs above
   int paired;
@@ -436,11 +434,11 @@ __global__ void __launch_bounds__(kThreads) trialEnergyKernel(TrialArgs a, Trial
     double x = 0.0;
     for (int w = 0; w < kThreads / 32; ++w) x = (c < kNumOut) ? x + red[w][c] : fmax(x, red[w][c]);
     a.partial[(static_cast<long long>(trial) * a.n_chunks + chunk) * (kNumOut + 1) + c] = x;
-    __threadfence();
   }
   __syncthreads();
   if (threadIdx.x == 0)
   {
+    __threadfence();  // of the CTA's stores, which the barrier has put before it
     const unsigned int done = atomicAdd(a.counters + trial, 1u);
     last = (done == static_cast<unsigned int>(a.n_chunks - 1));
   }
@@ -451,7 +449,6 @@ __global__ void __launch_bounds__(kThreads) trialEnergyKernel(TrialArgs a, Trial
   // together), then each channel's 16 sub-sums in order
   static_assert(kThreads == 16 * 16 && kNumOut + 1 <= 16, "16 threads for each of at most 16 channels");
   __shared__ double sub[kNumOut + 1][16];
-  __shared__ double tot[kNumOut + 1];
   const int cc = threadIdx.x >> 4, j0 = threadIdx.x & 15;
   if (cc <= kNumOut)
   {
@@ -470,34 +467,24 @@ __global__ void __launch_bounds__(kThreads) trialEnergyKernel(TrialArgs a, Trial
   {
     double x = 0.0;
     for (int j = 0; j < 16; ++j) x = (c < kNumOut) ? x + sub[c][j] : fmax(x, sub[c][j]);
-    tot[c] = x;
+    rg::post(a.out + trial * (kNumOut + 1) + c, x, a.call);
   }
-  __syncthreads();
-  if (threadIdx.x == 0)
-  {
-    rg_trial_energy o;
-    o.framework_vdw = tot[0];
-    o.framework_charge = tot[1];
-    o.molecule_vdw = tot[2];
-    o.molecule_charge = tot[3];
-    for (int g = 0; g < 4; ++g)
-    {
-      o.dudlambda_vdw[g] = tot[4 + g];
-      o.dudlambda_charge[g] = tot[8 + g];
-    }
-    o.external_field_vdw = tot[12];
-    o.overlap = static_cast<int32_t>(tot[kNumOut]);  // 0, 1 (overlap) or 2 (blocked pocket)
-    o.pad = 0;
-    a.out[trial] = o;
-    a.counters[trial] = 0u;
-    // the last trial to finish reports the call's end
-    __threadfence_system();
-    if (atomicAdd(a.counters + gridDim.x, 1u) == gridDim.x - 1)
-    {
-      a.counters[gridDim.x] = 0u;
-      rg::raiseFlag(a.flag, a.flag_value);
-    }
-  }
+  if (threadIdx.x == 0) a.counters[trial] = 0u;
+}
+
+// Room for the results of n trials, of no call yet
+cudaError_t growResults(rg_system* s, int n)
+{
+  if (s->out_host) cudaFreeHost(s->out_host);
+  s->out_host = nullptr;
+  s->out_trials = 0;
+  const size_t bytes = sizeof(ulonglong2) * (kNumOut + 1) * static_cast<size_t>(n);
+  cudaError_t err = cudaHostAlloc(reinterpret_cast<void**>(&s->out_host), bytes, cudaHostAllocMapped);
+  if (!err) err = cudaHostGetDevicePointer(reinterpret_cast<void**>(&s->out_mapped), s->out_host, 0);
+  if (err) return err;
+  std::memset(s->out_host, 0, bytes);
+  s->out_trials = n;
+  return cudaSuccess;
 }
 
 template <typename T>
@@ -552,12 +539,7 @@ rg_status rg_system_create(rg_ctx* ctx, const rg_forcefield* ff, const rg_box* b
   }
   if (!err) err = cudaStreamSynchronize(ctx->stream);
   if (!err) err = cudaMallocHost(reinterpret_cast<void**>(&s->trials_host), sizeof(rg_atom) * 4096);
-  if (!err)
-    err = cudaHostAlloc(reinterpret_cast<void**>(&s->out_host), sizeof(rg_trial_energy) * 4096, cudaHostAllocMapped);
-  if (!err) err = cudaHostGetDevicePointer(reinterpret_cast<void**>(&s->out_mapped), s->out_host, 0);
-  if (!err) err = cudaHostAlloc(reinterpret_cast<void**>(&s->flag_host), sizeof(unsigned int), cudaHostAllocMapped);
-  if (!err) err = cudaHostGetDevicePointer(reinterpret_cast<void**>(&s->flag_mapped), s->flag_host, 0);
-  if (!err) *s->flag_host = 0u;
+  if (!err) err = growResults(s, 64);
   if (!err) err = cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, ctx->device);
   if (err)
   {
@@ -611,7 +593,6 @@ rg_status rg_system_destroy(rg_system* s)
   if (s->ext_grid_owned) cudaFree(s->ext_grid);
   if (s->trials_host) cudaFreeHost(s->trials_host);
   if (s->out_host) cudaFreeHost(s->out_host);
-  if (s->flag_host) cudaFreeHost(s->flag_host);
   delete s;
   return RG_OK;
 }
@@ -760,12 +741,17 @@ rg_status runTrials(rg_system* s, const TrialCall& c, rg_trial_energy* out)
   const bool inParams = nt_atoms <= kParamTrialAtoms;
   if (!inParams) st = growDevice(ctx, &s->trials, &s->trial_cap, nt_atoms);
   if (!st) st = growDevice(ctx, &s->partial, &s->partial_cap, n_trials * n_chunks * (kNumOut + 1));
-  if (!st && s->counter_cap < n_trials + 1)
+  if (!st && s->counter_cap < n_trials)
   {
-    st = growDevice(ctx, &s->counters, &s->counter_cap, n_trials + 1);
+    st = growDevice(ctx, &s->counters, &s->counter_cap, n_trials);
     if (!st) RG_CUDA(ctx, cudaMemsetAsync(s->counters, 0, sizeof(unsigned int) * s->counter_cap, ctx->stream));
   }
   if (st) return st;
+  if (s->out_trials < n_trials)
+  {
+    RG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    RG_CUDA(ctx, growResults(s, 2 * n_trials));
+  }
   TrialParam small{};
   if (inParams)
     std::memcpy(small.a, c.trials, sizeof(rg_atom) * nt_atoms);
@@ -803,8 +789,7 @@ rg_status runTrials(rg_system* s, const TrialCall& c, rg_trial_energy* out)
   a.partial = s->partial;
   a.counters = s->counters;
   a.out = s->out_mapped;
-  a.flag = s->flag_mapped;
-  a.flag_value = ++s->calls;
+  a.call = ++s->calls;
   a.paired = c.paired ? 1 : 0;
   for (int t = 0; t < 2; ++t)
   {
@@ -826,9 +811,24 @@ rg_status runTrials(rg_system* s, const TrialCall& c, rg_trial_energy* out)
   dim3 grid(n_trials, n_chunks);
   kernel<<<grid, kThreads, 0, ctx->stream>>>(a, small);
   RG_CUDA(ctx, cudaGetLastError());
-  // the last CTA of each trial wrote its result into mapped pinned memory
-  if (rg_status ws = rg::waitFlag(ctx, s->flag_host, a.flag_value, c.what)) return ws;
-  std::memcpy(out, s->out_host, sizeof(rg_trial_energy) * n_trials);
+  for (int t = 0; t < n_trials; ++t)
+  {
+    double v[kNumOut + 1];
+    if (rg_status ws = rg::collect(ctx, s->out_host + t * (kNumOut + 1), kNumOut + 1, a.call, v, c.what)) return ws;
+    rg_trial_energy& o = out[t];
+    o.framework_vdw = v[0];
+    o.framework_charge = v[1];
+    o.molecule_vdw = v[2];
+    o.molecule_charge = v[3];
+    for (int g = 0; g < 4; ++g)
+    {
+      o.dudlambda_vdw[g] = v[4 + g];
+      o.dudlambda_charge[g] = v[8 + g];
+    }
+    o.external_field_vdw = v[12];
+    o.overlap = static_cast<int32_t>(v[kNumOut]);  // 0, 1 (overlap) or 2 (blocked pocket)
+    o.pad = 0;
+  }
   return RG_OK;
 }
 

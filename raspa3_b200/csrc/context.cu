@@ -47,22 +47,32 @@ bool supercellClip(const HostBox& b, double rc, double cutoff, double h[3], doub
   return clip;
 }
 
-rg_status waitFlag(rg_ctx* ctx, const volatile unsigned int* flag, unsigned int value, const char* what)
+rg_status collect(rg_ctx* ctx, const ulonglong2* from, int n, unsigned int call, double* out, const char* what)
 {
-  for (unsigned spins = 1; *flag != value; ++spins)
+  const volatile unsigned long long* words = reinterpret_cast<const volatile unsigned long long*>(from);
+  for (int i = 0; i < n; ++i)
   {
-    if ((spins & 0x3ff) != 0)
+    unsigned long long lo, hi;
+    bool idle = false;  // the stream was seen idle: what has not arrived then never will
+    for (unsigned spins = 1;; ++spins)
     {
-      __builtin_ia32_pause();
-      continue;
+      lo = words[2 * i];
+      hi = words[2 * i + 1];
+      if (lo >> 32 == call && hi >> 32 == call) break;
+      if (idle) return fail(ctx, RG_ERR_CUDA, std::string(what) + ": the kernel did not report");
+      if ((spins & 0x3ff) != 0)
+      {
+        __builtin_ia32_pause();
+        continue;
+      }
+      const cudaError_t err = cudaStreamQuery(ctx->stream);
+      if (err == cudaErrorNotReady) continue;
+      if (err != cudaSuccess) return cudaFail(ctx, err, what);
+      idle = true;
     }
-    const cudaError_t err = cudaStreamQuery(ctx->stream);
-    if (err == cudaErrorNotReady) continue;
-    if (err != cudaSuccess) return cudaFail(ctx, err, what);
-    // the stream is idle: the flag is set, unless the kernel never ran
-    if (*flag != value) return fail(ctx, RG_ERR_CUDA, std::string(what) + ": the kernel did not report");
+    const unsigned long long v = (lo & 0xffffffffull) | (hi << 32);
+    std::memcpy(out + i, &v, sizeof(double));
   }
-  __atomic_thread_fence(__ATOMIC_ACQUIRE);
   return RG_OK;
 }
 

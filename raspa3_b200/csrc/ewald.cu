@@ -43,7 +43,7 @@ struct rg_ewald
   double2* trial = nullptr;    // nk*(1+G)
   double* partial = nullptr;   // per-block partial sums
   unsigned int* counter = nullptr;
-  double* result = nullptr;    // 1 + G doubles (+ spare): device view of result_host (mapped pinned memory)
+  ulonglong2* result = nullptr;  // 1 + G results and (from kTermsAt) the atoms' terms: device view of result_host
   // the k-vectors by (kx, ky) pair: the pairs, and per pair the index of the k-vector with kz = -kmax_z..kmax_z (-1:
   // not in the set)
   int n_pairs = 0;
@@ -55,9 +55,7 @@ struct rg_ewald
   // staging of the last staged atoms: the context's scratch, set anew by each call that stages (stageRoom)
   void* moved = nullptr;
   void* moved_host = nullptr;
-  double* result_host = nullptr;  // mapped pinned: the kernels' last block writes the totals here directly
-  unsigned int* flag_host = nullptr;  // mapped pinned: the number of the last call whose totals are complete
-  unsigned int* flag = nullptr;
+  ulonglong2* result_host = nullptr;  // mapped pinned: the kernels' last blocks post the totals here (rg::collect)
   unsigned int calls = 0;
 };
 
@@ -82,27 +80,6 @@ struct MovedParam
 {
   MovedAtom a[kParamMoved];
 };
-
-// How a call's kernels tell the host that its totals are written: the last of `parts` reports raises the flag
-struct Report
-{
-  unsigned int* done;  // reports so far, when there is more than one part
-  unsigned int parts;
-  unsigned int* flag;
-  unsigned int value;
-};
-
-// By one thread, after a part's totals have been written (and, if by several threads, made visible to it)
-__device__ __forceinline__ void report(const Report& r)
-{
-  if (r.parts > 1)
-  {
-    __threadfence_system();
-    if (atomicAdd(r.done, 1u) != r.parts - 1) return;
-    *r.done = 0u;
-  }
-  rg::raiseFlag(r.flag, r.value);
-}
 
 // Sum of v over the block, complete in thread 0
 template <int G>
@@ -133,7 +110,7 @@ __device__ __forceinline__ void blockSum(double (&v)[1 + G], double (*red)[1 + k
 
 template <int G>
 __device__ __forceinline__ void blockReduceAndFinish(double (&v)[1 + G], double* partial, unsigned int* counter,
-                                                     double* result, const Report& done, unsigned n_blocks,
+                                                     ulonglong2* result, unsigned call, unsigned n_blocks,
                                                      unsigned block)
 {
   __shared__ double red[kThreads / 32][1 + kMaxGroups];
@@ -165,9 +142,8 @@ __device__ __forceinline__ void blockReduceAndFinish(double (&v)[1 + G], double*
   if (threadIdx.x == 0)
   {
 #pragma unroll
-    for (int c = 0; c < 1 + G; ++c) result[c] = v[c];
+    for (int c = 0; c < 1 + G; ++c) rg::post(result + c, v[c], call);
     *counter = 0u;  // ready for the next launch on this system
-    report(done);
   }
 }
 
@@ -190,7 +166,7 @@ __global__ void __launch_bounds__(kThreads) ewaldDeltaKernel(int nk, int kxm, in
                                                              const MovedAtom* __restrict__ moved,
                                                              const __grid_constant__ MovedParam small, int n_moved,
                                                              int tile, double* partial, unsigned int* counter,
-                                                             double* result, Report done)
+                                                             ulonglong2* result, unsigned call)
 {
   extern __shared__ double2 tab[];  // [tile][stride]
   __shared__ MovedAtom sm[kDeltaTile];
@@ -273,7 +249,7 @@ __global__ void __launch_bounds__(kThreads) ewaldDeltaKernel(int nk, int kxm, in
       trial[row + 1 + g] = TG;
     }
   }
-  blockReduceAndFinish<G>(v, partial, counter, result, done, gridDim.x, blockIdx.x);
+  blockReduceAndFinish<G>(v, partial, counter, result, call, gridDim.x, blockIdx.x);
 }
 
 // Partial sums of the structure factor of one chunk of atoms, for one (kx, ky) pair per thread and MT consecutive values
@@ -364,7 +340,7 @@ struct TermsParams
   int n_atoms, blocks;      // blocks = 0: none
   double* partial;          // [blocks][kTerms]
   unsigned int* counter;
-  double* result;
+  ulonglong2* result;
   double cell[9];           // c[col][row] by columns
   int triclinic;
   double alpha, coul, self;  // self = C alpha / sqrt(pi)
@@ -379,7 +355,7 @@ __device__ __forceinline__ void addToGroup(double* v, int g, double x)
   for (int k = 0; k < kMaxGroups; ++k)
     if (g == k + 1) v[k] += x;
 }
-__device__ __forceinline__ void atomTerms(const TermsParams& p, int omit_inter, int block, const Report& done)
+__device__ __forceinline__ void atomTerms(const TermsParams& p, int omit_inter, int block, unsigned call)
 {
   const MovedAtom* __restrict__ atoms = p.atoms;
   const int n_atoms = p.n_atoms, n_blocks = p.blocks;
@@ -444,10 +420,13 @@ __device__ __forceinline__ void atomTerms(const TermsParams& p, int omit_inter, 
     double x = 0.0;
     for (int w = 0; w < kThreads / 32; ++w) x += red[w][threadIdx.x];
     p.partial[block * kTerms + threadIdx.x] = x;
-    __threadfence();
   }
   __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(p.counter, 1u) == static_cast<unsigned>(n_blocks - 1);
+  if (threadIdx.x == 0)
+  {
+    __threadfence();  // of the block's stores, which the barrier has put before it
+    last = atomicAdd(p.counter, 1u) == static_cast<unsigned>(n_blocks - 1);
+  }
   __syncthreads();
   if (!last) return;
   __threadfence();
@@ -458,18 +437,9 @@ __device__ __forceinline__ void atomTerms(const TermsParams& p, int omit_inter, 
     for (int b = lane; b < n_blocks; b += 32) x += __ldcg(p.partial + b * kTerms + c);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (lane == 0)
-    {
-      p.result[c] = x;
-      __threadfence_system();
-    }
+    if (lane == 0) rg::post(p.result + c, x, call);
   }
-  __syncthreads();
-  if (threadIdx.x == 0)
-  {
-    *p.counter = 0u;
-    report(done);
-  }
+  if (threadIdx.x == 0) *p.counter = 0u;
 }
 
 // The chunks' sums of one (pair, m) added in a fixed order by kFinishLanes threads (a warp covers 4 neighbouring pairs),
@@ -484,12 +454,12 @@ __global__ void __launch_bounds__(kThreads) ewaldPairFinishKernel(int n_pairs, i
                                                                   const double* __restrict__ temp, double2* s_rigid,
                                                                   double2* __restrict__ stored, int omit_inter,
                                                                   double* partial, unsigned int* counter,
-                                                                  double* result, TermsParams terms, Report done)
+                                                                  ulonglong2* result, TermsParams terms, unsigned call)
 {
   if constexpr (!RIGID)
     if (static_cast<int>(blockIdx.x) < terms.blocks)
     {
-      atomTerms(terms, omit_inter, blockIdx.x, done);
+      atomTerms(terms, omit_inter, blockIdx.x, call);
       return;
     }
   const unsigned block = blockIdx.x - terms.blocks;
@@ -548,13 +518,13 @@ __global__ void __launch_bounds__(kThreads) ewaldPairFinishKernel(int n_pairs, i
     }
   }
   if constexpr (!RIGID)
-    blockReduceAndFinish<0>(e, partial, counter, result, done, gridDim.x - terms.blocks, block);
+    blockReduceAndFinish<0>(e, partial, counter, result, call, gridDim.x - terms.blocks, block);
 }
 
 // The atoms' own terms by themselves (no k-vectors, or dU/dlambda groups, whose Fourier sums take the kernels below)
-__global__ void __launch_bounds__(kThreads) ewaldAtomTermsKernel(TermsParams p, int omit_inter, Report done)
+__global__ void __launch_bounds__(kThreads) ewaldAtomTermsKernel(TermsParams p, int omit_inter, unsigned call)
 {
-  atomTerms(p, omit_inter, blockIdx.x, done);
+  atomTerms(p, omit_inter, blockIdx.x, call);
 }
 
 // With dU/dlambda groups: per-atom phase tables e^{i 2 pi m s_d}, m = 0..kmax_d, built in shared memory for a tile of
@@ -646,7 +616,7 @@ __global__ void __launch_bounds__(kThreads) ewaldFullFinishKernel(int64_t nk, in
                                                                   const double2* __restrict__ s_rigid,
                                                                   double2* __restrict__ stored, int omit_inter,
                                                                   double* partial, unsigned int* counter,
-                                                                  double* result, Report done)
+                                                                  ulonglong2* result, unsigned call)
 {
   const int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   double v[1 + G];
@@ -685,7 +655,7 @@ __global__ void __launch_bounds__(kThreads) ewaldFullFinishKernel(int64_t nk, in
       stored[k * (1 + G) + 1 + g] = accg[g];
     }
   }
-  blockReduceAndFinish<G>(v, partial, counter, result, done, gridDim.x, blockIdx.x);
+  blockReduceAndFinish<G>(v, partial, counter, result, call, gridDim.x, blockIdx.x);
 }
 
 inline int groupOf(const rg_atom& a) { return a.group_fractional & 0x0f; }
@@ -832,9 +802,6 @@ rg_status stageAtoms(rg_ewald* e, const rg_atom* old_atoms, int n_old, const rg_
   return RG_OK;
 }
 
-// The report of a call in `parts` parts
-Report nextReport(rg_ewald* e, unsigned int parts) { return Report{e->counter + 2, parts, e->flag, ++e->calls}; }
-
 template <int G>
 cudaError_t launchDelta(rg_ewald* e, int n_moved, const MovedParam* small)
 {
@@ -843,14 +810,14 @@ cudaError_t launchDelta(rg_ewald* e, int n_moved, const MovedParam* small)
   const int tile = std::max(1, std::min({kDeltaTile, n_moved, static_cast<int>(kDeltaShared / per_atom)}));
   ewaldDeltaKernel<G><<<(nk + kThreads - 1) / kThreads, kThreads, per_atom * tile, e->ctx->stream>>>(
       nk, kxm, kym, kzm, e->kvec, e->temp, e->stored, e->trial, small ? nullptr : static_cast<const MovedAtom*>(e->moved),
-      small ? *small : MovedParam{}, n_moved, tile, e->partial, e->counter, e->result, nextReport(e, 1));
+      small ? *small : MovedParam{}, n_moved, tile, e->partial, e->counter, e->result, ++e->calls);
   return cudaGetLastError();
 }
 
 // Pair sums and their finish over the staged atoms, for the framework (rigid) or the adsorbates. A block holds up to
 // kPairWarps warps of pairs; the atoms are cut into chunks so that the blocks fill every SM once (as many narrow blocks
 // per SM as make up kPairWarps warps), with at least 8 atoms each.
-rg_status launchPairs(rg_ewald* e, int n_atoms, bool rigid, const TermsParams& terms, const Report& done)
+rg_status launchPairs(rg_ewald* e, int n_atoms, bool rigid, const TermsParams& terms, unsigned call)
 {
   cudaStream_t stream = e->ctx->stream;
   const int kxm = e->ff.kmax_x, kym = e->ff.kmax_y, kzm = e->ff.kmax_z;
@@ -906,17 +873,17 @@ rg_status launchPairs(rg_ewald* e, int n_atoms, bool rigid, const TermsParams& t
   if (rigid)
     ewaldPairFinishKernel<true><<<blocks, kThreads, 0, stream>>>(e->n_pairs, kzm, n_chunks, sums, e->kmap, e->temp,
                                                                 e->s_rigid, nullptr, 0, nullptr, nullptr, nullptr, terms,
-                                                                done);
+                                                                call);
   else
     ewaldPairFinishKernel<false><<<blocks + terms.blocks, kThreads, 0, stream>>>(
         e->n_pairs, kzm, n_chunks, sums, e->kmap, e->temp, e->s_rigid, e->stored, e->omit_inter ? 1 : 0,
-        e->partial, e->counter, e->result, terms, done);
+        e->partial, e->counter, e->result, terms, call);
   RG_CUDA(e->ctx, cudaGetLastError());
   return RG_OK;
 }
 
 template <int G>
-rg_status launchFull(rg_ewald* e, int n_atoms, const Report& done)
+rg_status launchFull(rg_ewald* e, int n_atoms, unsigned call)
 {
   // atoms split into chunks so that k-blocks x chunks fill the GPU (about four CTAs per SM), at least one tile each
   const int blocks = static_cast<int>((e->nk + kThreads - 1) / kThreads);
@@ -940,18 +907,11 @@ rg_status launchFull(rg_ewald* e, int n_atoms, const Report& done)
     cudaMemsetAsync(sums, 0, need, e->ctx->stream);
   ewaldFullFinishKernel<G><<<blocks, kThreads, 0, e->ctx->stream>>>(e->nk, n_chunks, sums, e->temp, e->s_rigid,
                                                                     e->stored, e->omit_inter ? 1 : 0, e->partial,
-                                                                    e->counter, e->result, done);
+                                                                    e->counter, e->result, call);
   RG_CUDA(e->ctx, cudaGetLastError());
   return RG_OK;
 }
 
-// The totals of the call whose kernels raise the flag to `value`
-rg_status readResult(rg_ewald* e, unsigned int value, double* out, int n, const char* what)
-{
-  if (rg_status st = rg::waitFlag(e->ctx, e->flag_host, value, what)) return st;
-  std::memcpy(out, e->result_host, sizeof(double) * n);
-  return RG_OK;
-}
 }  // namespace
 
 extern "C"
@@ -1039,11 +999,9 @@ rg_status rg_ewald_create(rg_ctx* ctx, const rg_forcefield* ff, const rg_box* bo
     err = cudaMemcpyAsync(e->kmap, e->kmap_host.data(), sizeof(int) * e->kmap_host.size(), cudaMemcpyHostToDevice,
                           ctx->stream);
   if (!err)
-    err = cudaHostAlloc(reinterpret_cast<void**>(&e->result_host), sizeof(double) * (kTermsAt + kTerms), cudaHostAllocMapped);
+    err = cudaHostAlloc(reinterpret_cast<void**>(&e->result_host), sizeof(ulonglong2) * (kTermsAt + kTerms), cudaHostAllocMapped);
   if (!err) err = cudaHostGetDevicePointer(reinterpret_cast<void**>(&e->result), e->result_host, 0);
-  if (!err) err = cudaHostAlloc(reinterpret_cast<void**>(&e->flag_host), sizeof(unsigned int), cudaHostAllocMapped);
-  if (!err) err = cudaHostGetDevicePointer(reinterpret_cast<void**>(&e->flag), e->flag_host, 0);
-  if (!err) *e->flag_host = 0u;
+  if (!err) std::memset(e->result_host, 0, sizeof(ulonglong2) * (kTermsAt + kTerms));
   if (!err) err = cudaDeviceGetAttribute(&e->sms, cudaDevAttrMultiProcessorCount, ctx->device);
   if (!err && e->nk > 0)
     err = cudaMemcpyAsync(e->kvec, kv.data(), sizeof(char4) * e->nk, cudaMemcpyHostToDevice, ctx->stream);
@@ -1077,7 +1035,6 @@ rg_status rg_ewald_destroy(rg_ewald* e)
   cudaFree(e->pairs);
   cudaFree(e->kmap);
   if (e->result_host) cudaFreeHost(e->result_host);
-  if (e->flag_host) cudaFreeHost(e->flag_host);
   delete e;
   return RG_OK;
 }
@@ -1102,7 +1059,7 @@ rg_status rg_ewald_set_framework(rg_ewald* e, const rg_atom* fw, int n_fw)
   }
   rg_status st = stageAtoms(e, fw, n_fw, nullptr, 0, 1.0);
   if (st) return st;
-  st = launchPairs(e, n_fw, true, TermsParams{}, Report{});
+  st = launchPairs(e, n_fw, true, TermsParams{}, 0u);
   if (st) return st;
   RG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   return RG_OK;
@@ -1155,30 +1112,32 @@ rg_status rg_ewald_full(rg_ewald* e, const rg_atom* atoms, int n_atoms, const in
   tp.alpha = alpha;
   tp.coul = C;
   tp.self = C * alpha / std::sqrt(rg::kPi);
-  const Report done = nextReport(e, (e->nk > 0 ? 1u : 0u) + (tp.blocks > 0 ? 1u : 0u));
+  const unsigned call = ++e->calls;
   if (e->nk > 0)
   {
     rg_status st;
     switch (G)
     {
-      case 0: st = launchPairs(e, n_atoms, false, tp, done); break;
-      case 1: st = launchFull<1>(e, n_atoms, done); break;
-      case 2: st = launchFull<2>(e, n_atoms, done); break;
-      case 3: st = launchFull<3>(e, n_atoms, done); break;
-      default: st = launchFull<4>(e, n_atoms, done); break;
+      case 0: st = launchPairs(e, n_atoms, false, tp, call); break;
+      case 1: st = launchFull<1>(e, n_atoms, call); break;
+      case 2: st = launchFull<2>(e, n_atoms, call); break;
+      case 3: st = launchFull<3>(e, n_atoms, call); break;
+      default: st = launchFull<4>(e, n_atoms, call); break;
     }
     if (st) return st;
   }
   if (tp.blocks > 0 && (e->nk == 0 || G > 0))
   {
-    ewaldAtomTermsKernel<<<tp.blocks, kThreads, 0, ctx->stream>>>(tp, e->omit_inter ? 1 : 0, done);
+    ewaldAtomTermsKernel<<<tp.blocks, kThreads, 0, ctx->stream>>>(tp, e->omit_inter ? 1 : 0, call);
     RG_CUDA(ctx, cudaGetLastError());
   }
   double own[kTerms] = {};
   if (host_terms) hostTerms(e, atoms, n_atoms, molecule_sizes, n_molecules, own);
   double all[kTermsAt + kTerms] = {};
-  if (done.parts > 0)
-    if (rg_status st = readResult(e, done.value, all, kTermsAt + kTerms, "rg_ewald_full")) return st;
+  if (e->nk > 0)
+    if (rg_status st = rg::collect(ctx, e->result_host, 1 + G, call, all, "rg_ewald_full")) return st;
+  if (tp.blocks > 0)
+    if (rg_status st = rg::collect(ctx, e->result_host + kTermsAt, kTerms, call, all + kTermsAt, "rg_ewald_full")) return st;
   const double* res = all;
   const double* terms = host_terms ? own : all + kTermsAt;
   out->ewald_self = terms[0];
@@ -1303,7 +1262,7 @@ rg_status rg_ewald_delta(rg_ewald* e, const rg_atom* new_atoms, int n_new, const
   for (int g = 0; g < 4; ++g) out->dudlambda_ewald[g] += 2.0 * uIon * (netChargeNew * dNew[g] - net_charge * dOld[g]);
   if (e->nk > 0)
   {
-    rg_status st = readResult(e, e->calls, res, 1 + G, "rg_ewald_delta");
+    rg_status st = rg::collect(ctx, e->result_host, 1 + G, e->calls, res, "rg_ewald_delta");
     if (st) return st;
   }
   out->ewald_fourier += res[0];
