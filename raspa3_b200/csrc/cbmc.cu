@@ -438,13 +438,10 @@ __global__ void __launch_bounds__(kThreads) trialEnergyKernel(TrialArgs a, Trial
   __syncthreads();
   if (threadIdx.x == 0)
   {
-    __threadfence();  // of the CTA's stores, which the barrier has put before it
-    const unsigned int done = atomicAdd(a.counters + trial, 1u);
-    last = (done == static_cast<unsigned int>(a.n_chunks - 1));
+    last = rg::countIn(a.counters + trial) == static_cast<unsigned int>(a.n_chunks - 1);
   }
   __syncthreads();
   if (!last) return;
-  __threadfence();
   // the trial's total over its chunks: 16 threads per channel sum the chunks j, j + 16, ... (their loads in flight
   // together), then each channel's 16 sub-sums in order
   static_assert(kThreads == 16 * 16 && kNumOut + 1 <= 16, "16 threads for each of at most 16 channels");

@@ -94,6 +94,16 @@ inline void matvec(const double m[3][3], const double v[3], double out[3])
 
 namespace rg
 {
+// Counts a block in at the end of its part, by one thread behind a barrier of the block, and returns how many were in
+// before: what the block has written is visible to whoever counts in later. (__threadfence before a relaxed atomic is a
+// sequentially consistent fence: with 290 blocks ending together it took 2,000 to 9,000 cycles.)
+__device__ __forceinline__ unsigned int countIn(unsigned int* counter)
+{
+  unsigned int before;
+  asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(before) : "l"(counter) : "memory");
+  return before;
+}
+
 // A result for the host (rg::collect): two 64-bit words, each half of the value beside the call's number, so that the
 // host knows by itself when a value has arrived. A flag written after the values needs a system-wide fence before it,
 // which waits for the bus: the trial energies of 10 positions against 12,000 sites spent 8 of 15 us of their kernel in two

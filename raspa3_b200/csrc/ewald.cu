@@ -122,12 +122,10 @@ __device__ __forceinline__ void blockReduceAndFinish(double (&v)[1 + G], double*
     {
 #pragma unroll
       for (int c = 0; c < 1 + G; ++c) partial[block * (1 + kMaxGroups) + c] = v[c];
-      __threadfence();
-      last = atomicAdd(counter, 1u) == n_blocks - 1;
+      last = rg::countIn(counter) == n_blocks - 1;
     }
     __syncthreads();
     if (!last) return;
-    __threadfence();
     // the last block: each thread sums the partials of blocks threadIdx.x, threadIdx.x + kThreads, ... (all its loads in
     // flight together), then the same fixed-order warp and block reduction
 #pragma unroll
@@ -424,12 +422,10 @@ __device__ __forceinline__ void atomTerms(const TermsParams& p, int omit_inter, 
   __syncthreads();
   if (threadIdx.x == 0)
   {
-    __threadfence();  // of the block's stores, which the barrier has put before it
-    last = atomicAdd(p.counter, 1u) == static_cast<unsigned>(n_blocks - 1);
+    last = rg::countIn(p.counter) == static_cast<unsigned>(n_blocks - 1);
   }
   __syncthreads();
   if (!last) return;
-  __threadfence();
   // a warp per column, the blocks by lane, then a fixed shuffle tree
   for (int c = warp; c < kTerms; c += kThreads / 32)
   {
