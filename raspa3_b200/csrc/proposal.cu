@@ -168,7 +168,8 @@ __device__ __forceinline__ void forward(MlpForwardShared& S, int ig, int jq, flo
 
 // The bound is FP32 arithmetic on operands from shared memory: with one output per thread each FMA took two loads; in
 // 2 x 4 and 4 x 4 register tiles it takes 0.4. A step on 4,096 samples: 45.6 us before, 23.6 now, and the reduction with
-// the Adam step below 10.6 and 7.0.
+// the Adam step below 10.6 and 7.0 (each alone); one after the other 100 steps took 5.0 ms before, 2.6 ms so, and 2.05 ms
+// with each kernel's start overlapping the end of the one before.
 // One tile's loss and gradient partial; batch size B scales the loss. Samples: tile0 + i in order, or (random) drawn
 // from the n_samples by splitmix64 of (seed, step, slot).
 __global__ void __launch_bounds__(kThreads) mlpGradKernel(const float* __restrict__ theta, const float* __restrict__ s,
@@ -197,10 +198,15 @@ __global__ void __launch_bounds__(kThreads) mlpGradKernel(const float* __restric
     }
     idx[tid] = static_cast<int>(k);
   }
+  __syncthreads();
+  // the samples do not depend on the step before, whose reduction this kernel's start overlaps (launchGrad)
+  cudaTriggerProgrammaticLaunchCompletion();
+  const float goal = tid < count ? target[idx[tid]] : 0.0f;
+  features(F.phi, count, [&](int i, int a) { return s[3 * idx[i] + a]; });
+  cudaGridDependencySynchronize();
   loadWeights(F.w, theta);
   __syncthreads();
   for (int q = tid; q < kH * kH; q += kThreads) S.W2T[(q % kH) * kLdH + q / kH] = F.w.W2[(q / kH) * kLdH + q % kH];
-  features(F.phi, count, [&](int i, int a) { return s[3 * idx[i] + a]; });
   __syncthreads();
   float z1[2][4], z2[2][4];
   forward(F, ig, jq, z1, z2);
@@ -210,7 +216,7 @@ __global__ void __launch_bounds__(kThreads) mlpGradKernel(const float* __restric
     float d = 0.0f, lp = 0.0f;
     if (tid < count)
     {
-      const float r = F.f[tid] - target[idx[tid]];
+      const float r = F.f[tid] - goal;
       d = 2.0f * r / static_cast<float>(batch);
       lp = r * r;
     }
@@ -331,6 +337,8 @@ __global__ void __launch_bounds__(kThreads) reduceAdamKernel(float* __restrict__
     c1 = 1.0f - powf(b1, static_cast<float>(t));
     c2 = 1.0f - powf(b2, static_cast<float>(t));
   }
+  cudaTriggerProgrammaticLaunchCompletion();
+  cudaGridDependencySynchronize();
   for (int base = 0; base < n_tiles; base += kReduceTiles)
   {
     const int n = min(kReduceTiles, n_tiles - base);
@@ -577,8 +585,28 @@ rg_status ensurePartial(rg_mlp* m, int tiles)
   return RG_OK;
 }
 
+// Launches a training kernel; with `overlap` it may start while the kernel before it in the stream ends, and waits for
+// that one's results where it says so (cudaGridDependencySynchronize). Everything it reads before has to be older: the
+// first kernel of a training run is launched without, since its samples may come from the kernel before.
+template <typename... Params, typename... Args>
+cudaError_t launchOverlapping(void (*kernel)(Params...), int blocks, size_t shared, cudaStream_t stream, bool overlap,
+                              Args... args)
+{
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = shared;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = overlap ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 rg_status launchGrad(rg_mlp* m, const float* s, const float* t, int64_t n, bool random, int batch,
-                     unsigned long long seed, long long step)
+                     unsigned long long seed, long long step, bool overlap)
 {
   rg_ctx* ctx = m->ctx;
   const int tiles = (batch + kTile - 1) / kTile;
@@ -586,9 +614,8 @@ rg_status launchGrad(rg_mlp* m, const float* s, const float* t, int64_t n, bool 
   if (st) return st;
   constexpr int sh = static_cast<int>(sizeof(MlpGradShared));
   RG_CUDA(ctx, cudaFuncSetAttribute(mlpGradKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sh));
-  mlpGradKernel<<<tiles, kThreads, sh, ctx->stream>>>(m->theta, s, t, n, random, batch, seed, step, m->partial,
-                                                      m->lossPartial);
-  RG_CUDA(ctx, cudaGetLastError());
+  RG_CUDA(ctx, launchOverlapping(mlpGradKernel, tiles, sh, ctx->stream, overlap, m->theta, s, t, n, random, batch, seed,
+                                 step, m->partial, m->lossPartial));
   return RG_OK;
 }
 // Forward pass on n positions (s null: the centres of cells^3 cells), at most two CTAs per SM
@@ -691,7 +718,7 @@ rg_status rg_mlp_loss_and_gradient(rg_mlp* m, const float* s_device, const float
   if (!m || !s_device || !target_device || n < 1 || n > (1 << 24)) return RG_ERR_INVALID_ARGUMENT;
   rg_ctx* ctx = m->ctx;
   RG_CUDA(ctx, cudaSetDevice(ctx->device));
-  rg_status st = launchGrad(m, s_device, target_device, n, false, n, 0, 0);
+  rg_status st = launchGrad(m, s_device, target_device, n, false, n, 0, 0, false);
   if (st) return st;
   const int tiles = (n + kTile - 1) / kTile;
   reduceAdamKernel<<<kReduceBlocks, kThreads, 0, ctx->stream>>>(m->theta, m->m, m->v, m->partial, tiles, 0.0f, 0.f, 0.f,
@@ -713,14 +740,12 @@ rg_status rg_mlp_train(rg_mlp* m, const float* s_device, const float* target_dev
   const int tiles = (batch + kTile - 1) / kTile;
   for (int s = 0; s < steps; ++s)
   {
-    rg_status st = launchGrad(m, s_device, target_device, n_samples, true, batch, seed, m->t);
+    rg_status st = launchGrad(m, s_device, target_device, n_samples, true, batch, seed, m->t, s > 0);
     if (st) return st;
     ++m->t;
     constexpr float b1 = 0.9f, b2 = 0.999f;
-    reduceAdamKernel<<<kReduceBlocks, kThreads, 0, ctx->stream>>>(m->theta, m->m, m->v, m->partial, tiles, learning_rate,
-                                                                 b1, b2, 1e-8f, m->t, nullptr, m->lossPartial,
-                                                                 m->scalars, batch);
-    RG_CUDA(ctx, cudaGetLastError());
+    RG_CUDA(ctx, launchOverlapping(reduceAdamKernel, kReduceBlocks, 0, ctx->stream, true, m->theta, m->m, m->v, m->partial,
+                                   tiles, learning_rate, b1, b2, 1e-8f, m->t, nullptr, m->lossPartial, m->scalars, batch));
   }
   if (final_loss)
   {
