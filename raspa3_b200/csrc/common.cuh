@@ -29,6 +29,9 @@ struct rg_ctx
   // on first use).
   cudaStream_t copy_stream = nullptr;
   std::vector<cudaEvent_t> events;
+  // The device memory of the last tabulated proposal that was destroyed, for the next one (one buffer, freed with the
+  // context): freeing and mapping it anew took 1 to 5 ms when nothing else held its pages.
+  Slot spare_table;
 };
 
 namespace rg

@@ -230,6 +230,7 @@ rg_status rg_ctx_destroy(rg_ctx* ctx)
     if (s.ptr) cudaFree(s.ptr);
   for (auto& s : ctx->pinned)
     if (s.ptr) cudaFreeHost(s.ptr);
+  if (ctx->spare_table.ptr) cudaFree(ctx->spare_table.ptr);
   if (ctx->copy_stream)
   {
     cudaStreamSynchronize(ctx->copy_stream);

@@ -550,6 +550,7 @@ struct rg_proposal
   rg_ctx* ctx = nullptr;
   int G = 0;
   double eps = 0.0;
+  rg_ctx::Slot table;         // device memory of both arrays
   double* cdf = nullptr;      // inclusive cumulative cell probabilities, G^3
   double* density = nullptr;  // q per cell relative to uniform: (1 - eps) G^3 p_c + eps
   std::vector<double> host_density;
@@ -815,8 +816,14 @@ rg_status rg_proposal_create(rg_mlp* m, int32_t cells_per_axis, double eps_unifo
   double* sums = static_cast<double*>(scr);
   int* largest = reinterpret_cast<int*>(sums + blocks + 1);
   float* f = reinterpret_cast<float*>(sums + blocks + 2);
-  cudaError_t err = cudaMalloc(reinterpret_cast<void**>(&p->cdf), sizeof(double) * nc);
-  if (!err) err = cudaMalloc(reinterpret_cast<void**>(&p->density), sizeof(double) * nc);
+  cudaError_t err = cudaSuccess;
+  const size_t bytes = 2 * sizeof(double) * static_cast<size_t>(nc);
+  if (ctx->spare_table.bytes >= bytes)
+    std::swap(p->table, ctx->spare_table);
+  else if (!(err = cudaMalloc(&p->table.ptr, bytes)))
+    p->table.bytes = bytes;
+  p->cdf = static_cast<double*>(p->table.ptr);
+  p->density = p->cdf + nc;
   if (!err) err = cudaMemsetAsync(largest, 0x80, sizeof(int), ctx->stream);  // the integer of -3.39e38
   if (!err) st = launchForward(m, nullptr, G, nc, f, largest);
   if (!err && !st)
@@ -845,8 +852,9 @@ rg_status rg_proposal_destroy(rg_proposal* p)
 {
   if (!p) return RG_OK;
   if (p->ctx) cudaStreamSynchronize(p->ctx->stream);
-  cudaFree(p->cdf);
-  cudaFree(p->density);
+  // the larger of the two buffers stays with the context
+  if (p->ctx && p->table.bytes > p->ctx->spare_table.bytes) std::swap(p->table, p->ctx->spare_table);
+  if (p->table.ptr) cudaFree(p->table.ptr);
   delete p;
   return RG_OK;
 }
