@@ -1690,7 +1690,7 @@ rg_status rg_ewald_batch_set(rg_ewald_batch* b, int system, const double* sk)
   ewaldBatchPermuteKernel<<<static_cast<unsigned>((e->nk + kThreads - 1) / kThreads), kThreads, 0, ctx->stream>>>(
       e->nk, b->slot_of, list, sk ? 1 : 1 + e->n_groups, dst, 1);
   RG_CUDA(ctx, cudaGetLastError());
-  RG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  if (sk) RG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));  // the caller's buffer may be pinned
   return RG_OK;
 }
 
