@@ -150,10 +150,13 @@ __device__ __forceinline__ void blockReduceAndFinish(double (&v)[1 + G], double*
 // 60,000 FP64 instructions), so the chain is kept short: the phase of a k-vector is the product of three entries of
 // tables e^{i 2 pi m s_d}, one sincospi per thread and tile of atoms while the k-vector's own loads are in flight; a
 // sincospi per atom and k-vector is a chain of as many as there are atoms. Per call with 8,124 k-vectors and 6, 30 and
-// 120 atoms 18.7, 26.6 and 43.5 us before, 16.7, 23.5 and 36.4 us now. (One block of 1,024 threads for sets that fit it
-// saves the second reduction, but its one SM does all the products: 17.2, 29.9 and 69.3 us at 1,152 k-vectors against
-// 16.8, 23.1 and 34.6 us with blocks of 256 at 2,600.)
+// 120 atoms 18.7, 26.6 and 43.5 us before, 16.7, 23.5 and 36.4 us so, and with the results posted 12.6, 19.1 and 32.3 us.
+// (One block of 1,024 threads for sets that fit it saves the second reduction, but its one SM does all the products: 17.2,
+// 29.9 and 69.3 us at 1,152 k-vectors against 16.8, 23.1 and 34.6 us with blocks of 256 at 2,600.)
 constexpr int kDeltaTile = 16;                 // atoms whose tables are in shared memory at a time, at most
+// Up to this many blocks each block posts its own sums and the host adds them in block order: the reduction across blocks
+// on the device (an atomic, a second read and sum) makes a call of 8,124 k-vectors 14.5 us long, without it 12.6
+constexpr int kDeltaPosted = 64;
 constexpr size_t kDeltaShared = 40 << 10;      // bytes of tables at most: fewer atoms per tile for a large kmax
 template <int G>
 __global__ void __launch_bounds__(kThreads) ewaldDeltaKernel(int nk, int kxm, int kym, int kzm,
@@ -247,7 +250,16 @@ __global__ void __launch_bounds__(kThreads) ewaldDeltaKernel(int nk, int kxm, in
       trial[row + 1 + g] = TG;
     }
   }
-  blockReduceAndFinish<G>(v, partial, counter, result, call, gridDim.x, blockIdx.x);
+  if (gridDim.x > kDeltaPosted)
+  {
+    blockReduceAndFinish<G>(v, partial, counter, result, call, gridDim.x, blockIdx.x);
+    return;
+  }
+  __shared__ double red[kThreads / 32][1 + kMaxGroups];
+  blockSum<G>(v, red);
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int c = 0; c < 1 + G; ++c) rg::post(result + blockIdx.x * (1 + G) + c, v[c], call);
 }
 
 // Partial sums of the structure factor of one chunk of atoms, for one (kx, ky) pair per thread and MT consecutive values
@@ -332,6 +344,9 @@ __global__ void __launch_bounds__(32 * kPairWarps, kPairBlocks) ewaldPairSumsKer
 // charge, dU/dlambda [4], charge of each group [4]; per-block sums, added in block order by the last block.
 constexpr int kTerms = 11;
 constexpr int kTermsAt = 8;  // where they start in the result array (the Fourier sums come first)
+// results of one call at most: the recompute's, or the blocks' sums of a difference
+constexpr int kResults = kDeltaPosted * (1 + kMaxGroups);
+static_assert(kResults >= kTermsAt + kTerms, "room for both");
 struct TermsParams
 {
   const MovedAtom* atoms;
@@ -995,9 +1010,9 @@ rg_status rg_ewald_create(rg_ctx* ctx, const rg_forcefield* ff, const rg_box* bo
     err = cudaMemcpyAsync(e->kmap, e->kmap_host.data(), sizeof(int) * e->kmap_host.size(), cudaMemcpyHostToDevice,
                           ctx->stream);
   if (!err)
-    err = cudaHostAlloc(reinterpret_cast<void**>(&e->result_host), sizeof(ulonglong2) * (kTermsAt + kTerms), cudaHostAllocMapped);
+    err = cudaHostAlloc(reinterpret_cast<void**>(&e->result_host), sizeof(ulonglong2) * kResults, cudaHostAllocMapped);
   if (!err) err = cudaHostGetDevicePointer(reinterpret_cast<void**>(&e->result), e->result_host, 0);
-  if (!err) std::memset(e->result_host, 0, sizeof(ulonglong2) * (kTermsAt + kTerms));
+  if (!err) std::memset(e->result_host, 0, sizeof(ulonglong2) * kResults);
   if (!err) err = cudaDeviceGetAttribute(&e->sms, cudaDevAttrMultiProcessorCount, ctx->device);
   if (!err && e->nk > 0)
     err = cudaMemcpyAsync(e->kvec, kv.data(), sizeof(char4) * e->nk, cudaMemcpyHostToDevice, ctx->stream);
@@ -1258,8 +1273,12 @@ rg_status rg_ewald_delta(rg_ewald* e, const rg_atom* new_atoms, int n_new, const
   for (int g = 0; g < 4; ++g) out->dudlambda_ewald[g] += 2.0 * uIon * (netChargeNew * dNew[g] - net_charge * dOld[g]);
   if (e->nk > 0)
   {
-    rg_status st = rg::collect(ctx, e->result_host, 1 + G, e->calls, res, "rg_ewald_delta");
+    const int blocks = static_cast<int>((e->nk + kThreads - 1) / kThreads), posts = blocks <= kDeltaPosted ? blocks : 1;
+    double sums[kDeltaPosted * (1 + kMaxGroups)];
+    rg_status st = rg::collect(ctx, e->result_host, posts * (1 + G), e->calls, sums, "rg_ewald_delta");
     if (st) return st;
+    for (int b = 0; b < posts; ++b)
+      for (int c = 0; c < 1 + G; ++c) res[c] += sums[b * (1 + G) + c];
   }
   out->ewald_fourier += res[0];
   for (int g = 0; g < G; ++g) out->dudlambda_ewald[g] += res[1 + g];

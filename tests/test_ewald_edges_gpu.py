@@ -67,10 +67,11 @@ def test_full_recompute_and_framework(ctx, oracle, kmax, sphere, cell, molecules
     ew.close()
 
 
-# 297, 1,152, 2,600, 3,796 and 1,205 k-vectors: one k-vector per thread of one block, two, and blocks of 256; up to 16 atoms
-# travel in the launch's parameters and are one tile of the phase tables
+# 297 to 3,796 k-vectors are 2 to 15 blocks, each of which gives its own sums to the host; 17,328 are 68, whose sums the last
+# one adds (from 65 on); up to 16 atoms travel in the launch's parameters and are one tile of the phase tables
 @pytest.mark.parametrize("kmax,sphere,cell", [((5, 5, 5), True, BOX), ((8, 8, 8), True, SKEW), ((8, 8, 8), False, BOX),
-                                              ((12, 12, 12), True, SKEW), ((1, 100, 1), False, BOX)])
+                                              ((12, 12, 12), True, SKEW), ((1, 100, 1), False, BOX),
+                                              ((20, 20, 20), True, BOX)])
 @pytest.mark.parametrize("new,old,groups", [(0, 1, 0), (1, 1, 0), (3, 2, 0), (40, 41, 0), (1, 1, 1), (3, 3, 4)])
 def test_difference(ctx, oracle, kmax, sphere, cell, new, old, groups):
     """`new` and `old` molecules; with groups the first is fractional."""
