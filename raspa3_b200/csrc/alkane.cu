@@ -25,7 +25,7 @@
 // batch (1,016 framework atoms, 8 beads, one CTA of 512 threads) in cycles: pairs 5,400 (issue), reductions 2,300, trial
 // positions 1,900, selection 2,000; and once per growth 21,000 for the torsion weights (FP64 pipe). 64 systems, 200 moves:
 // 7.5 ms with the spins' cosines from cospi, two exponentials and three more shuffles per selection, the displacements
-// scaled twice and the system's constants in global memory, now 6.7 ms. Listing the pairs within the cutoff per thread
+// scaled twice and the system's constants in global memory, now 6.5 ms. Listing the pairs within the cutoff per thread
 // and evaluating them together was slower (5,400 against 7,100 cycles: each round waits for a chain of loads).
 #include <cooperative_groups.h>
 
@@ -135,7 +135,7 @@ struct Shared
   uint32_t tword[kMaxBeads][kMaxTrials];     // random word of the selected spin per step and direction
   double W, eext, dU, stats[kStats];
   int fail, kind, m, axis, n, accept;
-  unsigned long long pairs;
+  unsigned long long pairs[kMaxWarps];  // in-cutoff pairs of each warp
   double energy, disp, u_acc;
 };
 
@@ -385,12 +385,11 @@ __device__ __noinline__ void evalBeads(Shared& sh, const Params& p, const SysDev
   }
   if (lane < nbd)
   {
-    const int bb = (32 * warp + lane) % nbd;
-    sh.red[0][warp][bb] = afw;
-    sh.red[1][warp][bb] = amm;
+    sh.red[0][warp][b] = afw;
+    sh.red[1][warp][b] = amm;
   }
   inside = __reduce_add_sync(0xffffffffu, inside);
-  if (lane == 0 && inside) atomicAdd(&sh.pairs, static_cast<unsigned long long>(inside));
+  if (lane == 0) sh.pairs[warp] += inside;
   ovl = __reduce_or_sync(0xffffffffu, ovl);
   if (lane == 0) sh.red_ovl[warp] = ovl;
   __syncthreads();
@@ -834,9 +833,9 @@ __global__ void __launch_bounds__(T, 1) alkaneKernel(Params p, const int* __rest
   {
     sh.n = n0;
     sh.energy = p.energy[s];
-    sh.pairs = 0ull;
     for (int k = 0; k < kStats; ++k) sh.stats[k] = st[k];
   }
+  if (tid < kMaxWarps) sh.pairs[tid] = 0ull;
   const long long move0 = p.move_base[s];
   int eval = 0;  // evaluation counter (selects the exchange buffer), identical in every thread
   __syncthreads();
@@ -972,7 +971,12 @@ __global__ void __launch_bounds__(T, 1) alkaneKernel(Params p, const int* __rest
     }
     __syncthreads();
   }
-  if (tid == 0 && sh.pairs) atomicAdd(p.pairs + s, sh.pairs);
+  if (tid == 0)
+  {
+    unsigned long long pairs = 0;
+    for (int w = 0; w < T / 32; ++w) pairs += sh.pairs[w];
+    atomicAdd(p.pairs + s, pairs);
+  }
   if (rank == 0 && tid == 0)
   {
     p.n_mol[s] = sh.n;
@@ -1006,7 +1010,7 @@ __global__ void __launch_bounds__(128) beadKernel(Params p, int s, int fw_cap, c
     molS[i] = toFixed(S, d3(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]), S.types[b] | (m << 8));
   }
   if (tid < nbd) sh.bead[tid] = toFixed(S, d3(xyz[3 * tid], xyz[3 * tid + 1], xyz[3 * tid + 2]), types[tid]);
-  if (tid == 0) sh.pairs = 0ull;
+  if (tid < kMaxWarps) sh.pairs[tid] = 0ull;
   __syncthreads();
   int eval = 0;
   evalBeads(sh, p, S, fwS, S.n_fw, molS, n * nb, nbd, skip, cl, eval);
@@ -1028,7 +1032,7 @@ __global__ void __launch_bounds__(128) vacuumKernel(Params p, long long n, doubl
   copySystem(sh, p.sys[0]);
   const int tid = threadIdx.x, nb = S.nb;
   for (int i = tid; i < kMaxTypes * kMaxTypes; i += blockDim.x) sh.tab[i] = p.ljf[i];
-  if (tid == 0) sh.pairs = 0ull;
+  if (tid < kMaxWarps) sh.pairs[tid] = 0ull;
   int eval = 0;
   __syncthreads();
   for (long long c = blockIdx.x; c < n; c += gridDim.x)
