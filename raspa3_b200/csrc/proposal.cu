@@ -537,9 +537,11 @@ struct rg_mlp
   float* theta = nullptr;
   float* m = nullptr;
   float* v = nullptr;
+  // the tiles' partials of the last launch, set anew by each (ensurePartial): the context's scratch, or `own`
   float* partial = nullptr;
-  int partial_tiles = 0;
   float* lossPartial = nullptr;
+  float* own = nullptr;
+  int own_tiles = 0;
   float* scalars = nullptr;  // [0] loss
   float* grad = nullptr;     // gradient of rg_mlp_loss_and_gradient
   long long t = 0;           // Adam step count
@@ -571,18 +573,31 @@ rg_status proposalExport(rg_proposal* p, const double** cdf, const double** dens
 
 namespace
 {
+// Room for the partials of `tiles` tiles. Up to kSharedTiles (43 MB) they lie in scratch that all networks of the context
+// share (their kernels are ordered by its stream): a buffer of each network's own cost its first training 0.5 ms, now and
+// then 7. More than that a context would keep for good, so the network has its own.
+constexpr int kSharedTiles = 1024;
 rg_status ensurePartial(rg_mlp* m, int tiles)
 {
   rg_ctx* ctx = m->ctx;
-  if (m->partial_tiles >= tiles) return RG_OK;
-  RG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  cudaFree(m->partial);
-  cudaFree(m->lossPartial);
-  m->partial = nullptr;
-  m->lossPartial = nullptr;
-  RG_CUDA(ctx, cudaMalloc(reinterpret_cast<void**>(&m->partial), sizeof(float) * kParams * tiles));
-  RG_CUDA(ctx, cudaMalloc(reinterpret_cast<void**>(&m->lossPartial), sizeof(float) * tiles));
-  m->partial_tiles = tiles;
+  const size_t bytes = sizeof(float) * (kParams + 1) * static_cast<size_t>(tiles);
+  void* room = m->own;
+  if (tiles <= kSharedTiles)
+  {
+    if (rg_status st = rg::scratch(ctx, 11, bytes, &room)) return st;
+  }
+  else if (m->own_tiles < tiles)
+  {
+    RG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    cudaFree(m->own);
+    m->own = nullptr;
+    m->own_tiles = 0;
+    RG_CUDA(ctx, cudaMalloc(reinterpret_cast<void**>(&m->own), bytes));
+    m->own_tiles = tiles;
+    room = m->own;
+  }
+  m->partial = static_cast<float*>(room);
+  m->lossPartial = m->partial + static_cast<size_t>(kParams) * tiles;
   return RG_OK;
 }
 
@@ -687,10 +702,9 @@ rg_status rg_mlp_destroy(rg_mlp* m)
   cudaFree(m->theta);
   cudaFree(m->m);
   cudaFree(m->v);
-  cudaFree(m->partial);
-  cudaFree(m->lossPartial);
   cudaFree(m->scalars);
   cudaFree(m->grad);
+  cudaFree(m->own);
   delete m;
   return RG_OK;
 }

@@ -20,7 +20,8 @@ def ctx():
     c.close()
 
 
-@pytest.mark.parametrize("n", [1, 31, 32, 33, 255, 4097])
+# 32,768 and 32,769 samples are 1,024 and 1,025 tiles: partial sums in shared scratch and in the network's own
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 255, 4097, 32768, 32769])
 def test_batches_against_fp64(ctx, n):
     torch = pytest.importorskip("torch")
     mo = importlib.import_module("oracle.mlp")
