@@ -90,7 +90,9 @@ rg_status rg_ctx_create(int device, rg_ctx** out);
 /* Objects created on a context (rg_system, rg_ewald, rg_gcmc) must be destroyed before it. */
 rg_status rg_ctx_destroy(rg_ctx* ctx);
 /* Use the caller's CUDA stream (a created cudaStream_t or cudaStreamPerThread; NULL restores the context's own
- * non-blocking stream, so the legacy NULL stream itself cannot be selected). */
+ * non-blocking stream, so the legacy NULL stream itself cannot be selected). Waits on the host for what the energy calls
+ * and state copies made so far still have on the old stream, so that calls on the new one come after them; queued runs
+ * (rg_gcmc_run, rg_mixture_run, rg_alkane_run) it does not wait for. */
 rg_status rg_ctx_set_stream(rg_ctx* ctx, void* stream);
 void* rg_ctx_stream(rg_ctx* ctx);
 rg_status rg_ctx_synchronize(rg_ctx* ctx);

@@ -8,7 +8,7 @@
 // grids (one per pseudo-atom type plus the unit-charge Ewald grid) and the adsorbate atoms. One launch evaluates all
 // trials of a growth step: the grid is (trial, chunk), sized to one wave of resident CTAs; each CTA stages the trial's
 // atoms in shared memory (a call of up to 32 trial atoms brings them in the launch parameters, so it costs one launch
-// and one synchronisation), the threads of chunks 1.. stride over their chunk of partners (framework atoms for trial
+// and the wait for its results), the threads of chunks 1.. stride over their chunk of partners (framework atoms for trial
 // atoms without a grid, then adsorbate atoms from other molecules), and the per-trial totals are reduced in a fixed
 // order by the last CTA of the trial. Trial atoms with a grid (and not fractional) take the grid branch in chunk 0:
 // one tricubic interpolation of their VDW grid and, with charges, q times the unit-charge Ewald grid. A trial is flagged as overlapping if any VDW pair energy or
@@ -754,7 +754,7 @@ rg_status runTrials(rg_system* s, const TrialCall& c, rg_trial_energy* out)
     std::memcpy(small.a, c.trials, sizeof(rg_atom) * nt_atoms);
   else
   {
-    // the pinned staging buffer is free: every call ends by synchronising the stream
+    // the pinned staging buffer is free: the copy out of it ended before the kernel of the last call posted its results
     std::memcpy(s->trials_host, c.trials, sizeof(rg_atom) * nt_atoms);
     RG_CUDA(ctx, cudaMemcpyAsync(s->trials, s->trials_host, sizeof(rg_atom) * nt_atoms, cudaMemcpyHostToDevice,
                                  ctx->stream));
@@ -808,6 +808,7 @@ rg_status runTrials(rg_system* s, const TrialCall& c, rg_trial_energy* out)
   dim3 grid(n_trials, n_chunks);
   kernel<<<grid, kThreads, 0, ctx->stream>>>(a, small);
   RG_CUDA(ctx, cudaGetLastError());
+  if (rg_status ls = rg::leave(ctx)) return ls;
   for (int t = 0; t < n_trials; ++t)
   {
     double v[kNumOut + 1];

@@ -32,6 +32,10 @@ struct rg_ctx
   // The device memory of the last tabulated proposal that was destroyed, for the next one (one buffer, freed with the
   // context): freeing and mapping it anew took 1 to 5 ms when nothing else held its pages.
   Slot spare_table;
+  // Recorded behind the last kernel of a call that returned before the stream was done with it (rg::leave), until the
+  // stream is changed: the next stream's work comes after it.
+  cudaEvent_t left = nullptr;
+  bool left_pending = false;
 };
 
 namespace rg
@@ -57,6 +61,11 @@ rg_status copyStream(rg_ctx* ctx, cudaStream_t* out);
 rg_status event(rg_ctx* ctx, int i, cudaEvent_t* out);
 // Makes the context stream wait for everything queued on the copy stream so far.
 rg_status joinCopies(rg_ctx* ctx);
+
+// Marks the end of the work that a call leaves on the stream when it returns: results that are posted (rg::post) say
+// nothing of the kernel's other stores, nor of the counters that it resets behind them. On the same stream the next kernel
+// comes after them all; rg_ctx_set_stream waits for the mark. A stream that is being captured is refused.
+rg_status leave(rg_ctx* ctx);
 
 // Takes n results that the kernels of call number `call` post (rg::post) into mapped host memory `from`, as soon as each
 // is there. A launch that failed, or a stream that cannot be waited for (one being captured), ends the wait with its

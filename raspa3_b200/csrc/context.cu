@@ -47,6 +47,22 @@ bool supercellClip(const HostBox& b, double rc, double cutoff, double h[3], doub
   return clip;
 }
 
+rg_status leave(rg_ctx* ctx)
+{
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  RG_CUDA(ctx, cudaStreamIsCapturing(ctx->stream, &capture));
+  if (capture != cudaStreamCaptureStatusNone)
+  {
+    // refused as a wait for the stream is, which also ends the capture; its error is not the next launch's
+    const cudaError_t err = cudaStreamSynchronize(ctx->stream);
+    cudaGetLastError();
+    return cudaFail(ctx, err, "a stream that is being captured");
+  }
+  RG_CUDA(ctx, cudaEventRecord(ctx->left, ctx->stream));
+  ctx->left_pending = true;
+  return RG_OK;
+}
+
 rg_status collect(rg_ctx* ctx, const ulonglong2* from, int n, unsigned int call, double* out, const char* what)
 {
   const volatile unsigned long long* words = reinterpret_cast<const volatile unsigned long long*>(from);
@@ -210,9 +226,11 @@ rg_status rg_ctx_create(int device, rg_ctx** out)
   if (device < 0 || device >= count) return RG_ERR_INVALID_ARGUMENT;
   rg_ctx* ctx = new rg_ctx();
   ctx->device = device;
-  if (cudaSetDevice(device) != cudaSuccess || cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking) !=
-                                                  cudaSuccess)
+  if (cudaSetDevice(device) != cudaSuccess ||
+      cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaEventCreateWithFlags(&ctx->left, cudaEventDisableTiming) != cudaSuccess)
   {
+    if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
     delete ctx;
     return RG_ERR_CUDA;
   }
@@ -237,6 +255,7 @@ rg_status rg_ctx_destroy(rg_ctx* ctx)
     cudaStreamDestroy(ctx->copy_stream);
   }
   for (cudaEvent_t e : ctx->events) cudaEventDestroy(e);
+  if (ctx->left) cudaEventDestroy(ctx->left);
   if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
   delete ctx;
   return RG_OK;
@@ -245,7 +264,22 @@ rg_status rg_ctx_destroy(rg_ctx* ctx)
 rg_status rg_ctx_set_stream(rg_ctx* ctx, void* stream)
 {
   if (!ctx) return RG_ERR_INVALID_ARGUMENT;
-  ctx->stream = stream ? static_cast<cudaStream_t>(stream) : ctx->own_stream;
+  const cudaStream_t next = stream ? static_cast<cudaStream_t>(stream) : ctx->own_stream;
+  if (next != ctx->stream && ctx->left_pending)
+  {
+    // Calls that return posted results, or a state copied on the device, may still have a kernel on the old stream; what
+    // follows on the new one reads and overwrites the same buffers. The wait is for the mark behind that kernel, not
+    // for the old stream (which the caller may have destroyed by now, or given work of its own), and on the host, for
+    // the new stream may be capturing; the caller's thread may too, hence the relaxed mode around it.
+    RG_CUDA(ctx, cudaSetDevice(ctx->device));
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RG_CUDA(ctx, cudaThreadExchangeStreamCaptureMode(&mode));
+    const cudaError_t err = cudaEventSynchronize(ctx->left);
+    RG_CUDA(ctx, cudaThreadExchangeStreamCaptureMode(&mode));
+    if (err != cudaSuccess) return rg::cudaFail(ctx, err, "rg_ctx_set_stream");
+    ctx->left_pending = false;
+  }
+  ctx->stream = next;
   return RG_OK;
 }
 

@@ -10,11 +10,12 @@
 // buffers of (1 + groups) entries per k (the total and the dU/dlambda group sums), "stored" and "trial". A move
 // writes trial = stored + Delta rho; accepting swaps the two pointers instead of the reference's full vector copy.
 // The Fourier energy change per k is computed as temp*(2 Re(conj(S) dRho) + |dRho|^2), algebraically the reference's
-// temp*(|S + dRho|^2 - |S|^2) without the cancellation. Block partial sums are reduced in a fixed order by the last
-// block to finish (deterministic), which writes the totals straight into mapped pinned host memory. A move of up to 16
-// atoms travels in the launch's parameter block, so one difference costs one launch and one synchronisation. The full
-// recompute splits the atoms into chunks along a second grid dimension and sums the chunks' partial structure factors
-// in chunk order. Self, exclusion and net-charge terms are few-atom FP64 host sums.
+// temp*(|S + dRho|^2 - |S|^2) without the cancellation. Block partial sums are posted into mapped pinned host memory,
+// where the host adds them in block order (up to kDeltaPosted blocks), or reduced in a fixed order by the last block to
+// finish, which posts the totals; either is deterministic. A move of up to 16 atoms travels in the launch's parameter
+// block, so one difference costs one launch and the wait for the posts. The full recompute splits the atoms into chunks
+// along a second grid dimension and sums the chunks' partial structure factors in chunk order. The self, exclusion and
+// net-charge terms are FP64 sums, on the host for a move or a few atoms (kHostTerms), else on the device.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -1142,6 +1143,8 @@ rg_status rg_ewald_full(rg_ewald* e, const rg_atom* atoms, int n_atoms, const in
     ewaldAtomTermsKernel<<<tp.blocks, kThreads, 0, ctx->stream>>>(tp, e->omit_inter ? 1 : 0, call);
     RG_CUDA(ctx, cudaGetLastError());
   }
+  if (e->nk > 0 || tp.blocks > 0)
+    if (rg_status st = rg::leave(ctx)) return st;
   double own[kTerms] = {};
   if (host_terms) hostTerms(e, atoms, n_atoms, molecule_sizes, n_molecules, own);
   double all[kTermsAt + kTerms] = {};
@@ -1212,6 +1215,7 @@ rg_status rg_ewald_delta(rg_ewald* e, const rg_atom* new_atoms, int n_new, const
       default: err = launchDelta<4>(e, n, sp); break;
     }
     if (err) return rg::cudaFail(ctx, err, "ewaldDeltaKernel");
+    if (rg_status st = rg::leave(ctx)) return st;
   }
   // the moved atoms' own terms, while the kernel is in flight
   const double C = rg::coulombFactor();
@@ -1709,7 +1713,8 @@ rg_status rg_ewald_batch_set(rg_ewald_batch* b, int system, const double* sk)
   ewaldBatchPermuteKernel<<<static_cast<unsigned>((e->nk + kThreads - 1) / kThreads), kThreads, 0, ctx->stream>>>(
       e->nk, b->slot_of, list, sk ? 1 : 1 + e->n_groups, dst, 1);
   RG_CUDA(ctx, cudaGetLastError());
-  if (sk) RG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));  // the caller's buffer may be pinned
+  if (!sk) return rg::leave(ctx);
+  RG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));  // the caller's buffer may be pinned
   return RG_OK;
 }
 
