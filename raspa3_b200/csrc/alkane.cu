@@ -1684,7 +1684,8 @@ extern "C" rg_status rg_alkane_bead_energies(rg_alkane* a, int system, const dou
   int* dov = reinterpret_cast<int*>(dx + 96);
   RG_CUDA(ctx, cudaMemcpyAsync(dx, xyz_beads, sizeof(double) * 3 * n_beads, cudaMemcpyHostToDevice, ctx->stream));
   RG_CUDA(ctx, cudaMemcpyAsync(dt, types, sizeof(int) * n_beads, cudaMemcpyHostToDevice, ctx->stream));
-  RG_CUDA(ctx, cudaFuncSetAttribute(beadKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  // the limit is the kernel's on the device, for the batches of all contexts: the same whoever sets it
+  RG_CUDA(ctx, cudaFuncSetAttribute(beadKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, a->max_smem));
   beadKernel<<<1, 128, smem, ctx->stream>>>(a->p, system, S.n_fw, dx, dt, n_beads, skip, dfw, dmm, dov);
   RG_CUDA(ctx, cudaGetLastError());
   RG_CUDA(ctx, cudaMemcpyAsync(fw, dfw, sizeof(double) * n_beads, cudaMemcpyDeviceToHost, ctx->stream));

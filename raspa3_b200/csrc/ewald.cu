@@ -829,6 +829,7 @@ cudaError_t launchDelta(rg_ewald* e, int n_moved, const MovedParam* small)
 // Pair sums and their finish over the staged atoms, for the framework (rigid) or the adsorbates. A block holds up to
 // kPairWarps warps of pairs; the atoms are cut into chunks so that the blocks fill every SM once (as many narrow blocks
 // per SM as make up kPairWarps warps), with at least 8 atoms each.
+constexpr size_t kPairShared = 98304;  // bytes of tables at most
 rg_status launchPairs(rg_ewald* e, int n_atoms, bool rigid, const TermsParams& terms, unsigned call)
 {
   cudaStream_t stream = e->ctx->stream;
@@ -854,7 +855,7 @@ rg_status launchPairs(rg_ewald* e, int n_atoms, bool rigid, const TermsParams& t
   const int chunk = std::max(8, (n_atoms + want - 1) / want);
   const int n_chunks = std::max(1, (n_atoms + chunk - 1) / chunk);
   const size_t per_atom = sizeof(double2) * ((kxm + 1) + (2 * kym + 1) + mt);
-  const int tile = std::max(1, std::min({32, chunk, static_cast<int>(98304 / per_atom)}));
+  const int tile = std::max(1, std::min({32, chunk, static_cast<int>(kPairShared / per_atom)}));
   const int64_t total = static_cast<int64_t>(e->n_pairs) * (kzm + 1);
   void* scr = nullptr;
   if (rg_status st = rg::scratch(e->ctx, kSumsSlot, 2 * sizeof(double2) * static_cast<size_t>(n_chunks) * total, &scr))
@@ -865,18 +866,20 @@ rg_status launchPairs(rg_ewald* e, int n_atoms, bool rigid, const TermsParams& t
   {
     const dim3 grid(pair_blocks, n_chunks, m_tiles);
     const size_t shmem = per_atom * tile;
+    // The limit of a kernel's shared memory is the device's, not the context's: always the most that any call takes, so
+    // that no host thread lowers it between another's setting and launch.
     auto run = [&](auto kern)
     {
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(shmem));
+      const cudaError_t err =
+          cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kPairShared));
+      if (err) return err;
       kern<<<grid, 32 * warps, shmem, stream>>>(e->n_pairs, e->pairs, atoms, n_atoms, chunk, tile, kxm, kym, kzm,
                                                 sums);
+      return cudaGetLastError();
     };
-    switch (mt)
-    {
-      case 7: run(ewaldPairSumsKernel<7>); break;
-      case 6: run(ewaldPairSumsKernel<6>); break;
-      default: run(ewaldPairSumsKernel<5>); break;
-    }
+    RG_CUDA(e->ctx, mt == 7   ? run(ewaldPairSumsKernel<7>)
+                    : mt == 6 ? run(ewaldPairSumsKernel<6>)
+                              : run(ewaldPairSumsKernel<5>));
   }
   else
     RG_CUDA(e->ctx, cudaMemsetAsync(sums, 0, 2 * sizeof(double2) * total, stream));
@@ -910,7 +913,8 @@ rg_status launchFull(rg_ewald* e, int n_atoms, unsigned call)
   const int stride = (e->ff.kmax_x + 1) + (e->ff.kmax_y + 1) + (e->ff.kmax_z + 1);
   size_t shmem = sizeof(double2) * kFullTile * stride;
   auto kern = ewaldFullPartialKernel<G>;
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(shmem));
+  constexpr int most = sizeof(double2) * kFullTile * 3 * 128;  // kmax is at most 127; as in launchPairs
+  RG_CUDA(e->ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
   if (n_atoms > 0)
     kern<<<dim3(blocks, n_chunks), kThreads, shmem, e->ctx->stream>>>(
         e->nk, e->kvec, static_cast<const MovedAtom*>(e->moved), n_atoms, chunkAtoms, e->ff.kmax_x, e->ff.kmax_y,
@@ -1777,10 +1781,10 @@ rg_status rg_ewald_batch_delta(rg_ewald_batch* b, const rg_atom* atoms, int max_
                                ctx->stream));
   const int kxm = e->ff.kmax_x, kym = e->ff.kmax_y, kzm = e->ff.kmax_z;
   const size_t shmem = batchSharedBytes(stride, kxm, kym, kzm);
-  if (shmem > 200 * 1024)
+  constexpr int most = 200 * 1024;  // the limit set as in launchPairs
+  if (shmem > most)
     return rg::fail(ctx, RG_ERR_UNSUPPORTED, "rg_ewald_batch_delta: kmax too large for the shared-memory tables");
-  RG_CUDA(ctx, cudaFuncSetAttribute(ewaldBatchDeltaKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(shmem)));
+  RG_CUDA(ctx, cudaFuncSetAttribute(ewaldBatchDeltaKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
   dim3 grid(b->blocks, b->n);
   RG_CUDA(ctx, cudaEventRecord(b->ev[1], ctx->stream));
   ewaldBatchDeltaKernel<<<grid, kThreads, shmem, ctx->stream>>>(b->runs, b->n_runs, b->row_start, b->slots, b->n,

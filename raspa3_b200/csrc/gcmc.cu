@@ -184,12 +184,14 @@ struct Dyn
   double2* S;       // [nk]
   double2* D;       // [nk]
 };
-__host__ __device__ inline size_t dynFixedBytes(int na, const int* kmax, bool ewald)
+__host__ __device__ constexpr size_t dynFixedBytes(int na, const int* kmax, bool ewald)
 {
   size_t b = sizeof(double) * kMaxTrials * na * 8 + sizeof(PairTerm) * na * na + ((sizeof(int) * kMaxTrials * na + 15) & ~size_t(15));
   if (ewald) b += sizeof(double2) * 2 * na * ((kmax[0] + 1) + (2 * kmax[1] + 1) + (kmax[2] + 1));
   return b;
 }
+constexpr int kTopK[3] = {kMaxK - 1, kMaxK - 1, kMaxK - 1};
+static_assert(dynFixedBytes(kMaxAtoms, kTopK, true) <= kSharedPerCta, "no launch takes more than kSharedPerCta");
 __device__ __forceinline__ Dyn dynOf(const Params& p)
 {
   extern __shared__ __align__(16) unsigned char dynSmem[];
@@ -1024,6 +1026,16 @@ rg_status rg_gcmc_create(rg_system* system, rg_ewald* ewald, const rg_gcmc_compo
   const size_t sk_bytes = 2 * sizeof(double2) * static_cast<size_t>(p.nk);
   g->smem = fixed + sk_bytes <= kSharedPerCta;
   g->shmem = fixed + (g->smem ? sk_bytes : 0);
+  // The limit belongs to the kernel on the device, which the objects of all contexts share: the most that any of them
+  // takes, so that no host thread lowers it between another's setting and launch.
+  auto kern = p.quintic ? (g->smem ? gcmcKernel<true, true> : gcmcKernel<true, false>)
+                        : (g->smem ? gcmcKernel<false, true> : gcmcKernel<false, false>);
+  err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSharedPerCta));
+  if (err)
+  {
+    rg_gcmc_destroy(g);
+    return rg::cudaFail(ctx, err, "rg_gcmc_create");
+  }
   *out = g;
   return RG_OK;
 }
@@ -1056,10 +1068,6 @@ rg_status rg_gcmc_run(rg_gcmc* g, int64_t moves, int record)
     const int chunk = static_cast<int>(left < g->max_moves_per_launch ? left : g->max_moves_per_launch);
     auto launch = [&](auto kern)
     {
-      // another object's call may have set this kernel's limit lower
-      const cudaError_t err =
-          cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(g->shmem));
-      if (err) return err;
       kern<<<g->n_chains, kThreads, g->shmem, ctx->stream>>>(g->p, g->moves_done, chunk, record, g->block_len);
       return cudaGetLastError();
     };

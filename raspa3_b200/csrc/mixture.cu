@@ -1931,8 +1931,11 @@ extern "C" rg_status rg_mixture_create(rg_system* system, rg_ewald* ewald, const
   const long long share = (static_cast<long long>(p.capacity) * na + x->blocks - 1) / x->blocks;
   p.nslice = static_cast<int>(std::max<long long>(64, std::min(std::min(share, (budget - fixedBytes) / perSite), 65535ll)));
   x->smem = dynBytes(p.tabK, p.ncand_max, p.cand_atoms, p.kpc, p.nseg_max, p.nslice, ncell);
+  // the limit belongs to the kernel on the device, which the mixtures of all contexts share: all that there is, so that no
+  // host thread lowers it between another's setting and launch
   err = cudaFuncSetAttribute(p.quintic ? mixtureKernel<true> : mixtureKernel<false>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(x->smem));
+                             cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             optin - static_cast<int>(fa.sharedSizeBytes));
   if (err == cudaSuccess)
     err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, p.quintic ? mixtureKernel<true> : mixtureKernel<false>,
                                                         kThreads, x->smem);
@@ -2108,7 +2111,6 @@ extern "C" rg_status rg_mixture_run_many(rg_mixture* const* mixtures, int n, int
   int sms = 0, perSM = 0;
   RG_CUDA(ctx, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
   auto kernel = x0->p.quintic ? mixtureKernel<true> : mixtureKernel<false>;
-  RG_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
   RG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, kernel, kThreads, smem));
   if (static_cast<long long>(n) * x0->blocks > static_cast<long long>(sms) * perSM)
     return rg::fail(ctx, RG_ERR_INVALID_ARGUMENT, "rg_mixture_run_many: the systems' CTAs do not fit on the GPU at once");
