@@ -1435,7 +1435,13 @@ __global__ void __launch_bounds__(kThreads, 1) mixtureKernel(const __grid_consta
       __syncthreads();
       if (sh.accept)
       {
-        if (tid < 32 && m != sh.n - 1) storeMolecule(m, sh.preCl, sh.preLast);
+        if (tid < 32)
+        {
+          // every lane has read the count before lane 0 lowers it below: storeMolecule is for the whole warp or none of it
+          const bool moveLast = m != sh.n - 1;
+          __syncwarp();
+          if (moveLast) storeMolecule(m, sh.preCl, sh.preLast);
+        }
         if (tid == 0)
         {
           // remove m from its component list, then move the last molecule into slot m (from the values read before
