@@ -220,7 +220,7 @@ __device__ __forceinline__ double pairEnergy(const Params& p, const PairTerm& t,
     const double x = rr * t.inv_sig2;
     const double i3 = rgd::rcpHouseholder(x * x * x);
     e = t.eps4 * (i3 * (i3 - 1.0)) - t.shift;
-    if (e > p.ff.overlap) *ov = 1;
+    if (!(e <= p.ff.overlap)) *ov = 1;  // NaN too: the reciprocal's refinement makes it of 0 and of subnormal numbers
   }
   if (p.ff.use_charge && rr < p.rcc2)
   {
