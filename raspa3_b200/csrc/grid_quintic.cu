@@ -260,10 +260,25 @@ __global__ void __launch_bounds__(kThreads) quinticKernel(QuinticParams p, Quint
   double wc[3] = {0.0, 0.0, 0.0}, reach2 = 0.0;
   if constexpr (RECT64)
   {
-    const double h[3] = {p.cell[0][0] * p.delta[0], p.cell[1][1] * p.delta[1], p.cell[2][2] * p.delta[2]};
-    wc[0] = h[0] * (4 * (warp & 1) - 2);
-    wc[2] = h[2] * (2 * (warp >> 1) - 1);
-    const double reach = sqrt(p.rc2) + sqrt(2.25 * (h[0] * h[0] + h[1] * h[1]) + 0.25 * h[2] * h[2]) + 1e-6;
+    // by the cell's full vectors, as the points are: a cell given as rectangular may still be sheared
+    double half2 = 0.0;
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+      wc[r] = p.cell[0][r] * ((4 * (warp & 1) - 2) * p.delta[0]) + p.cell[2][r] * ((2 * (warp >> 1) - 1) * p.delta[2]);
+#pragma unroll
+    for (int g = 0; g < 4; ++g)  // the longest of the four diagonals of the warp's points
+    {
+      double d2 = 0.0;
+#pragma unroll
+      for (int r = 0; r < 3; ++r)
+      {
+        const double v = 1.5 * p.cell[0][r] * p.delta[0] + ((g & 1) ? -1.5 : 1.5) * p.cell[1][r] * p.delta[1] +
+                         ((g & 2) ? -0.5 : 0.5) * p.cell[2][r] * p.delta[2];
+        d2 += v * v;
+      }
+      half2 = fmax(half2, d2);
+    }
+    const double reach = sqrt(p.rc2) + sqrt(half2) + 1e-6;
     reach2 = reach * reach;
   }
 
