@@ -740,6 +740,16 @@ void hostTerms(const rg_ewald* e, const rg_atom* atoms, int n_atoms, const int32
       }
 }
 
+// Whether the terms are the host's. The device has the atoms' fractional coordinates alone and takes the minimum image in
+// those; for a cell given as rectangular whose vectors are off the axes that is another image than along its diagonal.
+bool hostTermsOf(const rg_ewald* e, int n_atoms)
+{
+  bool sheared = false;
+  for (int c = 0; c < 3; ++c)
+    for (int r = 0; r < 3; ++r) sheared = sheared || (c != r && e->box.c[c][r] != 0.0);
+  return n_atoms <= kHostTerms || (sheared && !e->box.triclinic);
+}
+
 // fractional coordinates and signed weights of the old (sign old_sign) and new atoms of a move
 void packMoved(const rg_ewald* e, const rg_atom* old_atoms, int n_old, const rg_atom* new_atoms, int n_new,
                double old_sign, MovedAtom* h)
@@ -1110,8 +1120,8 @@ rg_status rg_ewald_full(rg_ewald* e, const rg_atom* atoms, int n_atoms, const in
   const double C = rg::coulombFactor();
   const double alpha = e->alpha;
   // self, exclusion and net-charge sums: on the device beside the Fourier sums, or, for a few atoms, on the host while
-  // the kernels are in flight (kHostTerms)
-  const bool host_terms = n_atoms <= kHostTerms;
+  // the kernels are in flight
+  const bool host_terms = hostTermsOf(e, n_atoms);
   TermsParams tp{};
   tp.atoms = static_cast<const MovedAtom*>(e->moved);
   tp.n_atoms = n_atoms;

@@ -8,7 +8,7 @@ import pytest
 
 from raspa3_b200 import native
 from raspa3_b200.forcefield import box_struct, make_atoms, positions_of
-from raspa3_b200.synthetic import synthetic_forcefield
+from raspa3_b200.synthetic import random_molecules, synthetic_forcefield
 
 pytestmark = pytest.mark.gpu
 CELL = np.array([[17.0, 0.0, 0.0], [5.0, 16.0, 0.0], [-8.0, 6.0, 15.0]])
@@ -70,3 +70,22 @@ def test_lennard_jones_grid(ctx, rectangular, scheme, dims):
     assert open_.sum() > len(energy) // 8
     scale = np.maximum(np.abs(energy), math.sqrt(np.mean(energy[open_] ** 2)))
     assert np.max((np.abs(e - energy) / scale)[open_]) < 1e-9
+
+
+# the atoms' own terms of 255 and 258 atoms: on the host, and on the device for a cell along the axes
+@pytest.mark.parametrize("molecules", [85, 86])
+def test_ewald_exclusion(ctx, oracle, rectangular, monkeypatch, molecules):
+    """Self and exclusion energies against the oracle's: 1e-9, as for the other recomputes."""
+    obox = oracle.obox
+    monkeypatch.setattr(oracle, "obox", lambda cell, triclinic=None: obox(cell, False))
+    ff = synthetic_forcefield(charges=True, kmax=4)
+    mols = random_molecules(ff, CELL, molecules, seed=5)
+    shift = np.random.default_rng(2).integers(-1, 2, size=(len(mols), 3)) @ CELL  # split over the cell's faces
+    for a, axis in enumerate("xyz"):
+        mols[axis] += shift[:, a]
+    ew = native.Ewald(ctx, ff, CELL)
+    got = ew.full(mols, [3] * molecules)
+    ref, _ = oracle.ewald_fourier_energy(ff, CELL, mols, [3] * molecules)
+    for k in ("ewald_self", "ewald_exclusion"):
+        assert abs(got[k] - ref[k]) <= 1e-9 * max(1.0, abs(ref[k])), (k, got[k], ref[k])
+    ew.close()
