@@ -710,6 +710,11 @@ void addDud(double* arr, int gA, int gB, double sA, double sB, double factor)
 // the kernels here, while the device's chain of loads, erf and reductions made calls of 15 to 180 atoms 3 to 8 us longer.
 // For 12,000 atoms the erf alone take the host 130 us, and the device's share does not show.
 constexpr int kHostTerms = 256;
+// Without k-vectors, or with dU/dlambda groups (whose Fourier sums have kernels of their own), the device's share is a
+// launch by itself, which shows: up to this many pairs within molecules the host is the faster side. Of molecules of three
+// atoms (kmax 8, one group) 270, 540, 1,200 and 2,400 take 32, 41, 62 and 114 us with the host's terms and 40, 48, 62 and 93
+// with the device's; of molecules of ten 270 and 540 (1,215 and 2,430 pairs) 44 and 80, and 45 and 52.
+constexpr int64_t kHostPairs = 1300;
 void hostTerms(const rg_ewald* e, const rg_atom* atoms, int n_atoms, const int32_t* molecule_sizes, int n_molecules,
                double v[kTerms])
 {
@@ -742,12 +747,20 @@ void hostTerms(const rg_ewald* e, const rg_atom* atoms, int n_atoms, const int32
 
 // Whether the terms are the host's. The device has the atoms' fractional coordinates alone and takes the minimum image in
 // those; for a cell given as rectangular whose vectors are off the axes that is another image than along its diagonal.
-bool hostTermsOf(const rg_ewald* e, int n_atoms)
+bool hostTermsOf(const rg_ewald* e, int n_atoms, const int32_t* molecule_sizes, int n_molecules)
 {
+  if (n_atoms <= kHostTerms) return true;
+  if (e->nk == 0 || e->n_groups > 0)
+  {
+    int64_t pairs = 0;
+    for (int m = 0; m < n_molecules && !e->omit_inter; ++m)
+      pairs += static_cast<int64_t>(molecule_sizes[m]) * (molecule_sizes[m] - 1) / 2;
+    if (pairs <= kHostPairs) return true;
+  }
   bool sheared = false;
   for (int c = 0; c < 3; ++c)
     for (int r = 0; r < 3; ++r) sheared = sheared || (c != r && e->box.c[c][r] != 0.0);
-  return n_atoms <= kHostTerms || (sheared && !e->box.triclinic);
+  return sheared && !e->box.triclinic;
 }
 
 // fractional coordinates and signed weights of the old (sign old_sign) and new atoms of a move
@@ -1116,12 +1129,17 @@ rg_status rg_ewald_full(rg_ewald* e, const rg_atom* atoms, int n_atoms, const in
   }
   RG_CUDA(ctx, cudaSetDevice(ctx->device));
   const int G = e->n_groups;
-  if (rg_status st = stageFull(e, atoms, n_atoms, molecule_sizes, e->omit_inter ? 0 : n_molecules)) return st;
+  const bool host_terms = hostTermsOf(e, n_atoms, molecule_sizes, n_molecules);
+  if (e->nk == 0 && host_terms)
+  {
+    if (rg_status st = rg::checkFinite(ctx, atoms, n_atoms, "rg_ewald_full")) return st;
+  }
+  else if (rg_status st = stageFull(e, atoms, n_atoms, molecule_sizes, e->omit_inter ? 0 : n_molecules))
+    return st;
   const double C = rg::coulombFactor();
   const double alpha = e->alpha;
   // self, exclusion and net-charge sums: on the device beside the Fourier sums, or, for a few atoms, on the host while
   // the kernels are in flight
-  const bool host_terms = hostTermsOf(e, n_atoms);
   TermsParams tp{};
   tp.atoms = static_cast<const MovedAtom*>(e->moved);
   tp.n_atoms = n_atoms;
