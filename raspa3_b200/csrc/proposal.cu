@@ -85,7 +85,7 @@ __device__ __forceinline__ float dot4(float4 a, float4 b, float acc)
   return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, acc))));
 }
 
-__device__ void loadWeights(MlpWeights& S, const float* __restrict__ theta)
+__device__ void loadWeights(MlpWeights& S, const float* theta)
 {
   const float4* w1 = reinterpret_cast<const float4*>(theta + kOffW1);
   for (int q = threadIdx.x; q < kH * kIn / 4; q += kThreads)
@@ -172,11 +172,13 @@ __device__ __forceinline__ void forward(MlpForwardShared& S, int ig, int jq, flo
 // with each kernel's start overlapping the end of the one before.
 // One tile's loss and gradient partial; batch size B scales the loss. Samples: tile0 + i in order, or (random) drawn
 // from the n_samples by splitmix64 of (seed, step, slot).
-__global__ void __launch_bounds__(kThreads) mlpGradKernel(const float* __restrict__ theta, const float* __restrict__ s,
+// What the kernel before writes while this one may have started (theta here, the partials in the reduction) is not declared
+// __restrict__: a load through a read-only pointer may take a path that takes the data for constant while the kernel runs,
+// or be moved ahead of the wait.
+__global__ void __launch_bounds__(kThreads) mlpGradKernel(const float* theta, const float* __restrict__ s,
                                                           const float* __restrict__ target, int64_t n_samples,
                                                           bool random, int batch, unsigned long long seed,
-                                                          long long step, float* __restrict__ partial,
-                                                          float* __restrict__ lossPartial)
+                                                          long long step, float* partial, float* lossPartial)
 {
   extern __shared__ __align__(16) unsigned char smraw[];
   MlpGradShared& S = *reinterpret_cast<MlpGradShared*>(smraw);
@@ -318,12 +320,10 @@ __global__ void __launch_bounds__(kThreads) mlpGradKernel(const float* __restric
 // parameter bring the partials of kReduceTiles tiles into shared memory, all their loads in flight together; one thread
 // adds them in order (one thread that also loaded them waited for one load after another).
 constexpr int kReduceLanes = 8, kReduceTiles = 128;
-__global__ void __launch_bounds__(kThreads) reduceAdamKernel(float* __restrict__ theta, float* __restrict__ m,
-                                                             float* __restrict__ v, const float* __restrict__ partial,
+__global__ void __launch_bounds__(kThreads) reduceAdamKernel(float* theta, float* m, float* v, const float* partial,
                                                              int n_tiles, float lr, float b1, float b2, float eps,
-                                                             long long t, float* __restrict__ grad_out,
-                                                             const float* __restrict__ lossPartial,
-                                                             float* __restrict__ loss_out, int batch)
+                                                             long long t, float* grad_out, const float* lossPartial,
+                                                             float* loss_out, int batch)
 {
   constexpr int kItems = kThreads / kReduceLanes;
   __shared__ float tiles[kReduceTiles][kItems];
