@@ -229,7 +229,8 @@ __device__ __noinline__ double internalEnergy(const Params& p, const SysDev& S, 
 // trial whose cumulative shifted Boltzmann factor reaches u times the total. retrace: trial 0 (the old position).
 // Returns -1 when every trial overlaps. Called by all 32 lanes of warp 0.
 // The shift of the Boltzmann factors is the largest exponent rounded to FP32 (one warp instruction; any shift near it
-// serves), and the trials are in the first kMaxTrials lanes.
+// serves), and the trials are in the first kMaxTrials lanes. Beyond 1e10 the rounding alone is hundreds: the factors stay
+// finite then, so that a vanishing sum is 0 and not 0 times infinity.
 __device__ __forceinline__ int warpSelect(double lbf, bool ok, bool retrace, double u, double* sum)
 {
   const int lane = threadIdx.x & 31;
@@ -237,7 +238,7 @@ __device__ __forceinline__ int warpSelect(double lbf, bool ok, bool retrace, dou
   const int bits = __float_as_int(static_cast<float>(fmax(lbf, -1e38)));
   const int key = __reduce_max_sync(0xffffffffu, ok ? (bits >= 0 ? bits : bits ^ 0x7fffffff) : INT_MIN);
   const double mx = static_cast<double>(__int_as_float(key >= 0 ? key : key ^ 0x7fffffff));
-  double incl = ok ? exp(lbf - mx) : 0.0;
+  double incl = ok ? exp(fmin(lbf - mx, 700.0)) : 0.0;
   const double factor = exp(mx);
 #pragma unroll
   for (int o = 1; o < kMaxTrials; o <<= 1)
