@@ -1917,7 +1917,8 @@ extern "C" rg_status rg_mixture_create(rg_system* system, rg_ewald* ewald, const
   // most the old and the new molecule's atoms
   p.ncand_max = std::max(1, p.k2);
   p.cand_atoms = 2 * na;
-  const long long budget = static_cast<long long>(optin) - static_cast<long long>(fa.sharedSizeBytes) - 1024;
+  const long long budget = static_cast<long long>(optin) - static_cast<long long>(fa.sharedSizeBytes);
+  constexpr long long kLeastSlice = 16;  // sites staged where no more fit; 64 and more where they do
   auto fixedOf = [&](int cells) {
     return static_cast<long long>(
                dynBytes(p.tabK, p.ncand_max, p.cand_atoms, p.kpc, p.nseg_max, 0, cells ? p.nc[0] * p.nc[1] * p.nc[2] : 0)) +
@@ -1925,17 +1926,17 @@ extern "C" rg_status rg_mixture_create(rg_system* system, rg_ewald* ewald, const
   };
   auto perSiteOf = [&](int cells) { return static_cast<long long>(sizeof(int4) + (cells ? sizeof(unsigned short) : 0)); };
   // without room for the cells next to the k-range, the pair loop walks the slice as it is
-  if (p.cells && fixedOf(1) + perSiteOf(1) * 64 > budget) p.cells = 0;
+  if (p.cells && fixedOf(1) + perSiteOf(1) * kLeastSlice > budget) p.cells = 0;
   const int ncell = p.cells ? p.nc[0] * p.nc[1] * p.nc[2] : 0;
   const long long fixedBytes = fixedOf(p.cells);
   const long long perSite = perSiteOf(p.cells);
-  if (fixedBytes + perSite * 64 > budget)
+  if (fixedBytes + perSite * kLeastSlice > budget)
   {
     delete x;
     return rg::fail(ctx, RG_ERR_UNSUPPORTED, "rg_mixture: the CTA's k-range does not fit in shared memory (use more CTAs)");
   }
   const long long share = (static_cast<long long>(p.capacity) * na + x->blocks - 1) / x->blocks;
-  p.nslice = static_cast<int>(std::max<long long>(64, std::min(std::min(share, (budget - fixedBytes) / perSite), 65535ll)));
+  p.nslice = static_cast<int>(std::min({std::max(share, 64ll), (budget - fixedBytes) / perSite, 65535ll}));
   x->smem = dynBytes(p.tabK, p.ncand_max, p.cand_atoms, p.kpc, p.nseg_max, p.nslice, ncell);
   // the limit belongs to the kernel on the device, which the mixtures of all contexts share: all that there is, so that no
   // host thread lowers it between another's setting and launch

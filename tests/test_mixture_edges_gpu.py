@@ -1,4 +1,4 @@
-"""The mixture kernel at its edges: deletions that take the last molecule of the list."""
+"""The mixture kernel at its edges: deletions that take the last molecule of the list, and a k-range that only just fits."""
 
 import numpy as np
 import pytest
@@ -48,6 +48,32 @@ def test_deletion_of_the_last_molecule(ctx, blocks, swap_only):
         ref = ew.structure_factors(0 if len(comp) else 2)
         assert np.max(np.abs(mx.structure_factors() - ref)) <= 1e-9 * max(1.0, np.max(np.abs(ref)))
     assert deletions > 50
+    mx.close()
+    ew.close()
+    system.close()
+
+
+# one CTA with 6,347 and 5,669 k-vectors and the tables of 3 and 6 orientations: 211 KB of shared memory beside the kernel's
+# own, of 227 in all
+@pytest.mark.parametrize("kmax,orientations", [((11, 11, 11), 3), ((9, 10, 13), 6)])
+def test_largest_k_range_of_one_cta(ctx, kmax, orientations):
+    """Created and run; the structure factors are those of the molecules that are there (1e-9, as above)."""
+    ff = synthetic_forcefield(charges=True, alpha=0.265, kmax=max(kmax), sphere=False)
+    ff.kmax = kmax
+    system = native.System(ctx, ff, CELL, empty_framework())
+    ew = native.Ewald(ctx, ff, CELL)
+    ew.set_framework(empty_framework())
+    comps = [co2_component(), n2_component()]
+    mx = native.Mixture(system, ew, comps, beta_of(300.0), [fugacity_of(1e6)] * 2, np.zeros((0, 3, 3)),
+                        np.zeros(0, dtype=np.int32), max_molecules=60, seed=4, n_blocks=1, n_orient=orientations)
+    mx.set_state(0.0, ew.structure_factors(2))
+    mx.run(2000, record=True)
+    r = mx.results()
+    xyz, comp = mx.positions()
+    assert r["status"] == 0 and len(comp) > 4
+    ew.full(molecules_as_atoms(ff, comps, xyz, comp), [3] * len(comp))
+    ref = ew.structure_factors(0)
+    assert np.max(np.abs(mx.structure_factors() - ref)) <= 1e-9 * max(1.0, np.max(np.abs(ref)))
     mx.close()
     ew.close()
     system.close()
