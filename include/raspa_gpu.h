@@ -467,7 +467,9 @@ rg_status rg_gcmc_get_positions(rg_gcmc* gcmc, int chain, double* xyz, int capac
 /* Uses a learned first-bead proposal for the CBMC insertion and deletion trials of every chain (NULL: back to uniform
  * positions). The trial weights become exp(-beta U) / q with q the proposal density relative to uniform; the
  * acceptance rules are unchanged, so the sampled ensemble is the same. The simulation box must be an integer
- * replication of unit_cell, the cell the proposal is defined on. No counterpart in the reference. */
+ * replication of unit_cell, the cell the proposal is defined on. The chains read the proposal's table in every later
+ * run: destroy the proposal only after another one, or NULL, has been set, or after the chains. No counterpart in the
+ * reference. */
 rg_status rg_gcmc_set_proposal(rg_gcmc* gcmc, rg_proposal* proposal, const rg_box* unit_cell);
 
 /* ---- learned first-bead proposal (no counterpart in the reference; plugs into the uniform first-bead sampling of
@@ -727,7 +729,8 @@ rg_status rg_mixture_get_positions(rg_mixture* mixture, double* xyz, int32_t* co
                                    int* n_molecules);
 /* The current structure factors (framework included), 2 doubles per k-vector in the rg_ewald order: storedEik. */
 rg_status rg_mixture_get_structure_factors(rg_mixture* mixture, double* host, int64_t n_doubles);
-/* Learned first-bead proposal of one component (NULL: uniform). */
+/* Learned first-bead proposal of one component (NULL: uniform). The mixture reads the proposal's table in every later
+ * run: destroy the proposal only after another one, or NULL, has been set, or after the mixture. */
 rg_status rg_mixture_set_proposal(rg_mixture* mixture, int component, rg_proposal* proposal, const rg_box* unit_cell);
 rg_status rg_mixture_info(rg_mixture* mixture, int* blocks, int64_t* nk);
 

@@ -806,14 +806,14 @@ class Gcmc:
         check(self.ctx.handle, lib().rg_gcmc_run(self.handle, moves, 1 if record else 0), "rg_gcmc_run")
 
     def set_proposal(self, proposal, unit_cell=None):
-        """Learned first-bead proposal (None: uniform positions)."""
-        self._proposal = proposal
+        """Learned first-bead proposal (None: uniform positions); kept alive while it is in use."""
         if proposal is None:
             check(self.ctx.handle, lib().rg_gcmc_set_proposal(self.handle, None, None), "rg_gcmc_set_proposal")
         else:
             box = box_struct(unit_cell)
             check(self.ctx.handle, lib().rg_gcmc_set_proposal(self.handle, proposal.handle, ctypes.byref(box)),
                   "rg_gcmc_set_proposal")
+        self._proposal = proposal
 
     def results(self):
         out = (GcmcChainResult * self.n_chains)()
@@ -1095,6 +1095,7 @@ class Mixture:
         cc = np.ascontiguousarray(comp, dtype=np.int32)
         self.na = self.components[0].n_atoms
         self.max_molecules = max_molecules
+        self._proposals = {}
         h = ctypes.c_void_p()
         check(self.ctx.handle, lib().rg_mixture_create(system.handle, ewald.handle if ewald is not None else None,
                                                        ctypes.cast(arr, ctypes.c_void_p), len(self.components),
@@ -1164,6 +1165,7 @@ class Mixture:
         return {"blocks": b.value, "n_kvectors": nk.value}
 
     def set_proposal(self, component: int, proposal, unit_cell=None):
+        """Learned first-bead proposal of one component (None: uniform positions); kept alive while it is in use."""
         if proposal is None:
             check(self.ctx.handle, lib().rg_mixture_set_proposal(self.handle, component, None, None),
                   "rg_mixture_set_proposal")
@@ -1171,3 +1173,4 @@ class Mixture:
             box = box_struct(unit_cell)
             check(self.ctx.handle, lib().rg_mixture_set_proposal(self.handle, component, proposal.handle,
                                                                  ctypes.byref(box)), "rg_mixture_set_proposal")
+        self._proposals[component] = proposal
