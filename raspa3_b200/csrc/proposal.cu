@@ -865,9 +865,14 @@ rg_status rg_proposal_create(rg_mlp* m, int32_t cells_per_axis, double eps_unifo
 rg_status rg_proposal_destroy(rg_proposal* p)
 {
   if (!p) return RG_OK;
-  if (p->ctx) cudaStreamSynchronize(p->ctx->stream);
-  // the larger of the two buffers stays with the context
-  if (p->ctx && p->table.bytes > p->ctx->spare_table.bytes) std::swap(p->table, p->ctx->spare_table);
+  if (p->ctx)
+  {
+    // a run that reads the table may be on any stream that the context had before: wait for all, as a free does
+    cudaSetDevice(p->ctx->device);
+    cudaDeviceSynchronize();
+    // the larger of the two buffers stays with the context
+    if (p->table.bytes > p->ctx->spare_table.bytes) std::swap(p->table, p->ctx->spare_table);
+  }
   if (p->table.ptr) cudaFree(p->table.ptr);
   delete p;
   return RG_OK;

@@ -7,6 +7,9 @@ import numpy as np
 import pytest
 
 from raspa3_b200 import native
+from raspa3_b200.gcmc import beta_of, fugacity_of, methane_component
+from raspa3_b200.synthetic import synthetic_forcefield
+from test_gcmc_gpu import empty_framework
 
 CELL = np.diag([30.0, 30.0, 30.0])
 
@@ -52,3 +55,39 @@ def test_proposal_in_use_is_referenced(monkeypatch, cls, first):
     user.set_proposal(*first, None)
     gc.collect()
     assert ref() is None
+
+
+def _chains(torch, reuse):
+    """A run with one proposal, queued on a stream; then, on another, that proposal is destroyed and (reuse) its memory
+    taken for the next, which has another network's density."""
+    ctx = native.Context(0)
+    ff = synthetic_forcefield(charges=False)
+    system = native.System(ctx, ff, CELL, empty_framework())
+    g = native.Gcmc(system, None, methane_component(), beta_of(300.0), fugacity_of(2e6), n_chains=64, seed=9)
+    theta = np.random.default_rng(1).normal(size=(2, native.lib().rg_mlp_num_params())).astype(np.float32)
+    nets = [native.Mlp(ctx, seed=1) for _ in range(2)]
+    for m, t in zip(nets, theta):
+        m.set_params(0.3 * t)
+    first = native.Proposal(nets[0], cells_per_axis=40, eps_uniform=0.05)
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    g.set_proposal(first, CELL)
+    ctx.synchronize()
+    ctx.set_stream(streams[0].cuda_stream)
+    g.run(8000, record=True)
+    if reuse:
+        ctx.set_stream(streams[1].cuda_stream)
+        g.set_proposal(None)
+        first.close()
+        second = native.Proposal(nets[1], cells_per_axis=40, eps_uniform=0.05)
+        second.close()
+        ctx.set_stream(streams[0].cuda_stream)
+    out = g.results()
+    ctx.set_stream(None)
+    ctx.close()
+    return out
+
+
+@pytest.mark.gpu
+def test_destroyed_behind_a_run():
+    torch = pytest.importorskip("torch")
+    assert _chains(torch, False) == _chains(torch, True)
