@@ -29,8 +29,8 @@ struct rg_ctx
   // on first use).
   cudaStream_t copy_stream = nullptr;
   std::vector<cudaEvent_t> events;
-  // The device memory of the last tabulated proposal that was destroyed, for the next one (one buffer, freed with the
-  // context): freeing and mapping it anew took 1 to 5 ms when nothing else held its pages.
+  // The device memory of a tabulated proposal that was destroyed, for the next one (one buffer of up to 64 MB, freed with
+  // the context): freeing and mapping it anew took 1 to 5 ms when nothing else held its pages.
   Slot spare_table;
   // Recorded behind the last kernel of a call that returned before the stream was done with it (rg::leave), until the
   // stream is changed: the next stream's work comes after it.

@@ -806,6 +806,9 @@ rg_status rg_proposal_sample_targets(rg_system* system, int pseudo_atom, double 
   return RG_OK;
 }
 
+// Bytes of a destroyed table that stay with the context at most (128^3 cells have 34 MB; 256^3, 268 MB, are freed)
+constexpr size_t kKeptTable = 64 << 20;
+
 rg_status rg_proposal_create(rg_mlp* m, int32_t cells_per_axis, double eps_uniform, rg_proposal** out)
 {
   if (!m || !out || cells_per_axis < 1 || cells_per_axis > 256 || !(eps_uniform > 0.0) || eps_uniform > 1.0)
@@ -832,7 +835,8 @@ rg_status rg_proposal_create(rg_mlp* m, int32_t cells_per_axis, double eps_unifo
   float* f = reinterpret_cast<float*>(sums + blocks + 2);
   cudaError_t err = cudaSuccess;
   const size_t bytes = 2 * sizeof(double) * static_cast<size_t>(nc);
-  if (ctx->spare_table.bytes >= bytes)
+  // the kept table, unless it would be far too large for this one
+  if (ctx->spare_table.bytes >= bytes && ctx->spare_table.bytes <= 8 * bytes + (1 << 20))
     std::swap(p->table, ctx->spare_table);
   else if (!(err = cudaMalloc(&p->table.ptr, bytes)))
     p->table.bytes = bytes;
@@ -871,7 +875,8 @@ rg_status rg_proposal_destroy(rg_proposal* p)
     cudaSetDevice(p->ctx->device);
     cudaDeviceSynchronize();
     // the larger of the two buffers stays with the context
-    if (p->table.bytes > p->ctx->spare_table.bytes) std::swap(p->table, p->ctx->spare_table);
+    if (p->table.bytes <= kKeptTable && p->table.bytes > p->ctx->spare_table.bytes)
+      std::swap(p->table, p->ctx->spare_table);
   }
   if (p->table.ptr) cudaFree(p->table.ptr);
   delete p;

@@ -91,3 +91,23 @@ def _chains(torch, reuse):
 def test_destroyed_behind_a_run():
     torch = pytest.importorskip("torch")
     assert _chains(torch, False) == _chains(torch, True)
+
+
+# small after large and large after small, across the sizes that are kept (up to 64 MB, 161^3 cells) and handed on
+@pytest.mark.gpu
+def test_tables_of_changing_sizes():
+    ctx = native.Context(0)
+    m = native.Mlp(ctx, seed=5)
+    sizes = (2, 200, 3, 128, 60, 128, 1, 162, 8)
+    s = np.random.default_rng(2).random((50, 3))
+    fresh = {}
+    for cells in set(sizes):
+        one = native.Context(0)
+        n = native.Mlp(one, seed=5)
+        fresh[cells] = native.Proposal(n, cells_per_axis=cells).density(s)
+        one.close()
+    for cells in sizes:
+        p = native.Proposal(m, cells_per_axis=cells)
+        assert np.array_equal(p.density(s), fresh[cells])
+        p.close()
+    ctx.close()
