@@ -93,7 +93,7 @@ struct Params
   // per-chain state
   double4* pos;              // [chain][capacity * n_atoms]
   double2* sk;               // [chain][nk] structure factors (framework included)
-  double2* dsk;              // [chain][nk] scratch: structure-factor change of the current move
+  double2* dsk;              // [chain][nk] scratch: structure-factor change of the current move (null: in shared memory)
   int* n;                    // [chain]
   double* energy;            // [chain]
   double* stats;             // [chain][kStats]
@@ -942,9 +942,9 @@ rg_status rg_gcmc_create(rg_system* system, rg_ewald* ewald, const rg_gcmc_compo
   p.seed = params->seed;
   p.use_ewald = (ewald != nullptr && ff.use_charge) ? 1 : 0;
   int64_t nk = 0;
+  const double2* s_rigid = nullptr;
   if (p.use_ewald)
   {
-    const double2* s_rigid;
     double alpha, single_ion;
     const char4* kvec;
     const double* temp;
@@ -978,6 +978,17 @@ rg_status rg_gcmc_create(rg_system* system, rg_ewald* ewald, const rg_gcmc_compo
       }
     p.comp.self_excl = se;
     p.nk = nk;
+  }
+  // The structure factors and their change stay in shared memory where four CTAs still fit on an SM (the registers'
+  // limit): at kmax 8 the 1,152 k-vectors of the sphere take 37 KB. Larger sets stay in global memory. 200 moves of 1,184
+  // chains in a box of CO2 with the former kernel, all in global memory, and with this one: 13.5 and 5.5 ms at 1,182
+  // k-vectors (shared now), 20.5 and 13.8 at 3,609 (global), 39.6 and 30.8 at 6,062; of 148 chains at 3,609 7.4 and 4.4.
+  const size_t fixed = dynFixedBytes(comp->n_atoms, p.kmax, p.use_ewald != 0);
+  const size_t sk_bytes = 2 * sizeof(double2) * static_cast<size_t>(nk);
+  g->smem = fixed + sk_bytes <= kSharedPerCta;
+  g->shmem = fixed + (g->smem ? sk_bytes : 0);
+  if (p.use_ewald)
+  {
     // the k-vectors as runs of kz, and their prefactors by (|kz|, sign, run)
     const std::vector<int4> runs = rgd::ewaldRuns(ewald);  // longest first: the threads of large |kz| are neighbours
     p.n_runs = static_cast<int>(runs.size());
@@ -995,7 +1006,7 @@ rg_status rg_gcmc_create(rg_system* system, rg_ewald* ewald, const rg_gcmc_compo
     // all chains start from the framework structure factor
     const size_t skb = sizeof(double2) * static_cast<size_t>(nk) * n_chains;
     if (!err) err = cudaMalloc(reinterpret_cast<void**>(&p.sk), skb);
-    if (!err) err = cudaMalloc(reinterpret_cast<void**>(&p.dsk), skb);
+    if (!err && !g->smem) err = cudaMalloc(reinterpret_cast<void**>(&p.dsk), skb);
     for (int c = 0; c < n_chains && !err; ++c)
       err = cudaMemcpyAsync(p.sk + static_cast<size_t>(c) * nk, s_rigid, sizeof(double2) * nk,
                             cudaMemcpyDeviceToDevice, ctx->stream);
@@ -1020,12 +1031,6 @@ rg_status rg_gcmc_create(rg_system* system, rg_ewald* ewald, const rg_gcmc_compo
     rg_gcmc_destroy(g);
     return rg::cudaFail(ctx, err, "rg_gcmc_create");
   }
-  // The structure factors and their change stay in shared memory where four CTAs still fit on an SM (the registers'
-  // limit): at kmax 8 the 1,152 k-vectors of the sphere take 37 KB. Larger sets stay in global memory.
-  const size_t fixed = dynFixedBytes(comp->n_atoms, p.kmax, p.use_ewald != 0);
-  const size_t sk_bytes = 2 * sizeof(double2) * static_cast<size_t>(p.nk);
-  g->smem = fixed + sk_bytes <= kSharedPerCta;
-  g->shmem = fixed + (g->smem ? sk_bytes : 0);
   // The limit belongs to the kernel on the device, which the objects of all contexts share: the most that any of them
   // takes, so that no host thread lowers it between another's setting and launch.
   auto kern = p.quintic ? (g->smem ? gcmcKernel<true, true> : gcmcKernel<true, false>)
