@@ -56,7 +56,7 @@ struct rg_ewald
   // staging of the last staged atoms: the context's scratch, set anew by each call that stages (stageRoom)
   void* moved = nullptr;
   void* moved_host = nullptr;
-  ulonglong2* result_host = nullptr;  // mapped pinned: the kernels' last blocks post the totals here (rg::collect)
+  ulonglong2* result_host = nullptr;  // mapped pinned: the kernels post their sums or totals here (rg::collect)
   unsigned int calls = 0;
 };
 
@@ -1435,7 +1435,6 @@ struct rg_ewald_batch
   rg_ewald* ewald = nullptr;
   rg_ctx* ctx = nullptr;  // of the Ewald state, which may be gone when the batch is destroyed
   int n = 0;
-  int max_atoms = 0;
   // [2][n][slots]: S(k) by rows of (|kz|, sign), a row holding the k-vectors of that kz of all runs side by side, so that
   // neighbouring threads, which take neighbouring runs, read and write neighbouring numbers
   double2* sk = nullptr;
@@ -1484,8 +1483,9 @@ __host__ __device__ inline size_t batchSharedBytes(int stride, int kxm, int kym,
 // thread that adds to it and back (rows by kz, see rg_ewald_batch): the bound is HBM, 32 bytes per k-vector. Before, a
 // thread took one k-vector at a time in list order and read two phasors per atom and k-vector from shared memory, whose
 // bandwidth bound it: 114 us for 1,184 systems of 8,124 k-vectors. With four |kz| per thread, whose sums came before the
-// loads of S, three blocks fitted on an SM: 88 us. With two, S loaded first, four blocks fit: 73 us (47 us at the measured
-// copy rate, were all of S read and all of the trial S written through HBM).
+// loads of S, three blocks fitted on an SM: 88 us. With two, S loaded first, four blocks fit: 73 us, and 79 with the
+// kernel behind it that adds the blocks' energies (47 us at the measured copy rate, were all of S read and all of the trial
+// S written through HBM).
 __global__ void __launch_bounds__(kThreads, 4) ewaldBatchDeltaKernel(
     const int4* __restrict__ runs, int n_runs, const int* __restrict__ row_start, int64_t slots, int n_systems,
     const double* __restrict__ run_temp, double2* sk, const unsigned char* __restrict__ upload, int atom_stride, int kxm,

@@ -634,7 +634,7 @@ rg_status launchGrad(rg_mlp* m, const float* s, const float* t, int64_t n, bool 
                                  step, m->partial, m->lossPartial));
   return RG_OK;
 }
-// Forward pass on n positions (s null: the centres of cells^3 cells), at most two CTAs per SM
+// Forward pass on n positions (s null: the centres of cells^3 cells), at most three CTAs per SM
 rg_status launchForward(rg_mlp* m, const float* s, int cells, int64_t n, float* out, int* largest)
 {
   rg_ctx* ctx = m->ctx;
